@@ -114,3 +114,22 @@ def test_step_gravity_rebuilds_mask_after_wall_change(cuda, tf, oracle):
     b.config.newton_grav = False
     tf.step_gravity(b, solver)
     assert not b.grav_fx.any().item() and not b.grav_fy.any().item()
+
+
+@pytest.mark.parametrize("X,Y", [(1, 1), (2, 5), (16, 17), (33, 36), (75, 38), (125, 9), (90, 60), (129, 128), (250, 31),
+                                 (256, 255), (257, 300), (513, 4), (5, 640), (1025, 3), (2048, 2), (2, 2048)])
+def test_fp32_plan_lengths(cuda, tf, oracle, X, Y):
+    """The transform lengths' edges: two and three radices, each radix first,
+    in the middle and last, the odd radix 5 (whose middle frequency is stored
+    or mirrored by item), lengths met exactly and by one cell, the longest;
+    one row, an odd row left over from the pairs. FP32 rounding of at most a
+    few ulp per step over at most six steps stays far below the solve's bar."""
+    rng = np.random.default_rng(1000 * X + Y)
+    mass = rng.uniform(-1.0, 3.0, X * Y).astype(np.float32) * (rng.random(X * Y) < 0.3)
+    mass[0] = 1.0
+    mask = np.where(rng.random(X * Y) < 0.95, np.uint32(0xFFFFFFFF), np.uint32(0))
+    gx, gy = solve_gpu(tf, cuda, X, Y, mask, mass_f32=mass)
+    dx, dy = oracle.grav_solve(X, Y, mask, mass_f32=mass, dtype=np.float64)
+    scale = max(np.abs(dx).max(), np.abs(dy).max(), 1e-30)
+    assert np.abs(gx - dx).max() <= TOL * scale and np.abs(gy - dy).max() <= TOL * scale
+    assert np.all(gx[mask == 0] == 0) and np.all(gy[mask == 0] == 0)

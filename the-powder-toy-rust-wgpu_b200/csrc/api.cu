@@ -303,8 +303,8 @@ int tpt_grav_plan_destroy(tpt_grav_plan *p) {
 int tpt_grav_plan_dims(const tpt_grav_plan *p, uint32_t *n1, uint32_t *n2) {
     if (!p || !n1 || !n2) TPT_FAIL(TPT_ERR_NULL_POINTER, "tpt_grav_plan_dims: NULL pointer");
     if (p->precision == TPT_PRECISION_FP32) {
-        *n1 = p->fft.jobs_host[0].n1;
-        *n2 = p->fft.jobs_host[0].n2;
+        *n1 = p->fft.jobs_host[0].ax.n;
+        *n2 = p->fft.jobs_host[0].ay.n;
     } else {
         p->dft->dims(0, n1, n2);
     }
@@ -316,7 +316,7 @@ static int grav_solve_any(tpt_grav_plan *p, const int32_t *mi, const float *mf, 
     if (!p) TPT_FAIL(TPT_ERR_NULL_POINTER, "gravity plan is NULL");
     if ((!mi && !mf) || !mask || !gx || !gy) TPT_FAIL(TPT_ERR_NULL_POINTER, "gravity solve: NULL grid pointer");
     if (p->precision == TPT_PRECISION_FP32) {
-        gfft::JobIO io{mi, mf, mask, gx, gy, inv, 1};
+        gfft::JobIO io{mi, mf, mask, gx, gy, inv};
         return p->fft.launch((cudaStream_t)stream, &io);
     }
     dft::SolveIO io{mi, mf, mask, gx, gy, inv, p->X};

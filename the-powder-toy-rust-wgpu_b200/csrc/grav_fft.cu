@@ -1,405 +1,475 @@
 // grav_fft.cu -- kernels and plan of the FP32 FFT gravity solve; see
-// grav_fft.cuh for the algorithm.
+// grav_fft.cuh for the algorithm and grav_fft_mixed.cuh for the transforms.
 #include <math.h>
 
 #include <algorithm>
 #include <vector>
 
 #include "grav_fft.cuh"
-#include "grav_fft_warp.cuh"
+#include "grav_fft_mixed.cuh"
 #include "grav_plan.hpp"
 
 namespace tpt {
 namespace gfft {
 
-constexpr int NT = 256;
+// Threads per block, and the blocks per SM the registers are capped for (80
+// registers). What bounds the passes at this size is latency: a block's chain
+// of loads (job, grid, twiddles), barriers and instruction fetch, at 24 warps
+// per SM and 16 to 55% of the issue slots; DRAM stays below 15% of its rate.
+// Measured on B200, solve of 256 grids (8.1 M cells, sides 32 to 512):
+// 0.407 ms (0.988 ms with one warp per transform, padded to powers of two and
+// exchanged by lane shuffles); one 400x225 grid 22.6 us (55.3); one 1200x701
+// grid 90 us (698 us with radix-2 passes in shared memory). Blocks of about
+// 2048 row points and 4096 column points: 1024 and 1024 took 0.554 ms, 2048
+// and 2048 0.479, 4096 and 4096 0.464, 8192 and 4096 0.509 (before the grid
+// addresses were hoisted out of the radix loops, at 0.456).
+constexpr int NT = 128, NT_LARGE = 256, MIN_BLOCKS = 3;
+// Columns whose two buffers stay below this run in blocks of NT threads, eight
+// to an SM; the larger ones in their own launch, in blocks of NT_LARGE, so
+// that the smaller ones are not held to the larger ones' three blocks per SM.
+constexpr size_t COL_SMEM_SMALL = 28 * 1024;
 
-// ---- per-solve kernels (FP32) ---------------------------------------------
-__global__ void __launch_bounds__(NT) rows_forward(const Job *__restrict__ jobs, const BlockRef *__restrict__ refs,
-                                                   const JobIO io) {
-    extern __shared__ float2 sm2[];
-    const BlockRef r = refs[blockIdx.x];
-    const Job J = load_job(jobs, r.job, io);
-    const uint32_t y = r.item;
-    for (uint32_t i = threadIdx.x; i < J.n1; i += NT) sm2[i] = make_float2(0.f, 0.f);
-    __syncthreads();
-    for (uint32_t x = threadIdx.x; x < J.X; x += NT) {
-        size_t c = (size_t)y * J.pitch + x;
-        float v = 0.0f;
-        if (__ldg(J.mask + c) != 0u) v = J.mass_f ? __ldg(J.mass_f + c) : (float)__ldg(J.mass_i + c) * J.mass_scale_inv;
-        sm2[bitrev(x, J.l1)] = make_float2(v, 0.f);
+extern __shared__ float2 fft_smem[];
+
+// The block's job in shared memory, copied word by word by the block's
+// threads: from the table, or (a one-job call) from the kernel's parameters
+// with the call's own pointers, which spares two dependent loads.
+static_assert(sizeof(Job) % 4 == 0 && sizeof(Job) / 4 <= NT, "one word per thread");
+__device__ __forceinline__ const Job &stage_job(const Job *jobs, const BlockRef *refs, const Job &one, uint32_t per_block,
+                                                uint32_t &item) {
+    __shared__ __align__(16) uint32_t words[sizeof(Job) / 4];
+    uint32_t j = 0;
+    if (jobs != nullptr) {
+        const BlockRef r = refs[blockIdx.x];
+        j = r.job;
+        item = r.item;
+    } else {
+        item = blockIdx.x * per_block;
     }
+    const uint32_t *src = reinterpret_cast<const uint32_t *>(jobs != nullptr ? jobs + j : &one);
+    if (threadIdx.x < sizeof(Job) / 4) words[threadIdx.x] = src[threadIdx.x];
     __syncthreads();
-    fft_dit(sm2, (int)J.n1, J.l1, 1, J.tw1, false);
-    float2 *dst = J.work + (size_t)y * J.n1;
-    for (uint32_t k = threadIdx.x; k < J.n1; k += NT) dst[k] = sm2[k];
+    return *reinterpret_cast<const Job *>(words);
 }
 
-// `cb` columns per block (power of two dividing n1).
-__global__ void __launch_bounds__(NT) cols_convolve(const Job *__restrict__ jobs, const BlockRef *__restrict__ refs,
-                                                    int cb) {
-    extern __shared__ float2 sm2[];
-    const BlockRef r = refs[blockIdx.x];
-    const Job J = jobs[r.job];
-    const uint32_t c0 = r.item, n1 = J.n1, n2 = J.n2;
-    float2 *P = sm2, *Q = sm2 + (size_t)cb * n2;
-    for (uint32_t i = threadIdx.x; i < (uint32_t)cb * n2; i += NT) P[i] = make_float2(0.f, 0.f);
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < J.Y * (uint32_t)cb; i += NT) {
-        uint32_t j = i / cb, col = i - j * cb;
-        P[(size_t)col * n2 + bitrev(j, J.l2)] = J.work[(size_t)j * n1 + c0 + col];
-    }
-    __syncthreads();
-    fft_dit(P, (int)n2, J.l2, cb, J.tw2, false);
-    for (uint32_t i = threadIdx.x; i < n2 * (uint32_t)cb; i += NT) {
-        uint32_t k = i / cb, col = i - k * cb;
-        size_t s = (size_t)col * n2 + k, g = (size_t)k * n1 + c0 + col;
-        float2 p = P[s];
-        Q[s] = cmul(p, __ldg(J.ky + g));
-        P[s] = cmul(p, __ldg(J.kx + g));
-    }
-    __syncthreads();
-    fft_dif(P, (int)n2, J.l2, 2 * cb, J.tw2, true);
-    float2 *sx = J.spec, *sy = J.spec + (size_t)J.Y * n1;
-    for (uint32_t i = threadIdx.x; i < J.Y * (uint32_t)cb; i += NT) {
-        uint32_t j = i / cb, col = i - j * cb;
-        size_t s = (size_t)col * n2 + bitrev(j, J.l2), g = (size_t)j * n1 + c0 + col;
-        sx[g] = P[s];
-        sy[g] = Q[s];
-    }
+// Programmatic dependent launch: the next pass's blocks are launched as this
+// one's drain, stage their job, and wait here for its results.
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// ---- the three passes ------------------------------------------------------------
+// One function per radix and step: blocks of all lengths share them.
+template <int R, bool INV> __device__ __noinline__ void row_step2(const Axis &A, uint32_t cnt) {
+    step2<R, INV>(fft_smem, A, RowSeq{}, cnt);
+}
+template <int R, bool INV> __device__ __noinline__ void col_step2(float2 *S, const Axis &A, uint32_t lc) {
+    step2<R, INV>(S, A, ColSeq{lc}, 1u << lc);
 }
 
-__global__ void __launch_bounds__(NT) rows_inverse(const Job *__restrict__ jobs, const BlockRef *__restrict__ refs,
-                                                   const JobIO io) {
-    extern __shared__ float2 sm2[];
-    const BlockRef r = refs[blockIdx.x];
-    const Job J = load_job(jobs, r.job, io);
-    const uint32_t field = r.item / J.Y, y = r.item - field * J.Y;
-    const float2 *src = J.spec + ((size_t)field * J.Y + y) * J.n1;
-    for (uint32_t k = threadIdx.x; k < J.n1; k += NT) sm2[k] = src[k];
-    __syncthreads();
-    fft_dif(sm2, (int)J.n1, J.l1, 1, J.tw1, true);
-    float *out = field ? J.gy : J.gx;
-    for (uint32_t x = threadIdx.x; x < J.X; x += NT) {
-        size_t c = (size_t)y * J.pitch + x;
-        out[c] = __ldg(J.mask + c) != 0u ? sm2[bitrev(x, J.l1)].x : 0.0f;
-    }
-}
-
-// ---- the warp form: one warp per 1-D transform ---------------------------------
-// 128-thread CTAs: the kernels hold a whole transform per warp in registers,
-// so CTAs of four warps let several share an SM where CTAs of eight warps left
-// registers unused (C4 solve 1.36 -> 1.06 ms). The register caps trade a few
-// spills for more resident warps: forward rows 6 CTAs per SM (80 registers),
-// columns 4 (128), inverse rows 5 (96); uncapped (91, 168, 158 registers: 5,
-// 3, 3 CTAs) the C4 solve took 1.074 ms per tick, capped 0.988 ms.
-constexpr int NTW = 128;
-constexpr int WARPS = NTW / 32;
-
-// Forward transform of mass row y (real, zero beyond X and where the mask is
-// clear), stored in the warp FFT's permuted order.
-template <int M> __device__ __forceinline__ void row_fwd_warp(const Job &J, uint32_t y, int lane) {
-    float2 v[M];
+// Row pairs y = 2 p, 2 p + 1 (p0 <= p < p0 + cnt) as z = m[2p] + i m[2p+1].
+template <int R> __device__ __noinline__ void rows_load(const Job &J, uint32_t p0, uint32_t cnt) {
+    const uint32_t m = J.ax.m, X = J.X, Y = J.Y, pitch = J.pitch;
+    const bool real = J.mass_f != nullptr;
+    const uint32_t *mask = J.mask, *mass = real ? (const uint32_t *)J.mass_f : (const uint32_t *)J.mass_i;
+    const float inv = J.mass_scale_inv;
+    step1<R>(fft_smem, J.ax, RowSeq{}, cnt, [&](uint32_t c, uint32_t j, float2(&v)[R]) {
+        const uint32_t y = 2u * (p0 + c);
+        const bool two = y + 1u < Y;
+        const size_t o = (size_t)y * pitch + j;
+        const uint32_t *mk = mask + o, *ms = mass + o, *mk1 = two ? mk + pitch : mk, *ms1 = two ? ms + pitch : ms;
+        // mask and mass are requested together, not one after the other's test
+        uint32_t on[R], on1[R], raw[R], raw1[R];
 #pragma unroll
-    for (int j1 = 0; j1 < M; ++j1) {
-        const uint32_t x = 32u * j1 + lane;
-        float m = 0.0f;
-        if (x < J.X) {
-            const size_t c = (size_t)y * J.pitch + x;
-            if (__ldg(J.mask + c) != 0u) m = J.mass_f ? __ldg(J.mass_f + c) : (float)__ldg(J.mass_i + c) * J.mass_scale_inv;
+        for (int a = 0; a < R; ++a) {
+            const bool in = j + m * a < X;
+            on[a] = in ? __ldg(mk + m * a) : 0u;
+            raw[a] = in ? __ldg(ms + m * a) : 0u;
+            on1[a] = in && two ? __ldg(mk1 + m * a) : 0u;
+            raw1[a] = in ? __ldg(ms1 + m * a) : 0u;
         }
-        v[j1] = make_float2(m, 0.0f);
-    }
-    WarpFft<M>::forward(v, J.tw1, lane);
-    float2 *dst = J.work + (size_t)y * J.n1;
 #pragma unroll
-    for (int k = 0; k < M; ++k) dst[32 * k + lane] = v[k];
+        for (int a = 0; a < R; ++a) {
+            const float f0 = real ? __uint_as_float(raw[a]) : (float)(int32_t)raw[a] * inv;
+            const float f1 = real ? __uint_as_float(raw1[a]) : (float)(int32_t)raw1[a] * inv;
+            v[a] = make_float2(on[a] != 0u ? f0 : 0.0f, on1[a] != 0u ? f1 : 0.0f);
+        }
+    });
 }
-
-__global__ void __launch_bounds__(NTW, 6) rows_forward_w(const Job *__restrict__ jobs, const BlockRef *__restrict__ refs,
-                                                     uint32_t nrefs, const JobIO io) {
-    const uint32_t w = blockIdx.x * WARPS + threadIdx.x / 32;
-    if (w >= nrefs) return;
-    const int lane = threadIdx.x & 31;
-    const BlockRef r = refs[w];
-    const Job J = load_job(jobs, r.job, io);
-    switch (J.n1 >> 5) {
-        case 1: row_fwd_warp<1>(J, r.item, lane); break;
-        case 2: row_fwd_warp<2>(J, r.item, lane); break;
-        case 4: row_fwd_warp<4>(J, r.item, lane); break;
-        case 8: row_fwd_warp<8>(J, r.item, lane); break;
-        case 16: row_fwd_warp<16>(J, r.item, lane); break;
-        case 32: row_fwd_warp<32>(J, r.item, lane); break;
-        default: break;
+template <int R> __device__ __noinline__ void rows_last(const Job &J, uint32_t cnt) {
+    const Axis &A = J.ax;
+    for (uint32_t it = threadIdx.x; it < cnt * A.q; it += blockDim.x) {
+        uint32_t c, q;
+        RowSeq{}.split(it, A.q, A.div_q, c, q);
+        const float2 *t;
+        float2 *o = RowSeq{}.at(fft_smem, A, c, item_pos(A, q, t));
+        float2 w[R];
+#pragma unroll
+        for (int i = 0; i < R; ++i) w[i] = o[i];
+        dft<R>(w);
+#pragma unroll
+        for (int i = 0; i < R; ++i) o[i] = w[i];
     }
 }
 
-// The mass and the kernels are real, so the x spectrum of every row is
-// Hermitian: column n1 - kx of the convolved spectra is the conjugate of
-// column kx. Only the n1/2 + 1 columns with kx <= n1/2 are convolved; in the
-// warp FFT's storage order they are the even lanes' positions plus position 1
-// (kx = n1/2). Half-column index h maps to its storage column:
-__device__ __forceinline__ uint32_t half_col(uint32_t h, uint32_t m1) {
-    return h < 16u * m1 ? (h >> 4) * 32u + 2u * (h & 15u) : 1u;
+// With Z the transform of z, the rows' spectra are (Z[k] + conj Z[n-k]) / 2
+// and -i (Z[k] - conj Z[n-k]) / 2; their halves k <= n/2 go to `work`.
+__global__ void __launch_bounds__(NT_LARGE, MIN_BLOCKS) k_rows_forward(const Job *jobs, const BlockRef *refs,
+                                                             const __grid_constant__ Job one) {
+    uint32_t p0;
+    const Job &J = stage_job(jobs, refs, one, one.rows_f, p0);
+    pdl_release();
+    const Axis &A = J.ax;
+    const uint32_t cnt = min(J.rows_f, (J.Y + 1) / 2 - p0);
+    with_radix(A.r1, [&](auto R) { rows_load<decltype(R)::value>(J, p0, cnt); });
+    __syncthreads();
+    if (A.r2 > 1) {
+        with_radix(A.r2, [&](auto R) { row_step2<decltype(R)::value, false>(A, cnt); });
+        __syncthreads();
+    }
+    with_radix(A.r3, [&](auto R) { rows_last<decltype(R)::value>(J, cnt); });
+    __syncthreads();
+    // k = q + Q k3 and n - k: item Q - q, element R3 - 1 - k3 (q = 0: item 0, element R3 - k3 mod R3)
+    const uint32_t nh = J.nh, nhp = J.nhp, Y = J.Y;
+    for (uint32_t it = threadIdx.x; it < cnt * A.q; it += blockDim.x) {
+        uint32_t c, q;
+        RowSeq{}.split(it, A.q, A.div_q, c, q);
+        const float2 *t;
+        const float2 *za = RowSeq{}.at(fft_smem, A, c, item_pos(A, q, t));
+        const float2 *zb = RowSeq{}.at(fft_smem, A, c, item_pos(A, q ? A.q - q : 0u, t)) + (q ? A.r3 - 1u : 0u);
+        const uint32_t y = 2u * (p0 + c);
+        float2 *o = J.work + (size_t)y * nhp + q;
+        for (uint32_t i = 0; q + A.q * i < nh; ++i, ++za, o += A.q) {
+            const float2 a = *za, b = *zb;
+            o[0] = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
+            if (y + 1 < Y) o[nhp] = make_float2(0.5f * (a.y + b.y), 0.5f * (b.x - a.x));
+            zb = q || i ? zb - 1 : zb + (A.r3 - 1u);
+        }
+    }
 }
 
-// One column (storage column c of the row spectra): forward transform down
-// the column, product with each field's kernel spectrum, inverse transform;
-// the Y rows both fields need are left in tx / ty (shared memory). tx holds
-// the column's input before; fs (n2 entries, the same memory as ty) holds the
-// forward spectrum while the two products are taken, in the lane order the
-// registers use, so each lane reads back only what it wrote and the y field's
-// rows overwrite only entries their own lane has read. The two fields share
-// one copy of the inverse transform's code (a loop that is not unrolled).
-template <int M>
-__device__ __forceinline__ void col_warp(const Job &J, uint32_t c, float2 *tx, float2 *fs, int lane) {
-    float2 g[M];
+template <int R> __device__ __noinline__ void cols_load(const Job &J, uint32_t h0, uint32_t lc) {
+    const float2 *work = J.work + h0;
+    const uint32_t Y = J.Y, nhp = J.nhp, left = J.nh - h0;
+    const uint32_t m = J.ay.m;
+    const size_t stride = (size_t)m * nhp;
+    step1<R>(fft_smem, J.ay, ColSeq{lc}, 1u << lc, [&](uint32_t c, uint32_t j, float2(&v)[R]) {
+        const float2 *p = work + (size_t)j * nhp + c;
+        const uint32_t rows = c < left ? Y : 0u;
 #pragma unroll
-    for (int j1 = 0; j1 < M; ++j1) {
-        const uint32_t j = 32u * j1 + lane;
-        g[j1] = j < J.Y ? tx[j] : make_float2(0.0f, 0.0f);
-    }
-    WarpFft<M>::forward(g, J.tw2, lane);
+        for (int a = 0; a < R; ++a) v[a] = j + m * a < rows ? __ldg(p + a * stride) : make_float2(0.0f, 0.0f);
+    });
+}
+// Step 3, the two products and the inverses' first step. The spectrum of a
+// column stays in each item's own places while its products are inverted, the
+// first into the second buffer, the second in place.
+template <int R> __device__ __noinline__ void cols_products(const Job &J, uint32_t h0, uint32_t lc, float2 *S2) {
+    const Axis &A = J.ay;
+    const ColSeq sq{lc};
+    const uint32_t st = sq.step(1), nhp = J.nhp;
+    for (uint32_t it = threadIdx.x; it < A.q << lc; it += blockDim.x) {
+        uint32_t c, q;
+        sq.split(it, 0, 0, c, q);
+        if (h0 + c >= J.nh) continue;
+        const float2 *t;
+        const uint32_t pos = item_pos(A, q, t);
+        float2 *o = sq.at(fft_smem, A, c, pos);
+        const float2 *kern = J.kern + (size_t)q * nhp + h0 + c;
+        const size_t kstep = (size_t)A.q * nhp;
+        float2 w[R];
 #pragma unroll
-    for (int k = 0; k < M; ++k) fs[32 * k + lane] = g[k];
-    __syncwarp();
+        for (int i = 0; i < R; ++i) w[i] = o[i * st];
+        dft<R>(w);
+#pragma unroll
+        for (int i = 0; i < R; ++i) o[i * st] = w[i];
 #pragma unroll 1
-    for (int f = 0; f < 2; ++f) {
-        const float2 *kf = (f ? J.ky : J.kx) + (size_t)c * J.n2;
+        for (int f = 0; f < 2; ++f) {
+            const float sgn = f ? 1.0f : -1.0f;
 #pragma unroll
-        for (int k = 0; k < M; ++k) g[k] = cmulf(fs[32 * k + lane], __ldg(kf + 32 * k + lane));
-        WarpFft<M>::inverse(g, J.tw2, lane);
-        float2 *dst = f ? fs : tx;
-#pragma unroll
-        for (int j1 = 0; j1 < M; ++j1) {
-            const uint32_t j = 32u * j1 + lane;
-            if (j < J.Y) dst[j] = g[j1];
+            for (int i = 0; i < R; ++i) {
+                const float2 k = __ldg(kern + i * kstep), s = o[i * st];
+                const float b = sgn * k.y;
+                w[i] = make_float2(s.x * b - s.y * k.x, s.x * k.x + s.y * b);
+            }
+            unstep3<R>(f ? o : sq.at(S2, A, c, pos), st, t, w);
         }
     }
 }
+template <int R> __device__ __noinline__ void cols_store(const Job &J, uint32_t h0, uint32_t lc, float2 *S, float2 *out) {
+    const uint32_t Y = J.Y, nhp = J.nhp, left = J.nh - h0, m = J.ay.m;
+    const size_t stride = (size_t)m * nhp;
+    out += h0;
+    unstep1<R>(S, J.ay, ColSeq{lc}, 1u << lc, [&](uint32_t c, uint32_t j, const float2(&v)[R]) {
+        float2 *p = out + (size_t)j * nhp + c;
+        const uint32_t rows = c < left ? Y : 0u;
+#pragma unroll
+        for (int a = 0; a < R; ++a)
+            if (j + m * a < rows) p[a * stride] = v[a];
+    });
+}
 
-// A block takes WARPS consecutive half-column indices of one job: the Y x
-// WARPS tile is staged through shared memory (each row's columns lie within
-// 2 * WARPS consecutive positions), each warp transforms one column, and both
-// fields' Y x WARPS tiles go back the same way. Per warp: `ystride` entries of
-// the x field tile, `fstride` (>= n2) of the spectrum stash / y field tile.
-__global__ void __launch_bounds__(NTW, 4) cols_convolve_w(const Job *__restrict__ jobs, const BlockRef *__restrict__ refs,
-                                                      uint32_t ystride, uint32_t fstride) {
-    extern __shared__ float2 sm2[];
-    const BlockRef r = refs[blockIdx.x];
-    const Job J = jobs[r.job];
-    const uint32_t h0 = r.item, n1 = J.n1, Y = J.Y, m1 = n1 >> 5, nh = n1 / 2 + 1;
-    float2 *TX = sm2, *TY = sm2 + (size_t)WARPS * ystride;
-    for (uint32_t i = threadIdx.x; i < Y * WARPS; i += NTW) {
-        const uint32_t j = i / WARPS, col = i - j * WARPS;
-        if (h0 + col < nh) TX[(size_t)col * ystride + j] = J.work[(size_t)j * n1 + half_col(h0 + col, m1)];
-    }
+// 1 << lc columns of the half spectrum from h0.
+__global__ void __launch_bounds__(NT_LARGE, MIN_BLOCKS) k_columns(const Job *jobs, const BlockRef *refs,
+                                                             const __grid_constant__ Job one) {
+    uint32_t h0;
+    const Job &J = stage_job(jobs, refs, one, 1u << one.lc, h0);
+    pdl_release();
+    const Axis &A = J.ay;
+    const uint32_t lc = J.lc;
+    float2 *S2 = fft_smem + ((size_t)A.sz << lc);
+    pdl_wait();
+    with_radix(A.r1, [&](auto R) { cols_load<decltype(R)::value>(J, h0, lc); });
     __syncthreads();
-    const int wi = threadIdx.x / 32, lane = threadIdx.x & 31;
-    float2 *tx = TX + (size_t)wi * ystride, *ty = TY + (size_t)wi * fstride;
-    if (h0 + wi < nh) {
-        const uint32_t c = half_col(h0 + wi, m1);
-        switch (J.n2 >> 5) {
-            case 1: col_warp<1>(J, c, tx, ty, lane); break;
-            case 2: col_warp<2>(J, c, tx, ty, lane); break;
-            case 4: col_warp<4>(J, c, tx, ty, lane); break;
-            case 8: col_warp<8>(J, c, tx, ty, lane); break;
-            case 16: col_warp<16>(J, c, tx, ty, lane); break;
-            case 32: col_warp<32>(J, c, tx, ty, lane); break;
-            default: break;
-        }
+    if (A.r2 > 1) {
+        with_radix(A.r2, [&](auto R) { col_step2<decltype(R)::value, false>(fft_smem, A, lc); });
+        __syncthreads();
     }
+    with_radix(A.r3, [&](auto R) { cols_products<decltype(R)::value>(J, h0, lc, S2); });
     __syncthreads();
-    float2 *sx = J.spec, *sy = J.spec + (size_t)Y * n1;
-    for (uint32_t i = threadIdx.x; i < Y * WARPS; i += NTW) {
-        const uint32_t j = i / WARPS, col = i - j * WARPS;
-        if (h0 + col >= nh) continue;
-        const size_t g = (size_t)j * n1 + half_col(h0 + col, m1);
-        sx[g] = TX[(size_t)col * ystride + j];
-        sy[g] = TY[(size_t)col * fstride + j];
+    if (A.r2 > 1) {
+#pragma unroll 1
+        for (int f = 0; f < 2; ++f)
+            with_radix(A.r2, [&](auto R) { col_step2<decltype(R)::value, true>(f ? fft_smem : S2, A, lc); });
+        __syncthreads();
     }
+#pragma unroll 1
+    for (int f = 0; f < 2; ++f)
+        with_radix(A.r1, [&](auto R) {
+            cols_store<decltype(R)::value>(J, h0, lc, f ? fft_smem : S2, J.spec + (f ? (size_t)J.Y * J.nhp : 0));
+        });
 }
 
-// Inverse transform of spectrum row y of both fields at once: both outputs
-// are real, so gx + i gy is the inverse of Sx + i Sy. The full row spectra
-// are rebuilt from the convolved half: position p of the permuted order holds
-// frequency kx; an odd lane's position (except kx = n1/2) holds kx > n1/2,
-// whose value is the conjugate of the stored kx' = n1 - kx. Outputs: the first
-// X, masked.
-template <int M> __device__ __forceinline__ void row_inv_warp(const Job &J, uint32_t y, int lane) {
-    const float2 *rx = J.spec + (size_t)y * J.n1, *ry = J.spec + ((size_t)J.Y + y) * J.n1;
-    float2 v[M];
+template <int R> __device__ __noinline__ void rows_first(const Job &J, uint32_t y0, uint32_t cnt) {
+    const Axis &A = J.ax;
+    const size_t nhp = J.nhp, mirror = (size_t)J.Y * nhp;  // the second plane
+    for (uint32_t it = threadIdx.x; it < cnt * A.q; it += blockDim.x) {
+        uint32_t c, q;
+        RowSeq{}.split(it, A.q, A.div_q, c, q);
+        const float2 *t, *row = J.spec + (y0 + c) * nhp;
+        float2 *o = RowSeq{}.at(fft_smem, A, c, item_pos(A, q, t));
+        // frequency q + Q i: stored up to n/2 (Q R / 2), else as its mirror's
+        // conjugate; with an odd radix the middle element depends on q
+        const float2 *lo = row + q, *hi = row + mirror + (A.n - q);
+        float2 w[R];
 #pragma unroll
-    for (int k1 = 0; k1 < M; ++k1) {
-        const bool direct = (lane & 1) == 0 || (k1 == 0 && lane == 1);
-        uint32_t p = 32u * k1 + lane;
-        if (!direct) {
-            const uint32_t kx = (uint32_t)k1 + (uint32_t)M * (uint32_t)brev_c(lane, 5);
-            const uint32_t km = J.n1 - kx;
-            p = (km % (uint32_t)M) * 32u + (__brev(km / (uint32_t)M) >> 27);
+        for (int i = 0; i < R; ++i) {
+            const bool direct = R % 2 == 1 && i == R / 2 ? 2u * (q + A.q * i) <= A.n : i < (R + 1) / 2;
+            w[i] = __ldg(direct ? lo + A.q * i : hi - A.q * i);
+            if (!direct) w[i].y = -w[i].y;
         }
-        float2 sx = rx[p], sy = ry[p];
-        if (!direct) {
-            sx.y = -sx.y;
-            sy.y = -sy.y;
-        }
-        v[k1] = make_float2(sx.x - sy.y, sx.y + sy.x);  // sx + i sy
+        unstep3<R>(o, 1, t, w);
     }
-    WarpFft<M>::inverse(v, J.tw1, lane);
+}
+template <int R> __device__ __noinline__ void rows_store(const Job &J, uint32_t y0, uint32_t cnt) {
+    const uint32_t X = J.X, m = J.ax.m, pitch = J.pitch;
+    const uint32_t *mask = J.mask;
+    float *gx = J.gx, *gy = J.gy;
+    unstep1<R>(fft_smem, J.ax, RowSeq{}, cnt, [&](uint32_t c, uint32_t j, const float2(&v)[R]) {
+        const size_t r = (size_t)(y0 + c) * pitch + j;
+        const uint32_t *mk = mask + r;
+        float *px = gx + r, *py = gy + r;
+        uint32_t on[R];
 #pragma unroll
-    for (int j1 = 0; j1 < M; ++j1) {
-        const uint32_t x = 32u * j1 + lane;
-        if (x < J.X) {
-            const size_t c = (size_t)y * J.pitch + x;
-            const bool on = __ldg(J.mask + c) != 0u;
-            J.gx[c] = on ? v[j1].x : 0.0f;
-            J.gy[c] = on ? v[j1].y : 0.0f;
-        }
-    }
+        for (int a = 0; a < R; ++a) on[a] = j + m * a < X ? __ldg(mk + m * a) : 0u;
+#pragma unroll
+        for (int a = 0; a < R; ++a)
+            if (j + m * a < X) {
+                px[m * a] = on[a] != 0u ? v[a].x : 0.0f;
+                py[m * a] = on[a] != 0u ? v[a].y : 0.0f;
+            }
+    });
 }
 
-__global__ void __launch_bounds__(NTW, 5) rows_inverse_w(const Job *__restrict__ jobs, const BlockRef *__restrict__ refs,
-                                                     uint32_t nrefs, const JobIO io) {
-    const uint32_t w = blockIdx.x * WARPS + threadIdx.x / 32;
-    if (w >= nrefs) return;
-    const int lane = threadIdx.x & 31;
-    const BlockRef r = refs[w];
-    const Job J = load_job(jobs, r.job, io);
-    switch (J.n1 >> 5) {
-        case 1: row_inv_warp<1>(J, r.item, lane); break;
-        case 2: row_inv_warp<2>(J, r.item, lane); break;
-        case 4: row_inv_warp<4>(J, r.item, lane); break;
-        case 8: row_inv_warp<8>(J, r.item, lane); break;
-        case 16: row_inv_warp<16>(J, r.item, lane); break;
-        case 32: row_inv_warp<32>(J, r.item, lane); break;
-        default: break;
+// Rows y0 .. of gx + i gy, masked.
+__global__ void __launch_bounds__(NT_LARGE, MIN_BLOCKS) k_rows_inverse(const Job *jobs, const BlockRef *refs,
+                                                             const __grid_constant__ Job one) {
+    uint32_t y0;
+    const Job &J = stage_job(jobs, refs, one, one.rows_i, y0);
+    const Axis &A = J.ax;
+    const uint32_t cnt = min(J.rows_i, J.Y - y0);
+    pdl_wait();
+    with_radix(A.r3, [&](auto R) { rows_first<decltype(R)::value>(J, y0, cnt); });
+    __syncthreads();
+    if (A.r2 > 1) {
+        with_radix(A.r2, [&](auto R) { row_step2<decltype(R)::value, true>(A, cnt); });
+        __syncthreads();
     }
-}
-
-// Kernel spectra from the natural order (row ky, column kx) into the warp
-// form's layout: storage column c (frequency kx of permuted position c along
-// x), then permuted position p along y.
-__global__ void permute_spectrum(const float2 *__restrict__ nat, float2 *__restrict__ out, uint32_t n1, uint32_t n2) {
-    const size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= (size_t)n1 * n2) return;
-    const uint32_t c = (uint32_t)(id / n2), p = (uint32_t)(id - (size_t)c * n2);
-    const uint32_t m1 = n1 / 32, m2 = n2 / 32;
-    const uint32_t kx = (c / 32) + m1 * (uint32_t)brev_c((int)(c % 32), 5);
-    const uint32_t ky = (p / 32) + m2 * (uint32_t)brev_c((int)(p % 32), 5);
-    out[id] = nat[(size_t)ky * n1 + kx];
+    with_radix(A.r1, [&](auto R) { rows_store<decltype(R)::value>(J, y0, cnt); });
 }
 
 // ---- kernel spectra, FP64 (once per plan) ---------------------------------
+// One length-n transform per block in shared memory (natural order in and
+// out), Stockham passes of the radices 2, 3, 4 and 5; tw[k] = exp(-2 pi i k / n).
+template <int R>
+__device__ __forceinline__ void stockham_pass(const double2 *a, double2 *b, int n, int ns, const double2 *__restrict__ tw) {
+    const int step = n / R, tstep = n / (ns * R);
+    for (int j = threadIdx.x; j < step; j += blockDim.x) {
+        const int p = j % ns;
+        double2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const double2 w = __ldg(tw + p * r * tstep), x = a[j + r * step];
+            v[r] = make_double2(x.x * w.x - x.y * w.y, x.x * w.y + x.y * w.x);
+        }
+        double2 *o = b + (j - p) * R + p;
+#pragma unroll
+        for (int k = 0; k < R; ++k) {
+            double2 s = v[0];
+#pragma unroll
+            for (int r = 1; r < R; ++r) {
+                const double2 w = __ldg(tw + (r * k % R) * step);
+                s.x += v[r].x * w.x - v[r].y * w.y;
+                s.y += v[r].x * w.y + v[r].y * w.x;
+            }
+            o[k * ns] = s;
+        }
+    }
+}
+// Returns the buffer that holds the result; ends after a barrier.
+__device__ double2 *stockham_f64(double2 *a, double2 *b, int n, const double2 *__restrict__ tw) {
+    int rest = n;
+    for (int ns = 1; rest > 1;) {
+        const int R = rest % 4 == 0 ? 4 : rest % 2 == 0 ? 2 : rest % 3 == 0 ? 3 : 5;
+        if (R == 4) stockham_pass<4>(a, b, n, ns, tw);
+        else if (R == 2) stockham_pass<2>(a, b, n, ns, tw);
+        else if (R == 3) stockham_pass<3>(a, b, n, ns, tw);
+        else stockham_pass<5>(a, b, n, ns, tw);
+        __syncthreads();
+        double2 *t = a;
+        a = b;
+        b = t;
+        ns *= R;
+        rest /= R;
+    }
+    return a;
+}
+
 // build_kernel_field_kernel (crates/tpt-sim/src/gravity_gpu/fft.rs:208-237)
-// in double: K(d) = scale * d / |d|^3 with d folded into (-N/2, N/2].
-__global__ void kernel_field_f64(double2 *out, uint32_t n1, uint32_t n2, double scale) {
-    size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t cells = (size_t)n1 * n2;
-    if (id >= cells) return;
-    uint32_t px = (uint32_t)(id % n1), py = (uint32_t)(id / n1);
-    double dx = px, dy = py;
-    if (px * 2u >= n1) dx = (double)px - (double)n1;
-    if (py * 2u >= n2) dy = (double)py - (double)n2;
-    double vx = 0.0, vy = 0.0;
-    if (dx != 0.0 || dy != 0.0) {
-        double d = sqrt(dx * dx + dy * dy);
-        double inv = scale / (d * d * d);
-        vx = dx * inv;
-        vy = dy * inv;
-    }
-    out[id] = make_double2(vx, 0.0);
-    out[cells + id] = make_double2(vy, 0.0);
-}
-
-__global__ void spectrum_rows_f64(double2 *buf, uint32_t n1, uint32_t n2, int l1, const double2 *tw1) {
+// in double, one row: Kx + i Ky of K(d) = scale * d / |d|^3 with d folded into
+// (-N/2, N/2) (the offset N/2 left out), transformed along x.
+__global__ void spectrum_rows_f64(double2 *out, uint32_t n1, uint32_t n2, double scale, const double2 *tw1) {
     extern __shared__ double2 smd[];
-    const uint32_t row = blockIdx.x;  // field * n2 + y
-    double2 *src = buf + (size_t)row * n1;
-    for (uint32_t i = threadIdx.x; i < n1; i += blockDim.x) smd[bitrev(i, l1)] = src[i];
+    const uint32_t y = blockIdx.x;
+    const double dy = 2 * y < n2 ? (double)y : (double)y - (double)n2;
+    for (uint32_t i = threadIdx.x; i < n1; i += blockDim.x) {
+        const double dx = 2 * i < n1 ? (double)i : (double)i - (double)n1;
+        double2 v = make_double2(0.0, 0.0);
+        if (2 * i != n1 && 2 * y != n2 && (dx != 0.0 || dy != 0.0)) {
+            const double d = sqrt(dx * dx + dy * dy), inv = scale / (d * d * d);
+            v = make_double2(dx * inv, dy * inv);
+        }
+        smd[i] = v;
+    }
     __syncthreads();
-    fft_dit(smd, (int)n1, l1, 1, tw1, false);
-    for (uint32_t i = threadIdx.x; i < n1; i += blockDim.x) src[i] = smd[i];
+    const double2 *s = stockham_f64(smd, smd + n1, (int)n1, tw1);
+    for (uint32_t i = threadIdx.x; i < n1; i += blockDim.x) out[(size_t)y * n1 + i] = s[i];
 }
 
-__global__ void spectrum_cols_f64(const double2 *buf, uint32_t n1, uint32_t n2, int l2, const double2 *tw2,
-                                  double2 *out64, float2 *kx, float2 *ky) {
+// Column kx = blockIdx.x: the transform along y. Both fields' spectra are
+// purely imaginary, i a and i b, so that of Kx + i Ky is -b + i a.
+__global__ void spectrum_cols_f64(const double2 *rows, uint32_t n1, uint32_t n2, const double2 *tw2, float2 *kern,
+                                  uint32_t nhp) {
     extern __shared__ double2 smd[];
-    const uint32_t field = blockIdx.x / n1, c = blockIdx.x - field * n1;
-    const double2 *src = buf + (size_t)field * n1 * n2;
-    for (uint32_t j = threadIdx.x; j < n2; j += blockDim.x) smd[bitrev(j, l2)] = src[(size_t)j * n1 + c];
+    const uint32_t c = blockIdx.x;
+    for (uint32_t j = threadIdx.x; j < n2; j += blockDim.x) smd[j] = rows[(size_t)j * n1 + c];
     __syncthreads();
-    fft_dit(smd, (int)n2, l2, 1, tw2, false);
-    float2 *dst = field ? ky : kx;
-    for (uint32_t j = threadIdx.x; j < n2; j += blockDim.x) {
-        double2 v = smd[j];
-        if (out64) out64[(size_t)field * n1 * n2 + (size_t)j * n1 + c] = v;
-        if (dst) dst[(size_t)j * n1 + c] = make_float2((float)v.x, (float)v.y);
-    }
+    const double2 *s = stockham_f64(smd, smd + n2, (int)n2, tw2);
+    for (uint32_t j = threadIdx.x; j < n2; j += blockDim.x)
+        kern[(size_t)j * nhp + c] = make_float2((float)s[j].y, (float)-s[j].x);
 }
 
-// Twiddle table exp(-2 pi i k / n), k < n/2 (or k < n: `full`), evaluated in
-// double.
-template <typename T2> static std::vector<T2> twiddles(uint32_t n, bool full = false) {
-    std::vector<T2> t(std::max<uint32_t>(full ? n : n / 2, 1));
-    for (uint32_t k = 0; k < t.size(); ++k) {
-        double a = -2.0 * M_PI * (double)k / (double)n;
-        t[k].x = cos(a);
-        t[k].y = sin(a);
-    }
-    return t;
+// ---- lengths and tables --------------------------------------------------------
+// The axis of `cells` cells: the shortest even length that holds the linear
+// convolution, 2 cells - 1, as a product of two radices or else of three.
+// Neighbouring lengths lie within 1.25 of each other (1.07 on average above
+// 256), where padding to a power of two costs up to 2 in each direction.
+static bool axis_for(uint32_t cells, Axis *out) {
+    const uint32_t need = std::max<uint32_t>(2 * cells - 1, 32u);
+    Axis best{};
+    for (uint32_t r1 : kRadices)
+        for (uint32_t r2 = 1; r2 <= r1; ++r2) {
+            if (r2 > 1 && std::find(std::begin(kRadices), std::end(kRadices), r2) == std::end(kRadices)) continue;
+            for (uint32_t r3 : kRadices) {
+                const uint32_t n = r1 * r2 * r3;
+                if (r3 > r1 || n < need || n % 2) continue;
+                // ties: two radices before three, then the smallest sum
+                const bool better = best.n == 0 || n < best.n ||
+                                    (n == best.n && ((r2 == 1) != (best.r2 == 1) ? r2 == 1
+                                                                                 : r1 + r2 + r3 < best.r1 + best.r2 + best.r3));
+                if (better) {
+                    best.n = n;
+                    best.r1 = r1;
+                    best.r2 = r2;
+                    best.r3 = r3;
+                }
+            }
+        }
+    if (best.n == 0) return false;
+    auto magic = [](uint32_t d) { return (uint32_t)(((1ull << 32) + d - 1) / d); };
+    best.m = best.r2 * best.r3;
+    best.q = best.r1 * best.r2;
+    best.sr = best.r3 | 1u;
+    best.sb = (best.r2 * best.sr) | 1u;
+    best.sz = best.r1 * best.sb;
+    best.div_r1 = magic(best.r1);
+    best.div_r3 = magic(best.r3);
+    best.div_m = magic(best.m);
+    best.div_q = magic(best.q);
+    best.div_13 = magic(best.r1 * best.r3);
+    *out = best;
+    return true;
 }
 
-static int log2u(uint32_t n) {
-    int l = 0;
-    while ((1u << l) < n) ++l;
-    return l;
+// The axis's twiddles (layout: Axis::tw), evaluated in double.
+static void fill_twiddles(const Axis &a, std::vector<float2> &t) {
+    auto w = [](uint64_t k, uint32_t n) {
+        const double p = -2.0 * M_PI * (double)(k % n) / (double)n;
+        return make_float2((float)cos(p), (float)sin(p));
+    };
+    for (uint32_t k = 0; k < a.r1; ++k)
+        for (uint32_t j = 0; j < a.m; ++j) t.push_back(w((uint64_t)k * j, a.n));
+    if (a.r2 > 1)
+        for (uint32_t k = 0; k < a.r2; ++k)
+            for (uint32_t j = 0; j < a.r3; ++j) t.push_back(w((uint64_t)k * j, a.m));
 }
 
-uint32_t next_pow2(uint32_t v) {
-    uint32_t p = 1;
-    while (p < v) p <<= 1;
-    return p;
-}
-
-int col_block(uint32_t n2) {
-    int cb = 16;
-    while (cb > 1 && (size_t)cb * 2 * n2 * sizeof(float2) > 96 * 1024) cb >>= 1;
-    return cb;
-}
-
-int init_kernel_attrs() {
+static int init_kernel_attrs() {
     static bool done = false;
     if (done) return TPT_OK;
-    TPT_CUDA(cudaFuncSetAttribute(rows_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-    TPT_CUDA(cudaFuncSetAttribute(cols_convolve, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    TPT_CUDA(cudaFuncSetAttribute(rows_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-    TPT_CUDA(cudaFuncSetAttribute(spectrum_rows_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
-    TPT_CUDA(cudaFuncSetAttribute(spectrum_cols_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
-    TPT_CUDA(cudaFuncSetAttribute(cols_convolve_w, cudaFuncAttributeMaxDynamicSharedMemorySize, WARPS * (512 + 1024) * 8));
+    const int most = 227 * 1024;
+    const void *fns[] = {(const void *)k_rows_forward, (const void *)k_columns, (const void *)k_rows_inverse,
+                         (const void *)spectrum_rows_f64, (const void *)spectrum_cols_f64};
+    for (const void *f : fns) {
+        cudaFuncAttributes a{};
+        TPT_CUDA(cudaFuncGetAttributes(&a, f));
+        TPT_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes));
+    }
     done = true;
     return TPT_OK;
 }
 
-// Builds the FP64 kernel spectra of an n1 x n2 transform and stores them as
-// f32 (kx, ky) and/or keeps the f64 copy (out64: 2 x n2 x n1, may be null).
-// `scale` = -M_GRAV / (n1 * n2). Synchronous.
-int build_spectra(uint32_t n1, uint32_t n2, double scale, float2 *kx, float2 *ky, double2 *out64) {
-    int rc = init_kernel_attrs();
-    if (rc) return rc;
-    size_t cells = (size_t)n1 * n2;
+// Builds the kernel spectra of an n1 x n2 transform in FP64 and stores them
+// rounded. Synchronous.
+static int build_spectra(uint32_t n1, uint32_t n2, uint32_t nhp, float2 *kern) {
+    auto full_circle = [](uint32_t n) {
+        std::vector<double2> t(n);
+        for (uint32_t k = 0; k < n; ++k) {
+            const double a = -2.0 * M_PI * (double)k / (double)n;
+            t[k] = make_double2(cos(a), sin(a));
+        }
+        return t;
+    };
+    const double scale = -(double)6.673e-1f / ((double)n1 * (double)n2);
+    auto tw1 = full_circle(n1), tw2 = full_circle(n2);
     double2 *buf = nullptr, *t1 = nullptr, *t2 = nullptr;
-    auto tw1 = twiddles<double2>(n1), tw2 = twiddles<double2>(n2);
-    cudaError_t e = cudaMalloc(&buf, 2 * cells * sizeof(double2));
-    if (e == cudaSuccess) e = cudaMalloc(&t1, tw1.size() * sizeof(double2));
-    if (e == cudaSuccess) e = cudaMalloc(&t2, tw2.size() * sizeof(double2));
-    if (e == cudaSuccess) e = cudaMemcpy(t1, tw1.data(), tw1.size() * sizeof(double2), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(t2, tw2.data(), tw2.size() * sizeof(double2), cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMalloc(&buf, (size_t)n1 * n2 * sizeof(double2));
+    if (e == cudaSuccess) e = cudaMalloc(&t1, n1 * sizeof(double2));
+    if (e == cudaSuccess) e = cudaMalloc(&t2, n2 * sizeof(double2));
+    if (e == cudaSuccess) e = cudaMemcpy(t1, tw1.data(), n1 * sizeof(double2), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(t2, tw2.data(), n2 * sizeof(double2), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) {
-        kernel_field_f64<<<(unsigned)((cells + 255) / 256), 256>>>(buf, n1, n2, scale);
+        spectrum_rows_f64<<<n2, 256, 2 * n1 * sizeof(double2)>>>(buf, n1, n2, scale, t1);
         count_launch();
-        spectrum_rows_f64<<<2 * n2, 256, n1 * sizeof(double2)>>>(buf, n1, n2, log2u(n1), t1);
-        count_launch();
-        spectrum_cols_f64<<<2 * n1, 256, n2 * sizeof(double2)>>>(buf, n1, n2, log2u(n2), t2, out64, kx, ky);
+        spectrum_cols_f64<<<n1 / 2 + 1, 256, 2 * n2 * sizeof(double2)>>>(buf, n1, n2, t2, kern, nhp);
         count_launch();
         e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -412,177 +482,114 @@ int build_spectra(uint32_t n1, uint32_t n2, double scale, float2 *kx, float2 *ky
     return TPT_OK;
 }
 
-// The same spectra in the warp form's layout (permute_spectrum).
-int build_spectra_permuted(uint32_t n1, uint32_t n2, double scale, float2 *kx, float2 *ky) {
-    const size_t cells = (size_t)n1 * n2;
-    float2 *nat = nullptr;
-    TPT_CUDA(cudaMalloc(&nat, 2 * cells * sizeof(float2)));
-    int rc = build_spectra(n1, n2, scale, nat, nat + cells, nullptr);
-    if (rc == TPT_OK) {
-        const unsigned blocks = (unsigned)((cells + 255) / 256);
-        permute_spectrum<<<blocks, 256>>>(nat, kx, n1, n2);
-        count_launch();
-        permute_spectrum<<<blocks, 256>>>(nat + cells, ky, n1, n2);
-        count_launch();
-        cudaError_t e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaDeviceSynchronize();
-        if (e != cudaSuccess) {
-            set_error("gravity spectrum permutation failed: %s", cudaGetErrorString(e));
-            rc = TPT_ERR_CUDA;
-        }
-    }
-    cudaFree(nat);
-    return rc;
-}
-
 // ---- FFT gravity set (one plan or a batch) --------------------------------
 int FftSet::create(const std::vector<JobShape> &shapes) {
     int rc = init_kernel_attrs();
     if (rc) return rc;
     destroy();
     const size_t nj = shapes.size();
-    jobs_host.resize(nj);
-    warp = true;
-    for (const JobShape &sh : shapes)
-        if (next_pow2(2 * sh.X) > 1024u || next_pow2(2 * sh.Y) > 1024u) warp = false;
-    // padded lengths: next_pow2(2X) as the reference pads (gravity_gpu/mod.rs:
-    // 140-167), at least 32 in the warp form (any length >= 2X gives the same
-    // linear convolution)
-    auto pad = [&](uint32_t v) { return warp ? std::max<uint32_t>(32u, next_pow2(2 * v)) : next_pow2(2 * v); };
-    std::vector<BlockRef> rr, cr, ir;
-    size_t work_elems = 0, spec_elems = 0, kern_elems = 0;
-    std::vector<size_t> woff(nj), soff(nj), koff(nj);
-    std::vector<std::pair<uint32_t, uint32_t>> sizes;  // distinct (n1, n2)
-    std::vector<size_t> size_off;
+    jobs_host.assign(nj, Job{});
+    size_t work_elems = 0, kern_elems = 0;
+    std::vector<size_t> woff(nj), koff(nj);
+    struct Size {
+        uint32_t n1, n2;
+        bool lone;  // a single cell feels no force: a zero kernel, or the transforms' rounding would show
+        size_t off;
+    };
+    std::vector<Size> sizes;     // distinct kernels: the spectra depend on the lengths only
+    std::vector<uint32_t> lens;  // distinct lengths, their twiddle tables
+    std::vector<size_t> lens_off;
+    std::vector<float2> twh;
+    auto table = [&](const Axis &a) {
+        if (std::find(lens.begin(), lens.end(), a.n) != lens.end()) return;
+        lens.push_back(a.n);
+        lens_off.push_back(twh.size());
+        fill_twiddles(a, twh);
+    };
     for (size_t j = 0; j < nj; ++j) {
-        const JobShape &s = shapes[j];
-        uint32_t n1 = pad(s.X), n2 = pad(s.Y);
+        Job &J = jobs_host[j];
+        if (!axis_for(shapes[j].X, &J.ax) || !axis_for(shapes[j].Y, &J.ay))
+            TPT_FAIL(TPT_ERR_INVALID_DIMS, "gravity grid %ux%u exceeds the longest transform", shapes[j].X, shapes[j].Y);
+        J.X = J.pitch = shapes[j].X;
+        J.Y = shapes[j].Y;
+        J.nh = J.ax.n / 2 + 1;
+        J.nhp = (J.nh + 7) / 8 * 8;
+        J.mass_scale_inv = 1.0f / 65536.0f;
         woff[j] = work_elems;
-        work_elems += (size_t)s.Y * n1;
-        soff[j] = spec_elems;
-        spec_elems += (size_t)2 * s.Y * n1;
-        auto key = std::make_pair(n1, n2);
-        auto it = std::find(sizes.begin(), sizes.end(), key);
-        if (it == sizes.end()) {  // spectra depend on the padded size only
-            sizes.push_back(key);
-            size_off.push_back(kern_elems);
+        work_elems += (size_t)J.Y * J.nhp;
+        const bool lone = J.X == 1 && J.Y == 1;
+        auto it = std::find_if(sizes.begin(), sizes.end(),
+                               [&](const Size &s) { return s.n1 == J.ax.n && s.n2 == J.ay.n && s.lone == lone; });
+        if (it == sizes.end()) {
+            sizes.push_back({J.ax.n, J.ay.n, lone, kern_elems});
             koff[j] = kern_elems;
-            kern_elems += (size_t)2 * n1 * n2;
+            kern_elems += (size_t)J.ay.n * J.nhp;
         } else {
-            koff[j] = size_off[it - sizes.begin()];
+            koff[j] = it->off;
         }
-        max_n1 = std::max(max_n1, n1);
-        max_n2 = std::max(max_n2, n2);
-    }
-    // one twiddle table per distinct length
-    std::vector<uint32_t> lens;
-    for (auto &s : shapes) {
-        lens.push_back(pad(s.X));
-        lens.push_back(pad(s.Y));
-    }
-    std::sort(lens.begin(), lens.end());
-    lens.erase(std::unique(lens.begin(), lens.end()), lens.end());
-    size_t tw_elems = 0;
-    std::vector<size_t> twoff(lens.size());
-    for (size_t i = 0; i < lens.size(); ++i) {
-        twoff[i] = tw_elems;
-        tw_elems += std::max<uint32_t>(warp ? lens[i] : lens[i] / 2, 1);
+        table(J.ax);
+        table(J.ay);
     }
     TPT_CUDA(cudaMalloc(&work, std::max<size_t>(work_elems, 1) * sizeof(float2)));
-    TPT_CUDA(cudaMalloc(&spec, std::max<size_t>(spec_elems, 1) * sizeof(float2)));
+    TPT_CUDA(cudaMalloc(&spec, std::max<size_t>(2 * work_elems, 1) * sizeof(float2)));
     TPT_CUDA(cudaMalloc(&kern, std::max<size_t>(kern_elems, 1) * sizeof(float2)));
-    TPT_CUDA(cudaMalloc(&tw, std::max<size_t>(tw_elems, 1) * sizeof(float2)));
-    std::vector<float2> twh(tw_elems);
-    for (size_t i = 0; i < lens.size(); ++i) {
-        auto t = twiddles<float2>(lens[i], warp);
-        std::copy(t.begin(), t.end(), twh.begin() + twoff[i]);
+    TPT_CUDA(cudaMemset(kern, 0, std::max<size_t>(kern_elems, 1) * sizeof(float2)));
+    TPT_CUDA(cudaMalloc(&tw, std::max<size_t>(twh.size(), 1) * sizeof(float2)));
+    TPT_CUDA(cudaMemcpy(tw, twh.data(), twh.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    for (const Size &s : sizes) {
+        if (s.lone) continue;  // zeroed above
+        rc = build_spectra(s.n1, s.n2, (s.n1 / 2 + 1 + 7) / 8 * 8, kern + s.off);
+        if (rc) return rc;
     }
-    TPT_CUDA(cudaMemcpy(tw, twh.data(), tw_elems * sizeof(float2), cudaMemcpyHostToDevice));
-    auto tw_of = [&](uint32_t n) {
-        size_t i = std::lower_bound(lens.begin(), lens.end(), n) - lens.begin();
-        return tw + twoff[i];
-    };
-    // kernel spectra: one build per distinct (n1, n2), copied to each job
-    std::vector<std::pair<uint32_t, uint32_t>> built;
-    std::vector<size_t> built_off;
-    max_cb = 1;
+    auto tw_of = [&](uint32_t n) { return tw + lens_off[std::find(lens.begin(), lens.end(), n) - lens.begin()]; };
+    // Per block about `per` points of rows and twice that of columns (two to
+    // four work items per thread in each step: the job's staging and the code
+    // fetched serve all of them), fewer while that leaves SMs idle.
+    size_t points = 0;
+    for (const Job &J : jobs_host) points += (size_t)J.Y * J.ax.n;
+    uint32_t per = 2048;
+    while (per > 512 && points / per < 2 * 148) per /= 2;
+    std::vector<BlockRef> list[4];  // rows forward, columns, rows inverse, longer columns
+    size_t smem[4] = {};
     for (size_t j = 0; j < nj; ++j) {
-        const JobShape &s = shapes[j];
         Job &J = jobs_host[j];
-        J = Job{};
-        J.X = s.X;
-        J.pitch = s.X;
-        J.Y = s.Y;
-        J.n1 = pad(s.X);
-        J.n2 = pad(s.Y);
-        J.l1 = log2u(J.n1);
-        J.l2 = log2u(J.n2);
-        J.mass_scale_inv = 1.0f / 65536.0f;
         J.work = work + woff[j];
-        J.spec = spec + soff[j];
-        J.tw1 = tw_of(J.n1);
-        J.tw2 = tw_of(J.n2);
-        size_t plane = (size_t)J.n1 * J.n2;
-        auto key = std::make_pair(J.n1, J.n2);
-        auto it = std::find(built.begin(), built.end(), key);
-        if (it == built.end()) {
-            float2 *kx = kern + koff[j], *ky = kx + plane;
-            double scale = -(double)6.673e-1f / ((double)J.n1 * (double)J.n2);
-            int brc = warp ? build_spectra_permuted(J.n1, J.n2, scale, kx, ky)
-                           : build_spectra(J.n1, J.n2, scale, kx, ky, nullptr);
-            if (brc) return brc;
-            built.push_back(key);
-            built_off.push_back(koff[j]);
-            J.kx = kx;
-            J.ky = ky;
-        } else {
-            size_t o = built_off[it - built.begin()];
-            J.kx = kern + o;
-            J.ky = kern + o + plane;
-        }
-        for (uint32_t y = 0; y < s.Y; ++y) rr.push_back({(uint32_t)j, y});
-        int cb = std::min<int>(col_block(J.n2), (int)J.n1);
-        max_cb = std::max(max_cb, cb);
-        // warp form: one inverse row per y (both fields); shared-memory form:
-        // one per (field, y)
-        for (uint32_t i = 0; i < (warp ? 1u : 2u) * s.Y; ++i) ir.push_back({(uint32_t)j, i});
+        J.spec = spec + 2 * woff[j];
+        J.kern = kern + koff[j];
+        J.ax.tw = tw_of(J.ax.n);
+        J.ay.tw = tw_of(J.ay.n);
+        J.rows_f = J.rows_i = std::max<uint32_t>(1u, per / J.ax.n);
+        // columns: at least 4 (32-byte pieces of the rows), 2 when there are
+        // few blocks or their two buffers would leave one block per SM
+        J.lc = 2;
+        while (J.lc < 5 && (J.ay.n << (J.lc + 1)) <= 2 * per) ++J.lc;
+        while (J.lc > 1 && (points / per < 2 * 148 || ((size_t)J.ay.sz << J.lc) * 2 * sizeof(float2) > 100 * 1024)) --J.lc;
+        for (uint32_t p = 0; p < (J.Y + 1) / 2; p += J.rows_f) list[0].push_back({(uint32_t)j, p});
+        const size_t csm = ((size_t)J.ay.sz << J.lc) * 2 * sizeof(float2);
+        const int pc = csm <= COL_SMEM_SMALL ? 1 : 3;
+        for (uint32_t h = 0; h < J.nh; h += 1u << J.lc) list[pc].push_back({(uint32_t)j, h});
+        for (uint32_t y = 0; y < J.Y; y += J.rows_i) list[2].push_back({(uint32_t)j, y});
+        smem[0] = std::max(smem[0], J.rows_f * J.ax.sz * sizeof(float2));
+        smem[pc] = std::max(smem[pc], csm);
+        smem[2] = std::max(smem[2], J.rows_i * J.ax.sz * sizeof(float2));
     }
-    // the column kernel needs one cb for the whole launch: use the smallest
-    // needed by any job (power-of-two, divides every n1); the warp form
-    // takes WARPS columns per block
-    cb_launch = 16;
-    for (auto &J : jobs_host) cb_launch = std::min(cb_launch, std::min<int>(col_block(J.n2), (int)J.n1));
-    if (warp) cb_launch = WARPS;
-    max_y = 0;
-    for (auto &J : jobs_host) max_y = std::max(max_y, J.Y);
-    cr.clear();
-    for (size_t j = 0; j < nj; ++j) {
-        // warp form: WARPS half-column indices per block (n1/2 + 1 columns)
-        const uint32_t ncol = warp ? jobs_host[j].n1 / 2 + 1 : jobs_host[j].n1;
-        for (uint32_t c = 0; c < ncol; c += cb_launch) cr.push_back({(uint32_t)j, c});
+    std::vector<BlockRef> all;
+    Pass *passes[4] = {&rows, &cols[0], &inv, &cols[1]};
+    for (int p = 0; p < 4; ++p) {
+        // longest first, blocks of one length together (they run the same code)
+        std::stable_sort(list[p].begin(), list[p].end(), [&](const BlockRef &a, const BlockRef &b) {
+            const Job &ja = jobs_host[a.job], &jb = jobs_host[b.job];
+            return p & 1 ? ja.ay.n > jb.ay.n : ja.ax.n > jb.ax.n;
+        });
+        passes[p]->first = (uint32_t)all.size();
+        passes[p]->blocks = (uint32_t)list[p].size();
+        passes[p]->smem = smem[p];
+        passes[p]->threads = p == 3 ? NT_LARGE : NT;
+        all.insert(all.end(), list[p].begin(), list[p].end());
     }
-    if (warp) {
-        // blocks of the same transform length run the same code: keep them
-        // together so that co-resident blocks share the instruction cache
-        auto by = [&](bool col) {
-            return [&, col](const BlockRef &a, const BlockRef &b) {
-                const uint32_t la = col ? jobs_host[a.job].n2 : jobs_host[a.job].n1;
-                const uint32_t lb = col ? jobs_host[b.job].n2 : jobs_host[b.job].n1;
-                return la > lb;
-            };
-        };
-        std::stable_sort(rr.begin(), rr.end(), by(false));
-        std::stable_sort(cr.begin(), cr.end(), by(true));
-        std::stable_sort(ir.begin(), ir.end(), by(false));
-    }
-    n_rows = (uint32_t)rr.size();
-    n_cols = (uint32_t)cr.size();
-    n_inv = (uint32_t)ir.size();
-    TPT_CUDA(cudaMalloc(&jobs, nj * sizeof(Job)));
-    TPT_CUDA(cudaMalloc(&refs, (rr.size() + cr.size() + ir.size()) * sizeof(BlockRef)));
-    TPT_CUDA(cudaMemcpy(refs, rr.data(), rr.size() * sizeof(BlockRef), cudaMemcpyHostToDevice));
-    TPT_CUDA(cudaMemcpy(refs + rr.size(), cr.data(), cr.size() * sizeof(BlockRef), cudaMemcpyHostToDevice));
-    TPT_CUDA(cudaMemcpy(refs + rr.size() + cr.size(), ir.data(), ir.size() * sizeof(BlockRef), cudaMemcpyHostToDevice));
+    TPT_CUDA(cudaMalloc(&jobs, std::max<size_t>(nj, 1) * sizeof(Job)));
+    TPT_CUDA(cudaMalloc(&refs, std::max<size_t>(all.size(), 1) * sizeof(BlockRef)));
+    TPT_CUDA(cudaMemcpy(refs, all.data(), all.size() * sizeof(BlockRef), cudaMemcpyHostToDevice));
     return upload_jobs();
 }
 
@@ -607,27 +614,42 @@ int FftSet::set_io(size_t j, const int32_t *mass_i, const float *mass_f, float i
 }
 
 int FftSet::launch(cudaStream_t st, const JobIO *io) const {
-    if (n_rows == 0) return TPT_OK;
-    JobIO none{};
-    const JobIO &a = io ? *io : none;
-    if (warp) {
-        rows_forward_w<<<(n_rows + WARPS - 1) / WARPS, NTW, 0, st>>>(jobs, refs, n_rows, a);
-        TPT_LAUNCHED();
-        cols_convolve_w<<<n_cols, NTW, (size_t)WARPS * (max_y + max_n2) * sizeof(float2), st>>>(jobs, refs + n_rows,
-                                                                                               max_y, max_n2);
-        TPT_LAUNCHED();
-        rows_inverse_w<<<(n_inv + WARPS - 1) / WARPS, NTW, 0, st>>>(jobs, refs + n_rows + n_cols, n_inv, a);
+    if (rows.blocks == 0) return TPT_OK;
+    Job one{};
+    if (io) {
+        one = jobs_host[0];
+        one.mass_i = io->mass_i;
+        one.mass_f = io->mass_f;
+        one.mask = io->mask;
+        one.gx = io->gx;
+        one.gy = io->gy;
+        one.mass_scale_inv = io->mass_scale_inv;
+    }
+    // The column and inverse passes are programmatic dependents of the pass
+    // before them; the first pass is an ordinary launch, so nothing of a solve
+    // starts before the stream's earlier work is done.
+    auto run = [&](void (*kernel)(const Job *, const BlockRef *, const Job), const Pass &p, bool dependent) -> int {
+        if (p.blocks == 0) return TPT_OK;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(p.blocks);
+        cfg.blockDim = dim3(p.threads);
+        cfg.dynamicSmemBytes = p.smem;
+        cfg.stream = st;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = dependent ? 1 : 0;
+        TPT_CUDA(cudaLaunchKernelEx(&cfg, kernel, io ? (const Job *)nullptr : (const Job *)jobs,
+                                    (const BlockRef *)(refs + p.first), one));
         TPT_LAUNCHED();
         return TPT_OK;
-    }
-    rows_forward<<<n_rows, NT, max_n1 * sizeof(float2), st>>>(jobs, refs, a);
-    TPT_LAUNCHED();
-    cols_convolve<<<n_cols, NT, (size_t)cb_launch * 2 * max_n2 * sizeof(float2), st>>>(jobs, refs + n_rows,
-                                                                                        cb_launch);
-    TPT_LAUNCHED();
-    rows_inverse<<<n_inv, NT, max_n1 * sizeof(float2), st>>>(jobs, refs + n_rows + n_cols, a);
-    TPT_LAUNCHED();
-    return TPT_OK;
+    };
+    int rc = run(k_rows_forward, rows, false);
+    if (rc == TPT_OK) rc = run(k_columns, cols[1], true);
+    if (rc == TPT_OK) rc = run(k_columns, cols[0], true);
+    if (rc == TPT_OK) rc = run(k_rows_inverse, inv, true);
+    return rc;
 }
 
 void FftSet::destroy() {
@@ -641,9 +663,7 @@ void FftSet::destroy() {
     jobs = nullptr;
     refs = nullptr;
     jobs_host.clear();
-    n_rows = n_cols = n_inv = 0;
-    max_n1 = max_n2 = max_y = 0;
-    warp = false;
+    rows = cols[0] = cols[1] = inv = Pass{};
 }
 
 }  // namespace gfft

@@ -13,19 +13,19 @@ struct JobShape {
 
 namespace gfft {
 
-uint32_t next_pow2(uint32_t v);
-int build_spectra(uint32_t n1, uint32_t n2, double scale, float2 *kx, float2 *ky, double2 *out64);
-
 // A set of independent FP32 FFT gravity solves (one plan = one job; a batch
 // = one job per instance) that run as three launches.
 struct FftSet {
+    // One launch: its blocks (a range of `refs`) and dynamic shared memory.
+    struct Pass {
+        uint32_t first = 0, blocks = 0, threads = 0;
+        size_t smem = 0;
+    };
     std::vector<Job> jobs_host;
     Job *jobs = nullptr;
     BlockRef *refs = nullptr;
     float2 *work = nullptr, *spec = nullptr, *kern = nullptr, *tw = nullptr;
-    uint32_t n_rows = 0, n_cols = 0, n_inv = 0, max_n1 = 0, max_n2 = 0, max_y = 0;
-    int cb_launch = 1, max_cb = 1;
-    bool warp = false;  // every job's padded lengths lie in 32 .. 1024: the warp-register form
+    Pass rows, cols[2], inv;  // rows forward, columns (small and large shared memory), rows inverse
 
     int create(const std::vector<JobShape> &shapes);
     // Points job j at its inputs/outputs; returns 1 if anything changed
