@@ -312,12 +312,13 @@ def run_c3(solves: int):
     return out
 
 
-def air_launches(ticks, tuning, per_tick, chunk=1000):
+def air_launches(ticks, tuning, per_tick, chunk=1000, passes=2):
     """Air launches of `ticks` ticks stepped in graphs of `chunk` ticks.
-    `per_tick` is the profile's unblocked count (2, or 3 with a NoUpdate +
-    heat instance in the tile form); the tile form at temporal depth k runs
-    each block of n <= k ticks (cut at the chunk's end) as n + 1 launches,
-    plus one settle launch per tick with a NoUpdate + heat instance."""
+    `per_tick` is the profile's unblocked count (`passes`, or one more with a
+    NoUpdate + heat instance in the tile form); the tile form at temporal
+    depth k runs each block of n <= k ticks (cut at the chunk's end) as n - 1
+    launches more than its `passes` (2, or 3 as warp strips), plus one settle
+    launch per tick with a NoUpdate + heat instance."""
     import tpt_field as tf
 
     k = tuning.temporal_depth if tuning.air_form == tf.AIR_FORM_TILES else 1
@@ -330,7 +331,7 @@ def air_launches(ticks, tuning, per_tick, chunk=1000):
         t = 0
         while t < c:
             n = min(k, c - t)
-            total += n + 1 + (per_tick - 2) * n
+            total += n - 1 + passes + (per_tick - passes) * n
             t += n
     return total
 
@@ -431,12 +432,14 @@ def run_ours(args, rank, world, local):
     hbm, bf16, bf16s, peak_src = load_peaks()
     air_gbs = prof.cells * prof.ticks * B_AIR / (prof.air_ms / 1e3) / 1e9
     tuning = batch.tuning()
-    air_launch_ms = prof.air_ms / air_launches(prof.ticks, tuning, prof.air_launches_per_tick, chunk=prof.ticks)
+    # no workload has a NoUpdate + heat instance: the profile's count is the passes'
+    passes = prof.air_launches_per_tick
+    air_launch_ms = prof.air_ms / air_launches(prof.ticks, tuning, passes, chunk=prof.ticks, passes=passes)
     roof_air = {"kernel": "air tick (pressure+velocity, advection+heat+masks)", "bound": "hbm",
                 "achieved": round(air_gbs, 1), "peak": hbm, "unit": "GB/s", "frac": round(air_gbs / hbm, 4),
                 "peak_source": peak_src, "algorithmic_bytes_per_cell_tick": B_AIR,
                 "traffic": MEASURED_DRAM_BYTES.get(cid, {}).get("air_tick"),
-                "traffic_unit": "DRAM bytes per tick, both launches (ncu)",
+                "traffic_unit": "DRAM bytes per tick, all air launches (ncu)",
                 "ms_per_tick": round(prof.air_ms / prof.ticks, 5),
                 "avg_launch_ms": round(air_launch_ms, 5)}
     phases = {"air_ms_per_tick": prof.air_ms / prof.ticks, "grav_ms_per_tick": prof.grav_ms / prof.ticks}
@@ -450,7 +453,7 @@ def run_ours(args, rank, world, local):
     else:
         roof_grav = None
     dominant = roof_grav if (roof_grav and prof.grav_ms > prof.air_ms) else roof_air
-    launches = (air_launches(ticks, tuning, prof.air_launches_per_tick) + prof.grav_launches_per_tick * ticks) * \
+    launches = (air_launches(ticks, tuning, passes, passes=passes) + prof.grav_launches_per_tick * ticks) * \
         args.steps + (args.steps if ticks % 2 else 0)
 
     plain = None

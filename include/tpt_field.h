@@ -347,7 +347,9 @@ enum {
     /* Two launches per tick over tiles (32x8, 64x8, 32x16 or 64x16 cells),
      * halos staged by TMA: pass A (pressure, velocity) writes opv/ovx/ovy,
      * pass B (smoothing, advection, vorticity, fans, heat, convection, masks)
-     * reads them. */
+     * reads them. A batch of 1.5 million cells or more runs the same passes as
+     * strips, one per warp, of 26 to 30 columns and a number of rows that goes
+     * with the tile shape (24, 32, 16 and 40 on average), B as two launches. */
     TPT_AIR_FORM_TILES = 0,
     /* One fused launch per tick: CTAs sweep down column strips with every
      * stage pipelined over the rows (no intermediate grid in memory), plus a
@@ -362,7 +364,8 @@ enum {
  * gravity stream, the tile form with the work queue. */
 typedef struct tpt_batch_tuning {
     /* The air form's work unit. Tile form: the tile, tile_x x tile_y cells,
-     * one of 32x8 (the default), 64x8, 32x16 and 64x16, one thread per cell.
+     * one of 32x8 (the default), 64x8, 32x16 and 64x16, one thread per cell
+     * (or the strips that go with it, see TPT_AIR_FORM_TILES).
      * Sweep form: a CTA of tile_x lanes (a multiple of 32 in 64..256) sweeps
      * down strips of about tile_y rows (8..2048); each lane owns a column, a
      * strip is at most tile_x - 12 columns wide (six halo columns on each
@@ -429,9 +432,11 @@ typedef struct tpt_batch_profile {
     float air_ms;              /* `ticks` air ticks alone (all instances)  */
     float grav_ms;             /* `ticks` gravity solves alone             */
     uint32_t ticks;
-    /* Air launches per tick without temporal blocking: 2 (3 in the tile
-     * form with a NoUpdate + heat instance: its settle). At temporal depth
-     * k, a block of n <= k ticks makes n + 1 launches (plus the n settles). */
+    /* Air launches per tick without temporal blocking: 2, or 3 in the tile
+     * form of a batch of 1.5 million cells or more (one more in the tile form
+     * with a NoUpdate + heat instance: its settle). At temporal depth k, a
+     * block of n <= k ticks makes n - 1 launches more than one tick (plus the
+     * n settles). */
     uint32_t air_launches_per_tick;
     uint32_t grav_launches_per_tick;
     uint64_t cells;            /* sum of xcells*ycells over instances      */

@@ -185,3 +185,16 @@ def test_stream_ordering_and_launch_count(cuda, tf, oracle):
     s.synchronize()
     assert tf.launch_count() - n0 == 15
     assert_bit_exact(b.air_state(), oracle.air_steps(inst, 5), "stream")
+
+
+@pytest.mark.parametrize("X,Y,kw", [(707, 499, {}), (2048, 173, dict(gravity_mode=2, convection_mode=1)),
+                                    (172, 2047, dict(aheat_enable=0)), (613, 577, dict(air_mode=4)),
+                                    (1009, 359, dict(air_mode=2, gravity_mode=3, custom_gx=-20.0))])
+def test_large_grid_strips(cuda, tf, oracle, X, Y, kw):
+    """Grids large enough for the warp strips (350,000 cells), odd sides, a
+    strip's remainder of columns and rows, each pass left out by a mode."""
+    import workloads as W
+
+    assert X * Y >= 350000
+    inst = W.make_stress_instance(X, Y, X + Y, config=W.AirConfig(**kw))
+    assert_bit_exact(run_gpu(tf, cuda, inst, 2), oracle.air_steps(inst, 2), f"{X}x{Y}")

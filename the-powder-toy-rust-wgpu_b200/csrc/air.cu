@@ -1,8 +1,8 @@
 // air.cu -- the one-grid air step (tpt_air_step and its static-scratch
-// variant). Compiled with -fmad=false: see air.cuh.
+// variant): tiles, or warp strips for a large grid. Compiled with -fmad=false: see air.cuh.
 #include <algorithm>
 
-#include "air.cuh"
+#include "air_strip.cuh"
 #include "air_launch.hpp"
 
 namespace tpt {
@@ -42,16 +42,51 @@ __global__ void __launch_bounds__(NT) k_advect_heat(const AirInst I) {
     pass_b(I, x0, y0, S);
 }
 
-// Settle pass: new heat -> hv, NoUpdate convection -> vx/vy, wall masks
-// (settle.rs:50-93) and the optional HotAir pass (settle.rs:118-161). The
-// grid is dense here (pitch == X).
+// The same tick as warp strips (air_strip.cuh): warp w takes strip w % strips of
+// row block w / strips. Strips need fewer instructions per cell, but a warp
+// walks its rows one after the other: below about 350,000 cells the tiles, a
+// thread per cell, are done sooner. Measured on B200, us per tick, tiles and
+// strips: 401x225 24.5 and 35.9, 512x512 34.6 and 37.8, 700x600 48.4 and 44.9,
+// 1024x1024 93.9 and 81.9, 2048x2048 378 and 246.
+constexpr size_t STRIP_MIN_CELLS = 350000;
+struct OneGrid {
+    StripGrids P;
+    AirInst I;
+    uint32_t strips, rows;  // strips across the grid, rows per block
+};
+__device__ __forceinline__ bool strip_of(const OneGrid &G, int width, int &x0, int &y0, int &y1) {
+    const uint32_t w = blockIdx.x * (blockDim.x / 32u) + threadIdx.x / 32u, b = w / G.strips;
+    x0 = (int)((w - b * G.strips) * (uint32_t)width);
+    y0 = (int)(b * G.rows);
+    y1 = min(y0 + (int)G.rows, (int)G.I.Y);
+    return y0 < (int)G.I.Y;
+}
+__global__ void __launch_bounds__(STRIP_WARPS * 32, 8) k_strip_velocity(const __grid_constant__ OneGrid G) {
+    int x0, y0, y1;
+    if (strip_of(G, strip_width(PASS_VELOCITY), x0, y0, y1)) strip_a(G.P, G.I, 0u, x0, y0, y1);
+}
+__global__ void __launch_bounds__(STRIP_WARPS * 32, 6) k_strip_advect(const __grid_constant__ OneGrid G) {
+    int x0, y0, y1;
+    // into vx / vy, free since the velocity pass read them
+    if (strip_of(G, strip_width(PASS_ADVECT), x0, y0, y1)) strip_advect(G.P, G.I, G.P.vx, G.P.vy, 0u, x0, y0, y1);
+}
+__global__ void __launch_bounds__(STRIP_WARPS * 32, 6) k_strip_heat(const __grid_constant__ OneGrid G) {
+    int x0, y0, y1;
+    // from vx / vy into ovx / ovy; the settle pass copies them back
+    if (strip_of(G, strip_width(PASS_HEAT), x0, y0, y1))
+        strip_heat<false, true>(G.P, G.I, nullptr, nullptr, 0u, x0, y0, y1, 0u);
+}
+
+// Settle pass: new heat -> hv, convected velocity -> vx/vy where the heat pass
+// left it in ovx/ovy (`copy_v`), wall masks (settle.rs:50-93) and the optional
+// HotAir pass (settle.rs:118-161). The grid is dense here (pitch == X).
 __global__ void k_settle(const AirInst I, const uint32_t *__restrict__ pmap, const uint32_t *__restrict__ props,
-                         uint32_t nprops, uint32_t xres, uint32_t yres) {
+                         uint32_t nprops, uint32_t xres, uint32_t yres, bool copy_v) {
     const size_t n = (size_t)I.X * I.Y;
     for (size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x; g < n; g += (size_t)gridDim.x * blockDim.x) {
         if (I.aheat) {
             I.hv[g] = I.hv_out[g];
-            if (I.air_mode == 4u) {
+            if (copy_v) {
                 I.vx[g] = I.ovx[g];
                 I.vy[g] = I.ovy[g];
             }
@@ -86,20 +121,53 @@ __global__ void k_settle(const AirInst I, const uint32_t *__restrict__ pmap, con
     }
 }
 
+static StripGrids one_grid(const AirInst &I) {
+    StripGrids g{};
+    g.pv = I.pv, g.vx = I.vx, g.vy = I.vy, g.opv = I.opv, g.ovx = I.ovx, g.ovy = I.ovy;
+    g.hv = I.hv, g.hv_out = I.hv_out;
+    g.bair = I.bair, g.bairh = I.bairh;
+    g.wall = I.wall;
+    g.fvx = I.fvx, g.fvy = I.fvy;
+    return g;
+}
+
 int launch_single(const AirInst &I, const uint32_t *pmap, const uint32_t *props, uint32_t nprops, uint32_t xres,
                   uint32_t yres, cudaStream_t st) {
-    dim3 grid((I.X + TX - 1) / TX, (I.Y + TY - 1) / TY);
-    if (I.air_mode != 4u) {
-        k_pressure_velocity<<<grid, NT, 0, st>>>(I);
-        TPT_LAUNCHED();
+    const size_t n = (size_t)I.X * I.Y;
+    const bool strips = n >= STRIP_MIN_CELLS && I.X >= 3 && I.Y >= 3;
+    if (strips) {
+        OneGrid G{one_grid(I), I, 0u, 0u};
+        auto run = [&](void (*kernel)(const OneGrid), int pass) -> int {
+            const uint32_t w = (uint32_t)strip_width(pass);
+            G.strips = (I.X + w - 1) / w;
+            // about three strips per resident warp, of 4 to 32 rows
+            const size_t fit = (size_t)G.strips * I.Y / (3 * 148 * 24);
+            G.rows = (uint32_t)std::min<size_t>(32, std::max<size_t>(4, fit));
+            const uint32_t warps = G.strips * ((I.Y + G.rows - 1) / G.rows);
+            kernel<<<(warps + STRIP_WARPS - 1) / STRIP_WARPS, STRIP_WARPS * 32, 0, st>>>(G);
+            TPT_LAUNCHED();
+            return TPT_OK;
+        };
+        int rc = TPT_OK;
+        if (I.air_mode != 4u) {
+            rc = run(k_strip_velocity, PASS_VELOCITY);
+            if (rc == TPT_OK) rc = run(k_strip_advect, PASS_ADVECT);
+        }
+        if (rc == TPT_OK && I.aheat) rc = run(k_strip_heat, PASS_HEAT);
+        if (rc) return rc;
+    } else {
+        dim3 grid((I.X + TX - 1) / TX, (I.Y + TY - 1) / TY);
+        if (I.air_mode != 4u) {
+            k_pressure_velocity<<<grid, NT, 0, st>>>(I);
+            TPT_LAUNCHED();
+        }
+        if (I.air_mode != 4u || I.aheat) {
+            k_advect_heat<<<grid, NT, 0, st>>>(I);
+            TPT_LAUNCHED();
+        }
     }
-    if (I.air_mode != 4u || I.aheat) {
-        k_advect_heat<<<grid, NT, 0, st>>>(I);
-        TPT_LAUNCHED();
-    }
-    size_t n = (size_t)I.X * I.Y;
     unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, 148 * 16);
-    k_settle<<<blocks, 256, 0, st>>>(I, pmap, props, nprops, xres, yres);
+    k_settle<<<blocks, 256, 0, st>>>(I, pmap, props, nprops, xres, yres, I.aheat && (strips || I.air_mode == 4u));
     TPT_LAUNCHED();
     return TPT_OK;
 }

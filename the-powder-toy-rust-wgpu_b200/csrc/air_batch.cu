@@ -1,6 +1,5 @@
 // air_batch.cu -- the batched air tick's shared pieces: the sweep form's
-// velocity pre-pass, the copy-back, and the table of the tile form's shapes
-// (their kernels are in air_tiles.cu).
+// velocity pre-pass and the copy-back.
 //
 // Sweep form's pre-pass: the velocity pass of the instances whose previous
 // tick sampled velocity outside the sweep's rings (air_sweep.cu), writing
@@ -84,35 +83,6 @@ __global__ void kb_copy_back(const AirInst *__restrict__ insts, const TileRef *_
 int launch_copy_back(const AirInst *insts, const TileRef *tiles, uint32_t ntiles, uint32_t grid, cudaStream_t st) {
     kb_copy_back<<<grid, NT, 0, st>>>(insts, tiles, ntiles);
     TPT_LAUNCHED();
-    return TPT_OK;
-}
-
-const TileShape *const *tile_shapes() {
-    static const TileShape *const all[TILE_SHAPES] = {&tile_shape_s32x8, &tile_shape_s64x8, &tile_shape_s32x16,
-                                                      &tile_shape_s64x16};
-    return all;
-}
-
-const TileShape *tile_shape(uint32_t tx, uint32_t ty) {
-    for (int k = 0; k < TILE_SHAPES; ++k)
-        if (tile_shapes()[k]->tx == tx && tile_shapes()[k]->ty == ty) return tile_shapes()[k];
-    return nullptr;
-}
-
-// The batched air kernels' error words: the tile form's, one per shape, and
-// the temporally blocked launches' (the sweep form and the pre-pass have no
-// waits).
-int read_errors(uint32_t *out) {
-    uint32_t all = 0;
-    int frc = read_fused_errors(&all);
-    if (frc) return frc;
-    for (int k = 0; k < TILE_SHAPES; ++k) {
-        uint32_t v = 0;
-        int rc = tile_shapes()[k]->read_errors(&v);
-        if (rc) return rc;
-        all |= v;
-    }
-    *out = all;
     return TPT_OK;
 }
 

@@ -3,24 +3,26 @@
 
 #include <cuda.h>
 
+#include <vector>
+
 #include "common.cuh"
 
 namespace tpt {
 namespace air {
 
 // One tile of one batched instance: AIR_TX x AIR_TY cells for the pre-pass and
-// the copy-back, the tile form's shape for its passes.
+// the copy-back, the shape's tile for the tile kernels.
 struct TileRef {
     uint32_t inst;
     uint16_t tx, ty;
 };
 
-// ---- the tile form (air_tiles.cu) ---------------------------------------------
-// Tensor maps of one batched instance: the grids the two passes stage, with
-// the two halves of the heat and mask ping-pong.
-// The velocity pass's outputs (ovx, ovy, opv) alternate between two sets by
-// tick parity, so a launch that ends one tick and starts the next (the
-// temporally blocked form) reads one set while it writes the other.
+// Tensor maps of one batched instance for the tile kernels and the temporally
+// blocked launches: the grids they stage, with the two halves of the heat and
+// mask ping-pong. The
+// velocity pass's outputs (ovx, ovy, opv) alternate between two sets by tick
+// parity, so a launch that ends one tick and starts the next reads one set
+// while it writes the other.
 enum TensorMapSlot {
     TM_PV, TM_VX, TM_VY,
     TM_OV0, TM_OVX0 = TM_OV0, TM_OVY0, TM_OPV0,
@@ -28,14 +30,48 @@ enum TensorMapSlot {
     TM_BA0, TM_BA1, TM_BH0, TM_BH1, TM_HV0, TM_HV1, TM_COUNT
 };
 
-// One tile shape of the tile form (air_tiles.cu, compiled once per shape).
-// Its tiles are tx x ty cells, one thread per cell, each staged as a TMA box
-// of (tx + 8) x (ty + 6) cells: the tensor maps and the tile list of a batch
-// are built for the shape in use.
+// ---- the tile form (air_tiles.cu, air_strips.cu) -------------------------------------------
+// The passes of a tick as warp strips (air_strip.cuh): velocity, advection,
+// heat and masks. A strip's 32 lanes are its output columns and a halo on
+// each side.
+enum StripPass { PASS_VELOCITY, PASS_ADVECT, PASS_HEAT, STRIP_PASSES };
+constexpr int VELOCITY_HALO = 3, ADVECT_HALO = 2, HEAT_HALO = 1;
+constexpr int strip_halo(int pass) { return pass == PASS_VELOCITY ? VELOCITY_HALO : pass == PASS_ADVECT ? ADVECT_HALO : HEAT_HALO; }
+constexpr int strip_width(int pass) { return 32 - 2 * strip_halo(pass); }
+constexpr int STRIP_WARPS = 4;  // per CTA
+
+// Output rows y0 .. y0 + rows - 1 of the strip at column x0.
+struct StripRef {
+    uint32_t inst;
+    uint16_t x0, y0, rows, pad;
+};
+
+// Base addresses of the grids; an instance's cell (x, y) is at element
+// off + y * pitch + x of each. Passed as a kernel parameter: the addresses
+// stay in the constant bank instead of two registers each.
+struct StripGrids {
+    float *pv, *vx, *vy, *opv, *ovx, *ovy;
+    const float *hv;
+    float *hv_out;
+    const uint32_t *bair, *bairh;
+    uint32_t *bair_out, *bairh_out;
+    const uint32_t *wall;
+    uint32_t *emap;
+    const uint32_t *eair, *eairh;
+    const float *fvx, *fvy;
+};
+
+// One tile shape of the tile form: its tile kernels (air_tiles.cu, compiled
+// once per shape), which small batches run, and the rows of the warp strips
+// (air_strips.cu) that large ones run.
 struct TileShape {
     uint32_t tx, ty;
-    // sets the kernels' shared-memory limits and returns the resident CTAs
-    // per SM of the velocity pass (A) and the advection/heat pass (B)
+    uint32_t strip_rows;
+    // Tile kernels: tx x ty cells per CTA, one thread per cell, each grid staged
+    // as a TMA box of (tx + 8) x (ty + 6) cells: the tensor maps and the tile
+    // list of a batch are built for the shape in use. Sets the kernels'
+    // shared-memory limits and returns the resident CTAs per SM of the velocity
+    // pass (A) and the advection/heat pass (B).
     int (*prepare)(int *occupancy_a, int *occupancy_b);
     // The two passes of one tick of every instance: the velocity pass (A),
     // and the advection / heat / mask pass (B, with its NoUpdate settle)
@@ -62,6 +98,32 @@ constexpr int TILE_SHAPES = 4;
 // The offered shapes, 32x8 first; tile_shape(tx, ty) is null for any other.
 const TileShape *const *tile_shapes();
 const TileShape *tile_shape(uint32_t tx, uint32_t ty);
+// Appends a pass's strips of every instance (X, Y): about `rows` rows each,
+// `resident` warps working on them.
+void plan_strips(int pass, const std::vector<std::pair<uint32_t, uint32_t>> &grids, uint32_t rows, uint32_t resident,
+                 std::vector<StripRef> &out);
+// resident CTAs per SM, per pass
+int strip_occupancy(int occupancy[STRIP_PASSES]);
+
+// The passes of one tick of every instance.
+struct StripLaunch {
+    StripGrids grids[2];      // by tick parity: the hv / mask ping-pong and the velocity pass's outputs
+    const AirInst *insts;     // two per instance (the first one's scalars are used)
+    const StripRef *strips[STRIP_PASSES];
+    uint32_t nstrips[STRIP_PASSES], grid[STRIP_PASSES];
+    // the passes' work-queue counters (device, zero at creation), used as
+    // queues when use_queue (else the warps stride the list statically) and
+    // cleared either way, each by the launch of the pass before it
+    uint32_t *queues;
+    bool use_queue;
+};
+// the velocity pass (A)
+int launch_strips_a(const StripLaunch &s, uint32_t parity, cudaStream_t st);
+// the advection and the heat / mask passes (B, with its NoUpdate settle),
+// whose mask rebuild applies `emap_lag` pending emap decays
+int launch_strips_b(const StripLaunch &s, uint32_t parity, uint32_t emap_lag, bool any_noupdate_heat, cudaStream_t st);
+// the copy-back of NoUpdate instances' convected velocity after a pass B
+int launch_strips_settle(const StripLaunch &s, uint32_t parity, cudaStream_t st);
 
 // ---- temporal blocking of the tile form (air_fused.cu) ----------------------------
 // k ticks as A(t0), then k - 1 launches of B(t) + A(t + 1) over FUSED_TX x
@@ -125,12 +187,13 @@ int sweep_max_ctas_per_sm(uint32_t lanes, int *out);
 int launch_single(const AirInst &I, const uint32_t *pmap, const uint32_t *props, uint32_t nprops, uint32_t xres,
                   uint32_t yres, cudaStream_t st);
 
+// Reads and clears the device error words of the batched air kernels.
+int read_errors(uint32_t *out);
+
 // Copies the ping-pong halves that hold the newest state back to the
 // instance's canonical buffers (after an odd number of ticks).
 int launch_copy_back(const AirInst *insts, const TileRef *tiles, uint32_t ntiles, uint32_t grid, cudaStream_t st);
 
-// Reads and clears the device error word of the batched air kernels.
-int read_errors(uint32_t *out);
 
 }  // namespace air
 }  // namespace tpt

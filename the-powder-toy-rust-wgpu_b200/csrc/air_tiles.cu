@@ -354,7 +354,7 @@ int tile_read_errors(uint32_t *out) {
 #define AIR_CAT2(a, b) a##b
 #define AIR_CAT(a, b) AIR_CAT2(a, b)
 extern const TileShape AIR_CAT(tile_shape_, AIR_SHAPE_NS) = {(uint32_t)AIR_SHAPE_NS::TX, (uint32_t)AIR_SHAPE_NS::TY,
-                                                            tile_prepare, tile_launch_a, tile_launch_b,
+                                                            AIR_STRIP_ROWS, tile_prepare, tile_launch_a, tile_launch_b,
                                                             tile_launch_settle, tile_read_errors};
 
 }  // namespace air

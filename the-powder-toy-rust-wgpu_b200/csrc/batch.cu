@@ -6,7 +6,8 @@
 // 128-byte boundaries as TMA needs); cell (cx, cy) is at cy * pitch + cx.
 // The air state (pv, vx, vy, hv and the two wall masks) has a second copy
 // (ping-pong) for the air tick's two forms, chosen by the tuning: the tile
-// form (air_tiles.cu; two TMA-staged tile passes per tick, heat and masks in
+// form (air_tiles.cu, two TMA-staged tile passes per tick, or for a large
+// batch air_strips.cu, three passes of warp strips; heat and masks in
 // the ping-pong halves, pv/vx/vy in place; with temporal blocking, blocks of
 // k ticks whose middle launches fuse one tick's second pass with the next
 // tick's first, air_fused.cu) or the row sweep (air_sweep.cu; one launch per
@@ -76,6 +77,13 @@ __global__ void k_batch_io(const IoInst *io, uint32_t base, uint32_t *arena, uin
 // plus halos) by 64-row strips. Default tile form shape: 32 x 8 cells.
 constexpr uint32_t DEFAULT_LANES = 224, DEFAULT_ROWS = 64;
 constexpr uint32_t DEFAULT_TILE_X = 32, DEFAULT_TILE_Y = 8;
+// Cells from which a batch's tile form runs as warp strips (three launches a
+// tick, fewer instructions per cell) instead of tiles (two launches, every cell
+// a thread). Measured on B200 with FP32 gravity beside, us per tick, tiles and
+// strips: 0.55 M cells 77.6 and 82.2, 1.15 M 142.6 and 146.7, 1.81 M 238 and
+// 222, 2.26 M 263 and 241, 3.9 M 500 and 442, 6.1 M 677 and 596, 8.1 M 1003 and
+// 861 (air alone 613 and 454).
+constexpr size_t STRIP_MIN_CELLS = 1500000;
 
 // Splits every instance into column strips of at most lanes - 2 * SW_H
 // columns and row strips of about `rows` rows (sizes balanced within an
@@ -161,13 +169,18 @@ struct tpt_batch {
     // AIR_TX x AIR_TY tiles (the sweep's pre-pass, the copy-back)
     air::TileRef *tiles = nullptr;
     uint32_t ntiles = 0;
-    // the tile form at its current shape: tiles, tensor maps (boxes of the
-    // shape) and the advection/heat pass's resident CTAs per SM
+    // the tile form at its current shape. A small batch: tiles, tensor maps
+    // (boxes of the shape) and the passes' resident CTAs per SM
     const air::TileShape *shape = nullptr;
     air::TileRef *form_tiles = nullptr;
     uint32_t nform_tiles = 0;
     CUtensorMap *tmaps = nullptr;
-    int tile_occupancy_a = 1, tile_occupancy_b = 1;  // resident CTAs per SM of pass A / pass B
+    int tile_occupancy_a = 1, tile_occupancy_b = 1;
+    // a large one: its strips and their passes' resident CTAs per SM
+    bool use_strips = false;
+    air::StripRef *strips = nullptr;  // the passes' lists one after the other
+    uint32_t nstrips[air::STRIP_PASSES] = {};
+    int occupancy[air::STRIP_PASSES] = {1, 1, 1};
     // temporal blocking (tuning.temporal_depth > 1): the B(t) + A(t + 1)
     // launches' tiles and tensor maps (their own box), built on first use
     air::TileRef *fused_tiles = nullptr;
@@ -218,14 +231,43 @@ struct tpt_batch {
         L.want = want;
         return L;
     }
-    // the tile form's persistent grid: ctas_per_sm per SM (0: as many as fit,
-    // the residency of its advection/heat pass)
+    // base addresses of the grids at tick parity `par` (AirInst's halves)
+    air::StripGrids strip_grids(int par) const {
+        auto ff = [&](int field) { return f32 + (size_t)field * stride; };
+        auto uu = [&](int field) { return u32 + (size_t)field * stride; };
+        air::StripGrids g{};
+        g.pv = ff(F_PV), g.vx = ff(F_VX), g.vy = ff(F_VY);
+        g.opv = ff(par ? F_PV2 : F_OPV), g.ovx = ff(par ? F_VX2 : F_OVX), g.ovy = ff(par ? F_VY2 : F_OVY);
+        g.hv = ff(par ? F_HV2 : F_HV), g.hv_out = ff(par ? F_HV : F_HV2);
+        g.bair = uu(par ? U_BA2 : U_BA), g.bair_out = uu(par ? U_BA : U_BA2);
+        g.bairh = uu(par ? U_BH2 : U_BH), g.bairh_out = uu(par ? U_BH : U_BH2);
+        g.wall = uu(U_WALL), g.emap = uu(U_EMAP), g.eair = uu(U_EA), g.eairh = uu(U_EH);
+        g.fvx = ff(F_FVX), g.fvy = ff(F_FVY);
+        return g;
+    }
+    air::StripLaunch strip_launch() const {
+        air::StripLaunch s{};
+        s.grids[0] = strip_grids(0);
+        s.grids[1] = strip_grids(1);
+        s.insts = insts_tile;
+        const air::StripRef *list = strips;
+        for (int k = 0; k < air::STRIP_PASSES; ++k) {
+            s.strips[k] = list;
+            s.nstrips[k] = nstrips[k];
+            list += nstrips[k];
+            // persistent: ctas_per_sm per SM (0: as many as fit)
+            const uint32_t per_sm = tuning.ctas_per_sm ? tuning.ctas_per_sm : (uint32_t)occupancy[k];
+            s.grid[k] = std::max<uint32_t>(1u, std::min<uint32_t>((nstrips[k] + air::STRIP_WARPS - 1) / air::STRIP_WARPS, (uint32_t)sms * per_sm));
+        }
+        s.queues = tile_queue;
+        s.use_queue = tuning.work_queue != 0;
+        return s;
+    }
+    // the tile kernels' persistent grid: ctas_per_sm per SM (0: as many as fit)
     uint32_t tile_grid(int occupancy) const {
         const uint32_t per_sm = tuning.ctas_per_sm ? tuning.ctas_per_sm : (uint32_t)occupancy;
         return std::max<uint32_t>(1u, std::min<uint32_t>(nform_tiles, (uint32_t)sms * per_sm));
     }
-    uint32_t tile_grid_a() const { return tile_grid(tile_occupancy_a); }
-    uint32_t tile_grid_b() const { return tile_grid(tile_occupancy_b); }
     bool sweep_form() const { return tuning.air_form == TPT_AIR_FORM_SWEEP; }
     const AirInst *form_insts() const { return sweep_form() ? insts : insts_tile; }
     uint32_t fused_grid() const {
@@ -242,19 +284,25 @@ struct tpt_batch {
             return rc;
         }
         const uint32_t k = std::max<uint32_t>(1u, tuning.temporal_depth);
+        const bool queue = tuning.work_queue != 0;
+        const air::StripLaunch s = strip_launch();
         for (uint32_t t = 0; t < ticks && rc == TPT_OK;) {
-            const uint32_t n = std::min<uint32_t>(k, ticks - t);
-            rc = shape->launch_a(insts_tile, tmaps, form_tiles, nform_tiles, tile_grid_a(), t & 1u, tile_queue,
-                                 tuning.work_queue != 0, st);
+            const uint32_t n = std::min<uint32_t>(k, ticks - t), last = (t + n - 1) & 1u;
+            rc = use_strips ? air::launch_strips_a(s, t & 1u, st)
+                            : shape->launch_a(insts_tile, tmaps, form_tiles, nform_tiles, tile_grid(tile_occupancy_a),
+                                              t & 1u, tile_queue, queue, st);
             for (uint32_t j = 0; j + 1 < n && rc == TPT_OK; ++j) {
                 const uint32_t p = (t + j) & 1u;
                 rc = air::launch_fused_ba(insts_tile, tmaps_fused, fused_tiles, nfused_tiles, fused_grid(), p, j, st);
                 if (rc == TPT_OK && any_noupdate_heat)
-                    rc = shape->launch_settle(insts_tile, form_tiles, nform_tiles, tile_grid_b(), p, st);
+                    rc = use_strips ? air::launch_strips_settle(s, p, st)
+                                    : shape->launch_settle(insts_tile, form_tiles, nform_tiles,
+                                                           tile_grid(tile_occupancy_b), p, st);
             }
             if (rc == TPT_OK)
-                rc = shape->launch_b(insts_tile, tmaps, form_tiles, nform_tiles, tile_grid_b(), (t + n - 1) & 1u, n - 1,
-                                     any_noupdate_heat, tile_queue, tuning.work_queue != 0, st);
+                rc = use_strips ? air::launch_strips_b(s, last, n - 1, any_noupdate_heat, st)
+                                : shape->launch_b(insts_tile, tmaps, form_tiles, nform_tiles, tile_grid(tile_occupancy_b),
+                                                  last, n - 1, any_noupdate_heat, tile_queue, queue, st);
             t += n;
         }
         return rc;
@@ -274,11 +322,12 @@ struct tpt_batch {
         cudaFree(i32);
         cudaFree(insts);
         cudaFree(insts_tile);
-        cudaFree(tmaps);
         cudaFree(stage);
         cudaFree(io);
         cudaFree(tiles);
         cudaFree(form_tiles);
+        cudaFree(tmaps);
+        cudaFree(strips);
         cudaFree(fused_tiles);
         cudaFree(tmaps_fused);
         cudaFree(tile_queue);
@@ -478,23 +527,53 @@ static int upload_tile_maps(const std::vector<CUtensorMap> &tm, const std::vecto
     return TPT_OK;
 }
 
-// Builds the tile form's tile list and tensor maps for tile shape `sh` (the
-// boxes are the tile plus a 4-cell x and 3-cell y halo) and uploads them.
+// Plans the tile form for shape `sh` and uploads it: the tile list and the
+// tensor maps (boxes of the tile plus a 4-cell x and 3-cell y halo), or the
+// strips.
 static int set_tile_shape(tpt_batch *b, const air::TileShape *sh) {
-    int occ_a = 0, occ_b = 0;
-    int rc = sh->prepare(&occ_a, &occ_b);
+    if (!b->use_strips) {
+        int occ_a = 0, occ_b = 0;
+        int rc = sh->prepare(&occ_a, &occ_b);
+        if (rc) return rc;
+        if (occ_a < 1 || occ_b < 1)
+            TPT_FAIL(TPT_ERR_UNSUPPORTED, "the %ux%u tile kernels do not fit an SM", sh->tx, sh->ty);
+        std::vector<air::TileRef> tiles;
+        std::vector<CUtensorMap> tm;
+        rc = build_tile_maps(b, sh->tx, sh->ty, sh->tx + 8, sh->ty + 6, tm, tiles);
+        if (rc) return rc;
+        rc = upload_tile_maps(tm, tiles, &b->form_tiles, &b->tmaps);
+        if (rc) return rc;
+        b->nform_tiles = (uint32_t)tiles.size();
+        b->shape = sh;
+        b->tile_occupancy_a = occ_a;
+        b->tile_occupancy_b = occ_b;
+        return TPT_OK;
+    }
+    int occ[air::STRIP_PASSES] = {};
+    int rc = air::strip_occupancy(occ);
     if (rc) return rc;
-    if (occ_a < 1 || occ_b < 1) TPT_FAIL(TPT_ERR_UNSUPPORTED, "the %ux%u tile kernels do not fit an SM", sh->tx, sh->ty);
-    std::vector<air::TileRef> tiles;
-    std::vector<CUtensorMap> tm;
-    rc = build_tile_maps(b, sh->tx, sh->ty, sh->tx + 8, sh->ty + 6, tm, tiles);
-    if (rc) return rc;
-    rc = upload_tile_maps(tm, tiles, &b->form_tiles, &b->tmaps);
-    if (rc) return rc;
-    b->nform_tiles = (uint32_t)tiles.size();
+    std::vector<air::StripRef> list;
+    uint32_t count[air::STRIP_PASSES];
+    std::vector<std::pair<uint32_t, uint32_t>> grids;
+    for (const auto &d : b->descs) grids.push_back({d.air.xcells, d.air.ycells});
+    for (int k = 0; k < air::STRIP_PASSES; ++k) {
+        if (occ[k] < 1) TPT_FAIL(TPT_ERR_UNSUPPORTED, "the %ux%u tile kernels do not fit an SM", sh->tx, sh->ty);
+        const size_t before = list.size();
+        air::plan_strips(k, grids, sh->strip_rows, (uint32_t)(b->sms * occ[k] * air::STRIP_WARPS), list);
+        count[k] = (uint32_t)(list.size() - before);
+    }
+    air::StripRef *d = nullptr;
+    TPT_CUDA(cudaMalloc(&d, list.size() * sizeof(air::StripRef)));
+    cudaError_t e = cudaMemcpy(d, list.data(), list.size() * sizeof(air::StripRef), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+        cudaFree(d);
+        TPT_FAIL(TPT_ERR_CUDA, "strip upload failed: %s", cudaGetErrorString(e));
+    }
+    cudaFree(b->strips);
+    b->strips = d;
+    std::copy(count, count + air::STRIP_PASSES, b->nstrips);
+    std::copy(occ, occ + air::STRIP_PASSES, b->occupancy);
     b->shape = sh;
-    b->tile_occupancy_a = occ_a;
-    b->tile_occupancy_b = occ_b;
     return TPT_OK;
 }
 
@@ -640,8 +719,8 @@ int tpt_batch_create(uint32_t n, const tpt_instance_desc *descs, int precision, 
         e = cudaMemcpy(b->insts, b->insts_host.data(), b->insts_host.size() * sizeof(AirInst), cudaMemcpyHostToDevice);
     if (e == cudaSuccess)
         e = cudaMemcpy(b->tiles, tiles.data(), tiles.size() * sizeof(air::TileRef), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc(&b->tile_queue, 2 * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMemset(b->tile_queue, 0, 2 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&b->tile_queue, air::STRIP_PASSES * sizeof(uint32_t));
+    if (e == cudaSuccess) e = cudaMemset(b->tile_queue, 0, air::STRIP_PASSES * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMalloc(&b->ctl, (1 + 2 * (size_t)n) * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemset(b->ctl, 0, (1 + 2 * (size_t)n) * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking);
@@ -652,6 +731,9 @@ int tpt_batch_create(uint32_t n, const tpt_instance_desc *descs, int precision, 
         return bail(TPT_ERR_CUDA);
     }
     b->want = b->ctl + 1;
+    size_t cells = 0;
+    for (uint32_t i = 0; i < n; ++i) cells += (size_t)descs[i].air.xcells * descs[i].air.ycells;
+    b->use_strips = cells >= STRIP_MIN_CELLS;
     rc = set_tile_shape(b, air::tile_shape(DEFAULT_TILE_X, DEFAULT_TILE_Y));
     if (rc) return bail(rc);
     rc = set_sweep_shape(b, DEFAULT_LANES, DEFAULT_ROWS);
@@ -891,9 +973,9 @@ int tpt_batch_profile_phases(tpt_batch *b, uint32_t ticks, tpt_stream_t stream, 
         if (b->descs[i].newton_grav) out->grav_cells += c;
     }
     // sweep form: velocity pre-pass (flagged instances only) + sweep; tile
-    // form: pass A + pass B (+ a settle pass when an instance is NoUpdate with
-    // ambient heat)
-    out->air_launches_per_tick = b->sweep_form() ? 2 : (b->any_noupdate_heat ? 3 : 2);
+    // form: pass A + pass B, which is two launches as strips (+ a settle pass
+    // when an instance is NoUpdate with ambient heat)
+    out->air_launches_per_tick = b->sweep_form() ? 2 : (b->use_strips ? 3 : 2) + (b->any_noupdate_heat ? 1 : 0);
     out->grav_launches_per_tick = b->any_grav ? (b->precision == TPT_PRECISION_FP32 ? 3 : b->dft.launches()) : 0;
     out->grav_flops_per_tick = b->any_grav && b->precision != TPT_PRECISION_FP32 ? b->dft.flops() : 0.0;
     cudaEvent_t e0, e1, e2;
