@@ -240,3 +240,26 @@ def test_c5_batch_concurrent_branches_full_size(cuda, tf, oracle):
             assert emax <= TOL and el2 <= TOL, (i, emax, el2)
         assert_bit_exact(st, oracle.air_steps(inst, 5), f"C5 instance {i}")
     b.close()
+
+
+@pytest.mark.parametrize("shapes", [[(17, 16)], [(127, 129)], [(300, 31)], [(33, 300), (64, 32)],
+                                    [(130 + i, 129 + i) for i in range(26)], [(130 + i, 129 + i) for i in range(40)]],
+                         ids=["17x16", "127x129", "300x31", "two", "width 64", "width 128"])
+def test_split_bf16_tile_widths(cuda, tf, oracle, shapes):
+    """The N tile widths a set's tile count picks: 32 columns (single grids,
+    whose stages are programmatic dependents), 64 (26 grids) and 128 (40),
+    every instance within the FP64 bars, three ticks in a row."""
+    import workloads as W
+
+    insts = [W.make_stress_instance(X, Y, 77 + 13 * X + Y) for X, Y in shapes]
+    b = tf.Batch(insts, precision=tf.PRECISION_SPLIT_BF16)
+    b.step(3)
+    cuda.cuda.synchronize()
+    check_clean(tf)
+    for i, inst in enumerate(insts):
+        got = b.state(i)
+        dx, dy = oracle.grav_solve(inst.xcells, inst.ycells, inst.gmask, mass_fx=inst.mass_fx, dtype=np.float64)
+        for k, d in (("gx", dx), ("gy", dy)):
+            emax, el2 = errors(got[k], d)
+            assert emax <= TOL and el2 <= TOL, (i, k, emax, el2)
+    b.close()

@@ -81,9 +81,9 @@ constexpr uint32_t DEFAULT_TILE_X = 32, DEFAULT_TILE_Y = 8;
 // tick, fewer instructions per cell) instead of tiles (two launches, every cell
 // a thread). Measured on B200 with FP32 gravity beside, us per tick, tiles and
 // strips: 0.55 M cells 77.6 and 82.2, 1.15 M 142.6 and 146.7, 1.81 M 238 and
-// 222, 2.26 M 263 and 241, 3.9 M 500 and 442, 6.1 M 677 and 596, 8.1 M 1003 and
+// 222 (but 33 first ticks of 1.68 M 280 and 283, the walks long), 2.26 M 263 and 241, 3.9 M 500 and 442, 6.1 M 677 and 596, 8.1 M 1003 and
 // 861 (air alone 613 and 454).
-constexpr size_t STRIP_MIN_CELLS = 1500000;
+constexpr size_t STRIP_MIN_CELLS = 2000000;
 
 // Splits every instance into column strips of at most lanes - 2 * SW_H
 // columns and row strips of about `rows` rows (sizes balanced within an
