@@ -105,6 +105,31 @@ def test_grav_gather_repeated_bricks(cuda, oracle, plans, world):
     _same(V.download(bufs, air), d, ("grav_mass",))
 
 
+@pytest.mark.parametrize("n", [1, 16384, 16385, 32768])
+def test_grav_gather_list_lengths(cuda, oracle, plans, world, n):
+    """Both sides of the line between the list order and the memory order,
+    with repeated bricks and with bricks of gravity elements only, then a
+    short list on the same plan: the longer call leaves nothing behind."""
+    import voxel3d as V
+    import workloads as W
+
+    rng = np.random.default_rng(n)
+    d = _copy(world)
+    v = d["voxel"].reshape(256, 256, 256)  # y, z, x
+    v[:64, :64, :] = (v[:64, :64, :] & np.uint32(0xFFFFFF00)) | rng.integers(39, 44, (64, 64, 256), dtype=np.uint32)
+    d["sim_list"] = rng.integers(0, W.VOX_BRICKS, W.VOX_BRICKS).astype(np.uint32)
+    d["sim_count"] = np.array([n, 1, 1], np.uint32)
+    bufs, air = V.upload(d)
+    V.gravity_gather(plans["batched"], bufs)
+    oracle.vox_grav_gather(d)
+    _same(V.download(bufs, air), d, ("grav_mass",))
+    d["sim_count"][0] = 100
+    bufs.sim_count[0] = 100
+    V.gravity_gather(plans["batched"], bufs)
+    oracle.vox_grav_gather(d)
+    _same(V.download(bufs, air), d, ("grav_mass",))
+
+
 @pytest.mark.parametrize("form", sorted(FORMS))
 @pytest.mark.parametrize("iterations", [0, 1, 2, 3, 12])
 def test_air_solve(cuda, oracle, plans, world, form, iterations):

@@ -43,6 +43,9 @@ constexpr int SLAB = PL * PLANE;  // floats per CTA slab
 constexpr size_t CLUSTER_SMEM = 3 * SLAB * sizeof(float);
 static_assert(ROWS * PL * 4 <= 32, "a thread's cells fit one 32-bit mask");
 
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ------------------------------------------------------------- gathers ----
 // One warp per listed brick, persistent warps taking the list in order. Lane
 // l loads the 16 bytes of voxels x = 4*(l & 1) .. +3 of row z = (l >> 1) & 7,
@@ -71,10 +74,16 @@ __device__ __forceinline__ uint32_t cell_sum(uint32_t v) {
 // air_gather_kernel (air_kernel.rs:218-278). The mean temperature's sum is
 // exact in any order (at most 64 multiples of 1/8 below 8192), so it is
 // summed as integers and scaled once.
-__global__ void __launch_bounds__(256) k_air_gather(const uint32_t *__restrict__ voxel,
-                                                    const uint32_t *__restrict__ list,
-                                                    const uint32_t *__restrict__ count, float *__restrict__ solid,
-                                                    float *__restrict__ temp) {
+struct AirGather {
+    struct {
+        const uint32_t *voxel, *list, *count;
+        float *solid, *temp;
+    } w[MAX_BWORLDS];
+};
+__global__ void __launch_bounds__(256) k_air_gather(const __grid_constant__ AirGather G) {
+    const uint32_t *__restrict__ voxel = G.w[blockIdx.y].voxel, *__restrict__ list = G.w[blockIdx.y].list;
+    const uint32_t *__restrict__ count = G.w[blockIdx.y].count;
+    float *__restrict__ solid = G.w[blockIdx.y].solid, *__restrict__ temp = G.w[blockIdx.y].temp;
     const uint32_t n = min(__ldg(count), (uint32_t)TPT_VOX_BRICKS);
     const int lane = threadIdx.x & 31;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -111,70 +120,143 @@ __global__ void __launch_bounds__(256) k_air_gather(const uint32_t *__restrict__
     }
 }
 
-// Per-brick multiplicity of the active list: how many times each brick id
-// is listed (a compaction lists each active brick once). `mult` is cleared
-// before the launch; ids are taken modulo the brick count, as the gathers do.
-__global__ void k_brick_mult(const uint32_t *__restrict__ list, const uint32_t *__restrict__ count,
-                             uint32_t *__restrict__ mult) {
-    const uint32_t n = min(__ldg(count), (uint32_t)TPT_VOX_BRICKS);
-    for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < n; b += gridDim.x * blockDim.x)
-        atomicAdd(mult + (__ldg(list + b) & (TPT_VOX_BRICKS - 1u)), 1u);
-}
-
-// gravity_gather_kernel (gravity.rs:125-166) in memory order. The reference
-// adds each voxel's fixed-point mass to its cell with one atomic per voxel of
-// every listed brick; in wrapping i32 arithmetic the result is each cell's
-// voxel sum times the number of times its brick is listed, in any order.
-// Block (zc, yc) owns the 64 cells of one cell row. Its 16 voxel rows
-// (y = 4 yc + r / 4, z = 4 zc + r % 4) are read as 256-byte runs: warp w
-// holds rows 2w and 2w + 1, one per half-warp, and lane l of a half the word
-// quads of cells xc = 16 j + l, j = 0..3. A cell of an unlisted brick is
-// neither read nor written; aux_tmp is read only for the quads holding GRVT,
-// NBHL or NWHL.
-__global__ void __launch_bounds__(256) k_grav_gather_rows(const uint32_t *__restrict__ voxel,
-                                                          const int32_t *__restrict__ aux,
-                                                          const uint32_t *__restrict__ mult,
-                                                          int32_t *__restrict__ mass) {
-    __shared__ uint32_t part[8][N];
-    const uint32_t zc = blockIdx.x, yc = blockIdx.y;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t l = (uint32_t)lane & 15u, r = 2u * (uint32_t)warp + ((uint32_t)lane >> 4);
-    const uint32_t row = ((4u * yc + (r >> 2)) << 16) | ((4u * zc + (r & 3u)) << 8);
-    const uint32_t bbase = ((yc >> 1) << 10) | ((zc >> 1) << 5);
-    uint32_t s[4];
+// Adds `mult` times the fixed-point mass of a brick's voxels to its eight
+// cells (gravity.rs:74-109, 145-163); `queue` and `part` are this warp's
+// shared memory, `part` zero before and after.
+//
+// An element's mass costs about 40 instructions of selects and conversions,
+// and few voxels are gravity elements, so the warp first queues those: a lane
+// counts its own among its 16 words, a prefix sum over the lanes gives its
+// place, and all lanes evaluate the queue. An entry's low byte holds the
+// element (39..43 as 3..7, bits 0..2) and the cell (bits 3..5).
+__device__ __forceinline__ void gather_brick(const uint32_t *__restrict__ voxel, const int32_t *__restrict__ aux,
+                                             uint32_t brick, uint2 *queue, uint32_t *part, uint32_t mult, int lane,
+                                             int32_t *mass) {
+    const uint32_t base = brick_base(brick);
+    uint4 w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = __ldg(reinterpret_cast<const uint4 *>(voxel + base + lane_offset(lane, j)));
+    uint32_t n = 0u;
+    int4 t[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        const uint32_t xc = 16u * (uint32_t)j + l;
-        s[j] = 0u;
-        if (__ldg(mult + (bbase | (xc >> 1))) == 0u) continue;
-        const uint32_t o = row | (4u * xc);
-        const uint4 w = __ldg(reinterpret_cast<const uint4 *>(voxel + o));
-        const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
-        bool need = false;
+        const uint32_t ws[4] = {w[j].x, w[j].y, w[j].z, w[j].w};
+        bool need = false;  // tmp: GRVT, NBHL, NWHL
 #pragma unroll
-        for (int k = 0; k < 4; ++k) need |= ((ws[k] & 0xFFu) - 39u) < 3u;
-        int4 t = make_int4(0, 0, 0, 0);
-        if (need) t = __ldg(reinterpret_cast<const int4 *>(aux + o));
-        const int32_t ts[4] = {t.x, t.y, t.z, t.w};
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t ty = (ws[k] << 24) - (39u << 24);
+            n += ty < (5u << 24) ? 1u : 0u;
+            need |= ty < (3u << 24);
+        }
+        t[j] = make_int4(0, 0, 0, 0);
+        if (need) t[j] = __ldg(reinterpret_cast<const int4 *>(aux + base + lane_offset(lane, j)));
+    }
+    uint32_t at = n;  // inclusive prefix sum
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, at, d);
+        if (lane >= d) at += v;
+    }
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, at, 31);
+    if (total == 0u) return;
+    uint2 *q = queue + (at - n);
+    const uint32_t cell = (((uint32_t)lane & 1u) << 3) | (((uint32_t)lane & 8u) << 1);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const uint32_t ws[4] = {w[j].x, w[j].y, w[j].z, w[j].w};
+        const int32_t ts[4] = {t[j].x, t[j].y, t[j].z, t[j].w};
+        const uint32_t tag = cell + ((uint32_t)(j >> 1) << 5) - 36u;
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            s[j] += (uint32_t)voxel_mass(ws[k] & 0xFFu, (ws[k] >> 24) & 0xFFu, ts[k], (ws[k] >> 8) & 0xFFFFu);
+            if ((ws[k] << 24) - (39u << 24) < (5u << 24)) *q++ = make_uint2(ws[k] + tag, (uint32_t)ts[k]);
     }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        s[j] += __shfl_xor_sync(0xFFFFFFFFu, s[j], 16);
-        if (lane < 16) part[warp][16 * j + (int)l] = s[j];
+    __syncwarp();
+    // four sums per cell, so that the lanes' additions fall into all banks
+    for (uint32_t i = (uint32_t)lane; i < total; i += 32u) {
+        const uint2 e = queue[i];
+        const int32_t m = voxel_mass((e.x & 7u) + 36u, e.x >> 24, (int32_t)e.y, (e.x >> 8) & 0xFFFFu);
+        atomicAdd(part + (((e.x >> 1) & 0x1Cu) | (lane & 3)), (uint32_t)m);
     }
-    __syncthreads();
-    if (threadIdx.x < (unsigned)N) {
-        const uint32_t xc = threadIdx.x, m = __ldg(mult + (bbase | (xc >> 1)));
-        if (m != 0u) {
-            uint32_t tot = 0u;
+    __syncwarp();
+    uint32_t tot = part[lane];
+    part[lane] = 0u;
+    tot += __shfl_xor_sync(0xFFFFFFFFu, tot, 1);
+    tot += __shfl_xor_sync(0xFFFFFFFFu, tot, 2);
+    if ((lane & 3) == 0 && tot != 0u) {
+        const uint32_t c = (uint32_t)lane >> 2;  // x, z, y from bit 0
+        atomicAdd(reinterpret_cast<uint32_t *>(mass) + brick_cell(brick, c & 1u, c >> 2, (c >> 1) & 1u), mult * tot);
+    }
+    __syncwarp();
+}
+
+// gravity_gather_kernel (gravity.rs:125-166). The reference adds each voxel's
+// fixed-point mass to its cell with one atomic per voxel of every listed
+// brick; in wrapping i32 arithmetic the result is each cell's voxel sum times
+// the number of times its brick is listed, in any order.
+//
+// What bounds it is DRAM: a listed brick is 64 runs of 32 bytes of voxels and
+// the runs of aux_tmp beside its GRVT, NBHL and NWHL, and a DRAM burst holds
+// the runs of two or more neighbouring bricks. A list in no order reads bursts
+// twice when its neighbours are listed too, so:
+//
+//   up to LIST_BRICKS  k_grav_gather_list takes the list as it is, one warp
+//                      per listed brick;
+//   above              it counts how often each brick is listed, and
+//                      k_grav_gather_rows, launched behind it in any case,
+//                      takes the bricks in memory order: a block owns a row
+//                      of 32 bricks along x and its warps the row's listed
+//                      ones in turn, and it clears the row's counts for the
+//                      next call.
+//
+// Measured on B200, us per world over eight worlds in turn (1 GB of voxels and
+// aux_tmp), both launches, list against rows: 30% of the bricks listed 22.5 /
+// 24.5, 45% 27.5 / 27.2, 60% 30.8 (list alone) / 30.1, 80% 36.9 (list alone) /
+// 32.9, all 43.7 (list alone) / 34.9; the line lies at half. Evaluating every
+// voxel of whole cell rows took 44.6 at 30% and 45.7 with all: it was bound by
+// the integer pipe. The compulsory bytes of all bricks take about 20 us.
+constexpr uint32_t LIST_BRICKS = TPT_VOX_BRICKS / 2;
+constexpr int GATHER_WARPS = 4;
+
+__global__ void __launch_bounds__(GATHER_WARPS * 32) k_grav_gather_list(
+    const uint32_t *__restrict__ voxel, const int32_t *__restrict__ aux, const uint32_t *__restrict__ list,
+    const uint32_t *__restrict__ count, uint32_t *__restrict__ mult, int32_t *__restrict__ mass) {
+    __shared__ uint2 queue[GATHER_WARPS][512];
+    __shared__ uint32_t part[GATHER_WARPS][32];
+    pdl_release();
+    const uint32_t n = min(__ldg(count), (uint32_t)TPT_VOX_BRICKS);
+    if (n > LIST_BRICKS) {
+        for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < n; b += gridDim.x * blockDim.x)
+            atomicAdd(mult + (__ldg(list + b) & (TPT_VOX_BRICKS - 1u)), 1u);
+        return;
+    }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    part[warp][lane] = 0u;
+    __syncwarp();
+    for (uint32_t b = blockIdx.x * GATHER_WARPS + warp; b < n; b += gridDim.x * GATHER_WARPS)
+        gather_brick(voxel, aux, __ldg(list + b) & (TPT_VOX_BRICKS - 1u), queue[warp], part[warp], 1u, lane, mass);
+}
+
+__global__ void __launch_bounds__(GATHER_WARPS * 32) k_grav_gather_rows(
+    const uint32_t *__restrict__ voxel, const int32_t *__restrict__ aux, const uint32_t *__restrict__ count,
+    uint32_t *mult, int32_t *__restrict__ mass) {
+    __shared__ uint2 queue[GATHER_WARPS][512];
+    __shared__ uint32_t part[GATHER_WARPS][32];
+    pdl_wait();
+    if (__ldg(count) <= LIST_BRICKS) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t bbase = blockIdx.x << 5;
+    part[warp][lane] = 0u;
+    const uint32_t mine = __ldcg(mult + bbase + lane);
+    uint32_t listed = __ballot_sync(0xFFFFFFFFu, mine != 0u);
+    __syncthreads();  // every warp has read the row
+    if (warp == 0 && mine != 0u) mult[bbase + lane] = 0u;
+    for (int i = 0; i < warp; ++i) listed &= listed - 1u;
+    while (listed != 0u) {
+        const int b = __ffs(listed) - 1;
+        gather_brick(voxel, aux, bbase + (uint32_t)b, queue[warp], part[warp], __shfl_sync(0xFFFFFFFFu, mine, b), lane,
+                     mass);
 #pragma unroll
-            for (int w = 0; w < 8; ++w) tot += part[w][xc];
-            uint32_t *c = reinterpret_cast<uint32_t *>(mass) + ((yc << 12) | (zc << 6) | xc);
-            *c += m * tot;
-        }
+        for (int i = 0; i < GATHER_WARPS; ++i) listed &= listed - 1u;
     }
 }
 
@@ -654,17 +736,35 @@ static int gather_blocks(int per_sm) {
     return sms * per_sm;
 }
 
-int launch_air_gather(const World &w, cudaStream_t st) {
-    k_air_gather<<<gather_blocks(8), 256, 0, st>>>(w.voxel, w.sim_list, w.sim_count, w.solid, w.temp);
+int launch_air_gather(const World *w, uint32_t n, cudaStream_t st) {
+    AirGather G{};
+    for (uint32_t i = 0; i < n; ++i) G.w[i] = {w[i].voxel, w[i].sim_list, w[i].sim_count, w[i].solid, w[i].temp};
+    k_air_gather<<<dim3(gather_blocks(n == 1 ? 8 : 4), n), 256, 0, st>>>(G);
     TPT_LAUNCHED();
     return TPT_OK;
 }
 
 int launch_grav_gather(const World &w, uint32_t *brick_mult, cudaStream_t st) {
-    TPT_CUDA(cudaMemsetAsync(brick_mult, 0, TPT_VOX_BRICKS * sizeof(uint32_t), st));
-    k_brick_mult<<<TPT_VOX_BRICKS / 256, 256, 0, st>>>(w.sim_list, w.sim_count, brick_mult);
+    k_grav_gather_list<<<gather_blocks(8), GATHER_WARPS * 32, 0, st>>>(w.voxel, w.aux_tmp, w.sim_list, w.sim_count,
+                                                                       brick_mult, w.grav_mass);
     TPT_LAUNCHED();
-    k_grav_gather_rows<<<dim3(N, N), 256, 0, st>>>(w.voxel, w.aux_tmp, brick_mult, w.grav_mass);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(TPT_VOX_BRICKS / 32);
+    cfg.blockDim = dim3(GATHER_WARPS * 32);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_grav_gather_rows, (const uint32_t *)w.voxel,
+                                             (const int32_t *)w.aux_tmp, (const uint32_t *)w.sim_count, brick_mult,
+                                             w.grav_mass);
+    if (e != cudaSuccess) {
+        // the counts must not stay for the next call
+        cudaMemsetAsync(brick_mult, 0, TPT_VOX_BRICKS * sizeof(uint32_t), st);
+        TPT_CUDA(e);
+    }
     TPT_LAUNCHED();
     return TPT_OK;
 }

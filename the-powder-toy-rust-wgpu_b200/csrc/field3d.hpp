@@ -76,8 +76,10 @@ constexpr size_t BATCH_SCRATCH_BYTES = 5u * TPT_VOX_CELLS * sizeof(float) + TPT_
 int launch_batch(Batch &b, cudaStream_t st);
 
 int launch_air_clear(const World &w, cudaStream_t st);
-int launch_air_gather(const World &w, cudaStream_t st);
-// gravity::gather; brick_mult is TPT_VOX_BRICKS words of scratch.
+// air::gather of n <= MAX_BWORLDS worlds in one launch.
+int launch_air_gather(const World *w, uint32_t n, cudaStream_t st);
+// gravity::gather; brick_mult is TPT_VOX_BRICKS words of scratch, zero before
+// and after.
 int launch_grav_gather(const World &w, uint32_t *brick_mult, cudaStream_t st);
 int launch_grav_clear(const World &w, cudaStream_t st);
 // Whether the device can hold one cluster of the cluster kernel.

@@ -12,7 +12,8 @@ struct tpt_vox_plan {
     // Cluster form: one AirScratch (4 fields) per world of a launch.
     // Batched form: BATCH_SCRATCH_BYTES per world of a launch.
     float *scratch = nullptr;
-    uint32_t *brick_mult = nullptr;  // the gravity gather's per-brick list multiplicity
+    // the gravity gather's per-brick list multiplicity, zero between calls
+    uint32_t *brick_mult = nullptr;
     tpt::vox::AirScratch slot(uint32_t i) const {
         float *b = scratch + (size_t)i * tpt::vox::AIR_SCRATCH_FLOATS;
         return {b, b + TPT_VOX_CELLS};
@@ -147,7 +148,9 @@ int tpt_vox_plan_create(int form, tpt_vox_plan **out) {
     if (p->form == TPT_VOX_CLUSTER) bytes = (size_t)(vox::MAX_JOBS / 2) * vox::AIR_SCRATCH_FLOATS * sizeof(float);
     if (p->form == TPT_VOX_BATCHED) bytes = (size_t)vox::MAX_BWORLDS * vox::BATCH_SCRATCH_BYTES;
     cudaError_t e = cudaMalloc(&p->scratch, bytes);
-    if (e == cudaSuccess) e = cudaMalloc(&p->brick_mult, TPT_VOX_BRICKS * sizeof(uint32_t));
+    const size_t table = TPT_VOX_BRICKS * sizeof(uint32_t);
+    if (e == cudaSuccess) e = cudaMalloc(&p->brick_mult, table);
+    if (e == cudaSuccess) e = cudaMemset(p->brick_mult, 0, table);
     if (e != cudaSuccess) {
         cudaFree(p->scratch);
         delete p;
@@ -183,7 +186,8 @@ int tpt_vox_air_gather(tpt_vox_plan *plan, const tpt_vox_world *w, tpt_stream_t 
     int rc = check_gather(w);
     if (!rc) rc = check_ptrs("air gather", {w->solid, w->temp});
     if (rc) return rc;
-    return vox::launch_air_gather(world_of(*w), (cudaStream_t)stream);
+    const vox::World v = world_of(*w);
+    return vox::launch_air_gather(&v, 1, (cudaStream_t)stream);
 }
 
 int tpt_vox_air_solve(tpt_vox_plan *plan, const tpt_vox_world *w, uint32_t iterations, tpt_stream_t stream) {
@@ -241,15 +245,15 @@ int tpt_vox_field_step(tpt_vox_plan *plan, const tpt_vox_world *worlds, uint32_t
     }
     cudaStream_t st = (cudaStream_t)stream;
     if (plan->form == TPT_VOX_BATCHED) {
-        // per group of up to MAX_BWORLDS worlds: every world's gather, then
+        // per group of up to MAX_BWORLDS worlds: one launch of their gathers, then
         // one batched launch sequence of air and gravity for all of them
         for (uint32_t first = 0; first < n; first += vox::MAX_BWORLDS) {
             const uint32_t m = n - first < vox::MAX_BWORLDS ? n - first : vox::MAX_BWORLDS;
-            for (uint32_t i = first; i < first + m; ++i) {
-                int rc = vox::launch_air_gather(world_of(worlds[i]), st);
-                if (rc) return rc;
-            }
-            int rc = run_batch(plan, worlds + first, m, 3u, air_iterations, true, st);
+            vox::World v[vox::MAX_BWORLDS];
+            for (uint32_t i = 0; i < m; ++i) v[i] = world_of(worlds[first + i]);
+            int rc = vox::launch_air_gather(v, m, st);
+            if (rc) return rc;
+            rc = run_batch(plan, worlds + first, m, 3u, air_iterations, true, st);
             if (rc) return rc;
         }
         return TPT_OK;
@@ -257,7 +261,7 @@ int tpt_vox_field_step(tpt_vox_plan *plan, const tpt_vox_world *worlds, uint32_t
     if (plan->form != TPT_VOX_CLUSTER) {
         for (uint32_t i = 0; i < n; ++i) {
             const vox::World v = world_of(worlds[i]);
-            int rc = vox::launch_air_gather(v, st);
+            int rc = vox::launch_air_gather(&v, 1, st);
             if (!rc) rc = vox::launch_air_per_sweep(v, air_iterations, plan->scratch, st);
             if (!rc) rc = vox::launch_grav_per_sweep(v, st);
             if (!rc) rc = vox::launch_grav_clear(v, st);
@@ -274,7 +278,7 @@ int tpt_vox_field_step(tpt_vox_plan *plan, const tpt_vox_world *worlds, uint32_t
         for (uint32_t i = first; i < last; ++i) {
             const vox::World v = world_of(worlds[i]);
             const vox::AirScratch sc = plan->slot(i - first);
-            int rc = vox::launch_air_gather(v, st);
+            int rc = vox::launch_air_gather(&v, 1, st);
             if (!rc) rc = vox::launch_air_prep(v, sc, st);
             if (rc) return rc;
             jobs.job[jobs.n++] = vox::air_job_of(v, air_iterations, sc);
