@@ -178,3 +178,28 @@ def test_field_step_three_worlds_two_ticks(cuda, oracle, plans, world, form):
             oracle.vox_field_step(d, 12)
         for w, (d, (bufs, air)) in enumerate(zip(hosts, devs)):
             _same(V.download(bufs, air), d, AIR_KEYS + GRAV_KEYS + ("solid", "temp"), f"{form} tick {tick} world {w}: ")
+
+
+@pytest.mark.parametrize("worlds, iterations", [(4, 3), (17, 2)])
+def test_field_step_many_worlds(cuda, oracle, plans, world, worlds, iterations):
+    """The batched form's layouts for many worlds, and more worlds than one
+    launch takes; solid and pinned cells differ per world."""
+    import voxel3d as V
+    import workloads as W
+
+    rng = np.random.default_rng(11)
+    hosts = []
+    for w in range(worlds):
+        d = _copy(world)
+        n = [300, 1, 0][w % 3]
+        d["sim_list"] = rng.permutation(W.VOX_BRICKS)[: max(n, 1)].astype(np.uint32)
+        d["sim_count"] = np.array([n, 1, 1], np.uint32)
+        d["solid"] = np.roll(d["solid"], 5 * w)
+        d["vy"] = np.roll(d["vy"], 131 * w)
+        d["grav_mass"] = np.roll(d["grav_mass"], 4099 * w)
+        hosts.append(d)
+    devs = [V.upload(d) for d in hosts]
+    V.field_step(plans["batched"], devs, iterations)
+    for w, (d, (bufs, air)) in enumerate(zip(hosts, devs)):
+        oracle.vox_field_step(d, iterations)
+        _same(V.download(bufs, air), d, AIR_KEYS + GRAV_KEYS + ("solid", "temp"), f"world {w}: ")

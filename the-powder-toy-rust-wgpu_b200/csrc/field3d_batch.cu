@@ -9,9 +9,9 @@
 //           reference recomputes in every sweep.
 //   sweep s one launch per sweep index: the air sweep of every world while
 //           s < air iterations and the gravity sweep of every world while
-//           s < 24, side by side in the same grid. A thread updates one
-//           x-quad (4 cells, a float4); the x neighbours outside the quad
-//           come from the adjacent lanes.
+//           s < 24, side by side in the same grid. A thread updates x-quads
+//           (4 cells, a float4); the x neighbours outside the quad come from
+//           the adjacent lanes.
 //   finish  grid-wide, once: the air advection, the gravity force and the
 //           mass clear.
 //
@@ -30,10 +30,10 @@ namespace vox {
 namespace {
 
 constexpr int QUADS = CELLS / 4;
-constexpr int QBLOCK = 256;             // quads per block
-constexpr int QBLOCKS = QUADS / QBLOCK; // blocks per field of a world
-constexpr int CBLOCK = 256;             // cells per block of the per-cell passes
-constexpr int CBLOCKS = CELLS / CBLOCK;
+constexpr int PBLOCK = 128;             // quads per block of the passes around the sweeps
+constexpr int PBLOCKS = QUADS / PBLOCK;
+// Worlds from which a sweep's thread takes two quads (see k_b_sweep).
+constexpr uint32_t MANY_WORLDS = 4;
 static_assert(TPT_VOX_GRAV_ITERATIONS % 2 == 0, "an even sweep count leaves the last sweep in grav_potential");
 
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -45,47 +45,109 @@ __device__ __forceinline__ int field_of(uint32_t fields, int z) {
     return (fields & 1u) ? z : 1;
 }
 
-__global__ void __launch_bounds__(CBLOCK) k_b_prep(const __grid_constant__ Batch B) {
-    pdl_launch_dependents();
-    pdl_wait();
-    const BWorld &w = B.w[blockIdx.y];
-    const int f = field_of(B.fields, blockIdx.z);
-    const int i = blockIdx.x * CBLOCK + threadIdx.x;
-    int x, y, z;
-    coords(i, x, y, z);
-    if (f == 1) {
-        w.src[i] = grav_source(w.mass[i]);
-        return;
-    }
-    const float *vx = w.vx, *vy = w.vy, *vz = w.vz;
-    w.snap[i] = vx[i];
-    w.snap[CELLS + i] = vy[i];
-    w.snap[2 * CELLS + i] = vz[i];
-    const bool inner = x > 0 && y > 0 && z > 0 && x < N - 1 && y < N - 1 && z < N - 1;
-    const bool rim = x < 2 || x >= N - 2 || y < 2 || y >= N - 2 || z < 2 || z >= N - 2;
-    float dp = 0.0f, d = 0.0f;
-    if (inner) {
-        const float xm = vx[i - 1], xp = vx[i + 1], ym = vy[i - SY], yp = vy[i + SY], zm = vz[i - SZ],
-                    zp = vz[i + SZ];
-        dp = (xm - xp) + (ym - yp) + (zm - zp);
-        d = 0.5f * ((xp - xm) + (yp - ym) + (zp - zm));
-    }
-    w.div[i] = d;
-    w.pv[i] = pv_update(w.pv[i], rim, dp);  // the rim holds every cell outside `inner`
-    // pin mask of the quad: lanes 4k .. 4k+3 hold one quad's cells
-    const bool pinned = !inner || w.solid[i] > 0.5f;
-    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, pinned);
-    const int lane = threadIdx.x & 31;
-    if ((lane & 3) == 0) w.pin[i >> 2] = (uint8_t)((bal >> lane) & 0xFu);
+// The passes around the sweeps move every field of a world once and are bound
+// by DRAM when the worlds are many. A thread takes a quad, so a field's
+// neighbours are five float4 loads and two shuffles instead of 28 word loads:
+// the whole step with the layouts below, 1 / 2 / 4 / 8 worlds, went from 65 /
+// 104 / 165 / 284 us to 65 / 96 / 149 / 248.
+
+// A quad's neighbourhood of one field: its cells, the quads beside it in z and
+// y (zero outside the world) and the cells before and after it in x, from the
+// adjacent lanes (unused at the world's faces).
+struct Quad {
+    float4 c, zm, zp, ym, yp;
+    float l, r;
+    __device__ __forceinline__ float xm(int k) const { return k == 0 ? l : f4(c, k - 1); }
+    __device__ __forceinline__ float xp(int k) const { return k == 3 ? r : f4(c, k + 1); }
+};
+__device__ __forceinline__ void quad_x(Quad &q) {
+    q.l = __shfl_up_sync(0xFFFFFFFFu, q.c.w, 1, 16);
+    q.r = __shfl_down_sync(0xFFFFFFFFu, q.c.x, 1, 16);
+}
+__device__ __forceinline__ Quad load_quad(const float *a, int i0, int y, int z) {
+    Quad q;
+    q.c = ld4(a + i0);
+    q.zm = z > 0 ? ld4(a + i0 - SZ) : zero4();
+    q.zp = z + 1 < N ? ld4(a + i0 + SZ) : zero4();
+    q.ym = y > 0 ? ld4(a + i0 - SY) : zero4();
+    q.yp = y + 1 < N ? ld4(a + i0 + SY) : zero4();
+    quad_x(q);
+    return q;
 }
 
-__global__ void __launch_bounds__(QBLOCK) k_b_sweep(const __grid_constant__ Batch B, uint32_t s) {
+__global__ void __launch_bounds__(PBLOCK) k_b_prep(const __grid_constant__ Batch B) {
     pdl_launch_dependents();
     pdl_wait();
     const BWorld &w = B.w[blockIdx.y];
     const int f = field_of(B.fields, blockIdx.z);
-    const int q = blockIdx.x * QBLOCK + threadIdx.x;
+    const int q = blockIdx.x * PBLOCK + threadIdx.x;
     const int i0 = 4 * q, x0 = i0 & 63, z = (i0 >> 6) & 63, y = i0 >> 12;
+    if (f == 1) {
+        const int4 m = *reinterpret_cast<const int4 *>(w.mass + i0);
+        st4(w.src + i0, make_float4(grav_source(m.x), grav_source(m.y), grav_source(m.z), grav_source(m.w)));
+        return;
+    }
+    const bool row = y > 0 && z > 0 && y < N - 1 && z < N - 1;  // off the y and z faces
+    const bool row_rim = y < 2 || y >= N - 2 || z < 2 || z >= N - 2;
+    Quad vx;
+    vx.c = ld4(w.vx + i0);
+    const float4 vy = ld4(w.vy + i0), vz = ld4(w.vz + i0), solid = ld4(w.solid + i0);
+    const int4 pv = *reinterpret_cast<const int4 *>(w.pv + i0);
+    const float4 ym = row ? ld4(w.vy + i0 - SY) : zero4(), yp = row ? ld4(w.vy + i0 + SY) : zero4();
+    const float4 zm = row ? ld4(w.vz + i0 - SZ) : zero4(), zp = row ? ld4(w.vz + i0 + SZ) : zero4();
+    quad_x(vx);
+    const int32_t pvs[4] = {pv.x, pv.y, pv.z, pv.w};
+    int32_t pn[4];
+    float4 div;
+    uint32_t pins = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int x = x0 + k;
+        const bool inner = row && x > 0 && x < N - 1, rim = row_rim || x < 2 || x >= N - 2;
+        const float xm = vx.xm(k), xp = vx.xp(k);
+        const float dp = (xm - xp) + (f4(ym, k) - f4(yp, k)) + (f4(zm, k) - f4(zp, k));
+        const float d = 0.5f * ((xp - xm) + (f4(yp, k) - f4(ym, k)) + (f4(zp, k) - f4(zm, k)));
+        f4set(div, k, inner ? d : 0.0f);
+        pn[k] = pv_update(pvs[k], rim, dp);  // the rim holds every cell outside `inner`
+        if (!inner || f4(solid, k) > 0.5f) pins |= 1u << k;
+    }
+    st4(w.snap + i0, vx.c);
+    st4(w.snap + CELLS + i0, vy);
+    st4(w.snap + 2 * CELLS + i0, vz);
+    st4(w.div + i0, div);
+    *reinterpret_cast<int4 *>(w.pv + i0) = make_int4(pn[0], pn[1], pn[2], pn[3]);
+    w.pin[q] = (uint8_t)pins;
+}
+
+// One sweep. A thread takes the quads of YPT planes, one above the other, and
+// a block BZ rows in z: the quads beside its own in y and z are its own in
+// other threads' loads, or on the way into L1 for them. What bounds it is L1
+// and the latency of one dependent round to L2, where the fields stay; of the
+// layouts, (YPT, BZ, threads), measured on B200 as whole field steps with 12
+// air sweeps and 30% of the bricks listed, us for 1 / 2 / 4 / 8 worlds:
+//
+//   (1, 16, 256), a strip of 16 rows  66 / 108 / 177 / 310
+//   (1, 4, 256)                       65 / 104 / 167 / 295   below 4 worlds
+//   (2, 8, 128)                       67 / 109 / 165 / 284   from 4 worlds on
+//   (2, 8, 256)                       73 / 106 / 166 / 292
+//   (4, 8, 128)                       80 / 121 / 172 / 298
+//
+// Two quads a thread load 4 quads each instead of 5 but leave few warps when
+// the worlds are few. Several sweeps per launch over tiles with halo rows in
+// shared memory were slower for every number of worlds (two sweeps: 68 / 120 /
+// 194 / 363 at best): the halo's redundant cells and the shared-memory traffic
+// outweigh the launches.
+template <int YPT, int BZ, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_b_sweep(const __grid_constant__ Batch B, uint32_t s) {
+    constexpr int BY = THREADS / 16 / BZ * YPT;  // planes of a block
+    pdl_launch_dependents();
+    pdl_wait();
+    const BWorld &w = B.w[blockIdx.y];
+    const int f = field_of(B.fields, blockIdx.z);
+    const int x0 = 4 * (threadIdx.x & 15), row = threadIdx.x >> 4;
+    const int z = (int)(blockIdx.x % (N / BZ)) * BZ + row % BZ;
+    const int y0 = (int)(blockIdx.x / (N / BZ)) * BY + row / BZ * YPT;
+    const int i0 = y0 * SY + z * SZ + x0;
     const bool even = (s & 1u) == 0u;
     const float *S;
     float *T;
@@ -96,88 +158,100 @@ __global__ void __launch_bounds__(QBLOCK) k_b_sweep(const __grid_constant__ Batc
         S = even ? w.pot : w.pot_tmp;
         T = even ? w.pot_tmp : w.pot;
     }
-    const float4 c = ld4(S + i0);
-    const float l = __shfl_up_sync(0xFFFFFFFFu, c.w, 1, 16);
-    const float r = __shfl_down_sync(0xFFFFFFFFu, c.x, 1, 16);
-    const float4 zm = z > 0 ? ld4(S + i0 - SZ) : zero4(), zp = z + 1 < N ? ld4(S + i0 + SZ) : zero4();
-    const float4 ym = y > 0 ? ld4(S + i0 - SY) : zero4(), yp = y + 1 < N ? ld4(S + i0 + SY) : zero4();
-    float4 out;
-    if (f == 0) {
-        const float4 d = ld4(w.div + i0);
-        const uint32_t pins = w.pin[q];
+    const float *source = f == 0 ? w.div : w.src;
+    float4 c[YPT + 2], zm[YPT], zp[YPT], sr[YPT];
+    c[0] = y0 > 0 ? ld4(S + i0 - SY) : zero4();
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const float xm = k == 0 ? l : f4(c, k - 1), xp = k == 3 ? r : f4(c, k + 1);
-            f4set(out, k, air_sweep_cell(xm, xp, f4(zm, k), f4(zp, k), f4(ym, k), f4(yp, k), f4(d, k),
-                                         (pins >> k) & 1u));
-        }
-    } else {
-        const float4 sr = ld4(w.src + i0);
-        const bool face = y == 0 || z == 0 || y == N - 1 || z == N - 1;
+    for (int j = 0; j < YPT; ++j) c[j + 1] = ld4(S + i0 + j * SY);
+    c[YPT + 1] = y0 + YPT < N ? ld4(S + i0 + YPT * SY) : zero4();
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const int x = x0 + k;
-            const float xm = k == 0 ? l : f4(c, k - 1), xp = k == 3 ? r : f4(c, k + 1);
-            f4set(out, k, grav_sweep_cell(xm, xp, f4(zm, k), f4(zp, k), f4(ym, k), f4(yp, k), f4(sr, k), f4(c, k),
-                                          face || x == 0 || x == N - 1));
-        }
+    for (int j = 0; j < YPT; ++j) {
+        zm[j] = z > 0 ? ld4(S + i0 + j * SY - SZ) : zero4();
+        zp[j] = z + 1 < N ? ld4(S + i0 + j * SY + SZ) : zero4();
+        sr[j] = ld4(source + i0 + j * SY);
     }
-    st4(T + i0, out);
+#pragma unroll
+    for (int j = 0; j < YPT; ++j) {
+        const int y = y0 + j;
+        const float l = __shfl_up_sync(0xFFFFFFFFu, c[j + 1].w, 1, 16);
+        const float r = __shfl_down_sync(0xFFFFFFFFu, c[j + 1].x, 1, 16);
+        float4 out;
+        if (f == 0) {
+            const uint32_t pins = w.pin[(i0 + j * SY) >> 2];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float xm = k == 0 ? l : f4(c[j + 1], k - 1), xp = k == 3 ? r : f4(c[j + 1], k + 1);
+                f4set(out, k, air_sweep_cell(xm, xp, f4(zm[j], k), f4(zp[j], k), f4(c[j], k), f4(c[j + 2], k),
+                                             f4(sr[j], k), (pins >> k) & 1u));
+            }
+        } else {
+            const bool face = y == 0 || z == 0 || y == N - 1 || z == N - 1;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int x = x0 + k;
+                const float xm = k == 0 ? l : f4(c[j + 1], k - 1), xp = k == 3 ? r : f4(c[j + 1], k + 1);
+                f4set(out, k, grav_sweep_cell(xm, xp, f4(zm[j], k), f4(zp[j], k), f4(c[j], k), f4(c[j + 2], k),
+                                              f4(sr[j], k), f4(c[j + 1], k), face || x == 0 || x == N - 1));
+            }
+        }
+        st4(T + i0 + j * SY, out);
+    }
 }
 
-__global__ void __launch_bounds__(CBLOCK) k_b_finish(const __grid_constant__ Batch B) {
+__global__ void __launch_bounds__(PBLOCK) k_b_finish(const __grid_constant__ Batch B) {
     pdl_launch_dependents();
     pdl_wait();
     const BWorld &w = B.w[blockIdx.y];
     const int f = field_of(B.fields, blockIdx.z);
-    const int i = blockIdx.x * CBLOCK + threadIdx.x;
-    int x, y, z;
-    coords(i, x, y, z);
-    const bool hxm = x > 0, hxp = x + 1 < N, hzm = z > 0, hzp = z + 1 < N, hym = y > 0, hyp = y + 1 < N;
-    auto at = [&](const float *a, bool ok, int j) { return ok ? a[j] : 0.0f; };
+    const int i0 = 4 * (int)(blockIdx.x * PBLOCK + threadIdx.x), x0 = i0 & 63, z = (i0 >> 6) & 63, y = i0 >> 12;
     if (f == 1) {
         // gravity_force_kernel (gravity.rs:199-224) on the last sweep, then
         // gravity_clear_kernel (gravity.rs:112-118) when asked
-        const float *u = w.pot;
-        const bool boundary = !(hxm && hxp && hym && hyp && hzm && hzp);
-        if (boundary) {
-            w.fx[i] = seed_f32(u[i], 0.0f);
-            w.fy[i] = seed_f32(u[i], 0.0f);
-            w.fz[i] = seed_f32(u[i], 0.0f);
-        } else {
-            w.fx[i] = (u[i - 1] - u[i + 1]) * 0.5f;
-            w.fz[i] = (u[i - SZ] - u[i + SZ]) * 0.5f;
-            w.fy[i] = (u[i - SY] - u[i + SY]) * 0.5f;
+        const Quad u = load_quad(w.pot, i0, y, z);
+        const bool face = y == 0 || z == 0 || y == N - 1 || z == N - 1;
+        float4 fx, fy, fz;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const bool boundary = face || x0 + k == 0 || x0 + k == N - 1;
+            const float seed = seed_f32(f4(u.c, k), 0.0f);
+            f4set(fx, k, boundary ? seed : (u.xm(k) - u.xp(k)) * 0.5f);
+            f4set(fz, k, boundary ? seed : (f4(u.zm, k) - f4(u.zp, k)) * 0.5f);
+            f4set(fy, k, boundary ? seed : (f4(u.ym, k) - f4(u.yp, k)) * 0.5f);
         }
-        if (B.clear_mass) w.mass[i] = 0;
+        st4(w.fx + i0, fx);
+        st4(w.fy + i0, fy);
+        st4(w.fz + i0, fz);
+        if (B.clear_mass) *reinterpret_cast<int4 *>(w.mass + i0) = make_int4(0, 0, 0, 0);
         return;
     }
     // air_advect_kernel (air_kernel.rs:414-536) from the snapshot
-    if (w.solid[i] > 0.5f) {
-        w.vx[i] = 0.0f;
-        w.vy[i] = 0.0f;
-        w.vz[i] = 0.0f;
-        return;
+    const float4 solid = ld4(w.solid + i0);
+    const Quad t = load_quad(w.temp, i0, y, z);
+    float4 buoy;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float lt = nb_average(f4(t.c, k), t.xm(k), t.xp(k), f4(t.zm, k), f4(t.zp, k), f4(t.ym, k), f4(t.yp, k),
+                                    x0 + k, y, z);
+        f4set(buoy, k, (lt - kAmbient) * kBuoyancy);
     }
-    const float *pr = (B.air_iters & 1u) ? w.p_tmp : w.p;  // the last sweep's buffer
-    const float *temp = w.temp, *snap = w.snap;
-    const float lt = nb_average(temp[i], at(temp, hxm, i - 1), at(temp, hxp, i + 1), at(temp, hzm, i - SZ),
-                                at(temp, hzp, i + SZ), at(temp, hym, i - SY), at(temp, hyp, i + SY), x, y, z);
-    const float buoy = (lt - kAmbient) * kBuoyancy;
-    const float pc = pr[i];
-    const float grad[3] = {pressure_grad(at(pr, hxm, i - 1), at(pr, hxp, i + 1), pc, x),
-                           pressure_grad(at(pr, hym, i - SY), at(pr, hyp, i + SY), pc, y),
-                           pressure_grad(at(pr, hzm, i - SZ), at(pr, hzp, i + SZ), pc, z)};
-    float out[3];
+    const Quad p = load_quad((B.air_iters & 1u) ? w.p_tmp : w.p, i0, y, z);  // the last sweep's buffer
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const float *sn = snap + (size_t)a * CELLS;
-        out[a] = advect_cell(sn[i], at(sn, hxm, i - 1), at(sn, hxp, i + 1), at(sn, hzm, i - SZ), at(sn, hzp, i + SZ),
-                             at(sn, hym, i - SY), at(sn, hyp, i + SY), a, grad[a], a == 1 ? buoy : 0.0f, x, y, z);
+        const Quad v = load_quad(w.snap + (size_t)a * CELLS, i0, y, z);
+        float4 out;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int x = x0 + k;
+            const float pc = f4(p.c, k);
+            const float grad = a == 0   ? pressure_grad(p.xm(k), p.xp(k), pc, x)
+                               : a == 1 ? pressure_grad(f4(p.ym, k), f4(p.yp, k), pc, y)
+                                        : pressure_grad(f4(p.zm, k), f4(p.zp, k), pc, z);
+            const float o = advect_cell(f4(v.c, k), v.xm(k), v.xp(k), f4(v.zm, k), f4(v.zp, k), f4(v.ym, k),
+                                        f4(v.yp, k), a, grad, a == 1 ? f4(buoy, k) : 0.0f, x, y, z);
+            f4set(out, k, f4(solid, k) > 0.5f ? 0.0f : o);
+        }
+        st4((a == 0 ? w.vx : a == 1 ? w.vy : w.vz) + i0, out);
     }
-    w.vx[i] = out[0];
-    w.vy[i] = out[1];
-    w.vz[i] = out[2];
 }
 
 template <typename... Args>
@@ -196,12 +270,18 @@ int launch_pdl(void (*kernel)(Args...), dim3 grid, dim3 block, cudaStream_t st, 
     return TPT_OK;
 }
 
+// One sweep of the `nf` fields of B, YPT quads a thread.
+template <int YPT, int BZ, int THREADS>
+int launch_sweep(const Batch &B, uint32_t nf, uint32_t s, cudaStream_t st) {
+    return launch_pdl(k_b_sweep<YPT, BZ, THREADS>, dim3(QUADS / YPT / THREADS, B.n, nf), dim3(THREADS), st, B, s);
+}
+
 }  // namespace
 
 int launch_batch(Batch &b, cudaStream_t st) {
     if (b.n == 0 || (b.fields & 3u) == 0u) return TPT_OK;
     const uint32_t nf = (b.fields & 1u) + ((b.fields >> 1) & 1u);
-    int rc = launch_pdl(k_b_prep, dim3(CBLOCKS, b.n, nf), dim3(CBLOCK), st, (const Batch)b);
+    int rc = launch_pdl(k_b_prep, dim3(PBLOCKS, b.n, nf), dim3(PBLOCK), st, (const Batch)b);
     if (rc) return rc;
     const uint32_t air = (b.fields & 1u) ? b.air_iters : 0u, grav = (b.fields & 2u) ? TPT_VOX_GRAV_ITERATIONS : 0u;
     const uint32_t sweeps = air > grav ? air : grav;
@@ -209,10 +289,10 @@ int launch_batch(Batch &b, cudaStream_t st) {
     for (uint32_t s = 0; s < sweeps; ++s) {
         bs.fields = (s < air ? 1u : 0u) | (s < grav ? 2u : 0u);
         const uint32_t n = (bs.fields & 1u) + ((bs.fields >> 1) & 1u);
-        rc = launch_pdl(k_b_sweep, dim3(QBLOCKS, b.n, n), dim3(QBLOCK), st, (const Batch)bs, s);
+        rc = b.n < MANY_WORLDS ? launch_sweep<1, 4, 256>(bs, n, s, st) : launch_sweep<2, 8, 128>(bs, n, s, st);
         if (rc) return rc;
     }
-    return launch_pdl(k_b_finish, dim3(CBLOCKS, b.n, nf), dim3(CBLOCK), st, (const Batch)b);
+    return launch_pdl(k_b_finish, dim3(PBLOCKS, b.n, nf), dim3(PBLOCK), st, (const Batch)b);
 }
 
 }  // namespace vox
