@@ -15,12 +15,18 @@
 //   finish  grid-wide, once: the air advection, the gravity force and the
 //           mass clear.
 //
-// Every launch is a programmatic dependent launch: it lets the next launch
-// start as soon as all its blocks are running (griddepcontrol.launch_dependents)
-// and waits for the previous grid's completion and memory
-// (griddepcontrol.wait) before touching global memory, so a sweep's launch
-// latency overlaps the previous sweep's tail. The fields of a world stay in
-// L2 (1 MiB each) across the sweeps.
+// Every launch is a programmatic dependent launch: it waits for the previous
+// grid's completion and memory (griddepcontrol.wait), then lets the next one
+// start (griddepcontrol.launch_dependents), so that a launch's latency
+// overlaps the grid before it. As the release comes after the wait, a grid
+// that runs knows every grid before its predecessor complete, and may load
+// what those wrote, and its predecessor does not write, before its own wait:
+// a sweep after the first its source and pins, the finishing pass the
+// temperature and solid fields (all past L1, which an earlier step may have
+// filled). That took the step of one world from 65.0 to 57.4 us, of eight
+// from 248 to 239; releasing before the wait, without early loads, 65.0; after
+// it, without them, 62.8. The fields of a world stay in L2 (1 MiB each) across
+// the sweeps.
 #include "field3d.hpp"
 #include "field3d_cell.cuh"
 
@@ -49,7 +55,7 @@ __device__ __forceinline__ int field_of(uint32_t fields, int z) {
 // by DRAM when the worlds are many. A thread takes a quad, so a field's
 // neighbours are five float4 loads and two shuffles instead of 28 word loads:
 // the whole step with the layouts below, 1 / 2 / 4 / 8 worlds, went from 65 /
-// 104 / 165 / 284 us to 65 / 96 / 149 / 248.
+// 104 / 165 / 284 us to 65 / 96 / 149 / 248 (without the early loads).
 
 // A quad's neighbourhood of one field: its cells, the quads beside it in z and
 // y (zero outside the world) and the cells before and after it in x, from the
@@ -64,20 +70,26 @@ __device__ __forceinline__ void quad_x(Quad &q) {
     q.l = __shfl_up_sync(0xFFFFFFFFu, q.c.w, 1, 16);
     q.r = __shfl_down_sync(0xFFFFFFFFu, q.c.x, 1, 16);
 }
+// L2: past L1.
+template <bool L2 = false>
+__device__ __forceinline__ float4 load4(const float *a) {
+    return L2 ? __ldcg(reinterpret_cast<const float4 *>(a)) : ld4(a);
+}
+template <bool L2 = false>
 __device__ __forceinline__ Quad load_quad(const float *a, int i0, int y, int z) {
     Quad q;
-    q.c = ld4(a + i0);
-    q.zm = z > 0 ? ld4(a + i0 - SZ) : zero4();
-    q.zp = z + 1 < N ? ld4(a + i0 + SZ) : zero4();
-    q.ym = y > 0 ? ld4(a + i0 - SY) : zero4();
-    q.yp = y + 1 < N ? ld4(a + i0 + SY) : zero4();
+    q.c = load4<L2>(a + i0);
+    q.zm = z > 0 ? load4<L2>(a + i0 - SZ) : zero4();
+    q.zp = z + 1 < N ? load4<L2>(a + i0 + SZ) : zero4();
+    q.ym = y > 0 ? load4<L2>(a + i0 - SY) : zero4();
+    q.yp = y + 1 < N ? load4<L2>(a + i0 + SY) : zero4();
     quad_x(q);
     return q;
 }
 
 __global__ void __launch_bounds__(PBLOCK) k_b_prep(const __grid_constant__ Batch B) {
-    pdl_launch_dependents();
     pdl_wait();
+    pdl_launch_dependents();
     const BWorld &w = B.w[blockIdx.y];
     const int f = field_of(B.fields, blockIdx.z);
     const int q = blockIdx.x * PBLOCK + threadIdx.x;
@@ -124,7 +136,8 @@ __global__ void __launch_bounds__(PBLOCK) k_b_prep(const __grid_constant__ Batch
 // other threads' loads, or on the way into L1 for them. What bounds it is L1
 // and the latency of one dependent round to L2, where the fields stay; of the
 // layouts, (YPT, BZ, threads), measured on B200 as whole field steps with 12
-// air sweeps and 30% of the bricks listed, us for 1 / 2 / 4 / 8 worlds:
+// air sweeps and 30% of the bricks listed, before the early loads and the
+// passes below, us for 1 / 2 / 4 / 8 worlds:
 //
 //   (1, 16, 256), a strip of 16 rows  66 / 108 / 177 / 310
 //   (1, 4, 256)                       65 / 104 / 167 / 295   below 4 worlds
@@ -140,8 +153,6 @@ __global__ void __launch_bounds__(PBLOCK) k_b_prep(const __grid_constant__ Batch
 template <int YPT, int BZ, int THREADS>
 __global__ void __launch_bounds__(THREADS) k_b_sweep(const __grid_constant__ Batch B, uint32_t s) {
     constexpr int BY = THREADS / 16 / BZ * YPT;  // planes of a block
-    pdl_launch_dependents();
-    pdl_wait();
     const BWorld &w = B.w[blockIdx.y];
     const int f = field_of(B.fields, blockIdx.z);
     const int x0 = 4 * (threadIdx.x & 15), row = threadIdx.x >> 4;
@@ -160,6 +171,18 @@ __global__ void __launch_bounds__(THREADS) k_b_sweep(const __grid_constant__ Bat
     }
     const float *source = f == 0 ? w.div : w.src;
     float4 c[YPT + 2], zm[YPT], zp[YPT], sr[YPT];
+    uint32_t pn[YPT];
+    auto load_source = [&]() {
+#pragma unroll
+        for (int j = 0; j < YPT; ++j) {
+            sr[j] = __ldcg(reinterpret_cast<const float4 *>(source + i0 + j * SY));
+            pn[j] = f == 0 ? __ldcg(w.pin + ((i0 + j * SY) >> 2)) : 0u;
+        }
+    };
+    if (s > 0) load_source();  // the first sweep's predecessor is the pass that writes it
+    pdl_wait();
+    pdl_launch_dependents();
+    if (s == 0) load_source();
     c[0] = y0 > 0 ? ld4(S + i0 - SY) : zero4();
 #pragma unroll
     for (int j = 0; j < YPT; ++j) c[j + 1] = ld4(S + i0 + j * SY);
@@ -168,7 +191,6 @@ __global__ void __launch_bounds__(THREADS) k_b_sweep(const __grid_constant__ Bat
     for (int j = 0; j < YPT; ++j) {
         zm[j] = z > 0 ? ld4(S + i0 + j * SY - SZ) : zero4();
         zp[j] = z + 1 < N ? ld4(S + i0 + j * SY + SZ) : zero4();
-        sr[j] = ld4(source + i0 + j * SY);
     }
 #pragma unroll
     for (int j = 0; j < YPT; ++j) {
@@ -177,7 +199,7 @@ __global__ void __launch_bounds__(THREADS) k_b_sweep(const __grid_constant__ Bat
         const float r = __shfl_down_sync(0xFFFFFFFFu, c[j + 1].x, 1, 16);
         float4 out;
         if (f == 0) {
-            const uint32_t pins = w.pin[(i0 + j * SY) >> 2];
+            const uint32_t pins = pn[j];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const float xm = k == 0 ? l : f4(c[j + 1], k - 1), xp = k == 3 ? r : f4(c[j + 1], k + 1);
@@ -199,12 +221,12 @@ __global__ void __launch_bounds__(THREADS) k_b_sweep(const __grid_constant__ Bat
 }
 
 __global__ void __launch_bounds__(PBLOCK) k_b_finish(const __grid_constant__ Batch B) {
-    pdl_launch_dependents();
-    pdl_wait();
     const BWorld &w = B.w[blockIdx.y];
     const int f = field_of(B.fields, blockIdx.z);
     const int i0 = 4 * (int)(blockIdx.x * PBLOCK + threadIdx.x), x0 = i0 & 63, z = (i0 >> 6) & 63, y = i0 >> 12;
     if (f == 1) {
+        pdl_wait();
+        pdl_launch_dependents();
         // gravity_force_kernel (gravity.rs:199-224) on the last sweep, then
         // gravity_clear_kernel (gravity.rs:112-118) when asked
         const Quad u = load_quad(w.pot, i0, y, z);
@@ -225,8 +247,8 @@ __global__ void __launch_bounds__(PBLOCK) k_b_finish(const __grid_constant__ Bat
         return;
     }
     // air_advect_kernel (air_kernel.rs:414-536) from the snapshot
-    const float4 solid = ld4(w.solid + i0);
-    const Quad t = load_quad(w.temp, i0, y, z);
+    const float4 solid = __ldcg(reinterpret_cast<const float4 *>(w.solid + i0));
+    const Quad t = load_quad<true>(w.temp, i0, y, z);
     float4 buoy;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -234,6 +256,8 @@ __global__ void __launch_bounds__(PBLOCK) k_b_finish(const __grid_constant__ Bat
                                     x0 + k, y, z);
         f4set(buoy, k, (lt - kAmbient) * kBuoyancy);
     }
+    pdl_wait();
+    pdl_launch_dependents();
     const Quad p = load_quad((B.air_iters & 1u) ? w.p_tmp : w.p, i0, y, z);  // the last sweep's buffer
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
