@@ -48,6 +48,18 @@ namespace {
 
 constexpr uint32_t kMaxAirIterations = 65536;
 
+// Zeroes device memory before it returns, on a stream of its own: the first
+// call on the plan may come on any stream, and others may be capturing.
+cudaError_t zero_now(void *p, size_t bytes) {
+    cudaStream_t st = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e != cudaSuccess) return e;
+    e = cudaMemsetAsync(p, 0, bytes, st);
+    const cudaError_t done = cudaStreamSynchronize(st);
+    cudaStreamDestroy(st);
+    return e != cudaSuccess ? e : done;
+}
+
 bool aligned16(const void *p) { return ((uintptr_t)p & 15u) == 0u; }
 
 // Checks the pointers a call reads or writes: non-NULL and 16-byte aligned
@@ -150,9 +162,10 @@ int tpt_vox_plan_create(int form, tpt_vox_plan **out) {
     cudaError_t e = cudaMalloc(&p->scratch, bytes);
     const size_t table = TPT_VOX_BRICKS * sizeof(uint32_t);
     if (e == cudaSuccess) e = cudaMalloc(&p->brick_mult, table);
-    if (e == cudaSuccess) e = cudaMemset(p->brick_mult, 0, table);
+    if (e == cudaSuccess) e = zero_now(p->brick_mult, table);
     if (e != cudaSuccess) {
         cudaFree(p->scratch);
+        cudaFree(p->brick_mult);
         delete p;
         TPT_FAIL(e == cudaErrorMemoryAllocation ? TPT_ERR_OUT_OF_MEMORY : TPT_ERR_CUDA,
                  "tpt_vox_plan_create: scratch allocation failed: %s", cudaGetErrorString(e));
