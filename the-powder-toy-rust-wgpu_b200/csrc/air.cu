@@ -8,38 +8,79 @@
 namespace tpt {
 namespace air {
 
+// What bounds a tick of one grid of up to a few hundred thousand cells is its
+// serial chain: three launches, and in each the barriers, the ring cells that
+// a thread takes one after the other, and the walk of the advection.
+//
+// The kernels are programmatic dependent launches: each waits for the one
+// before it to complete before it touches memory, and starts as soon as that
+// one's blocks exit, or, the settle pass, have staged their tile. (Releasing
+// pass B from pass A's staging as well puts its blocks unevenly beside those
+// still running: 401x225 16.7 -> 20.0 us.)
+//
+// A block has more threads than its tile has cells: pass A's +2 ring has 432
+// cells and pass B's +1 ring 340, and each ring is one turn instead of two.
+// Measured on B200, us per tick in a graph, before (256 threads, ordinary
+// launches) and now: 16x16 10.9 and 8.1, 64x48 16.3 and 11.4, 153x96 18.5 and
+// 13.4, 300x200 18.6 and 14.3, 401x225 20.2 and 16.7, 512x512 32.0 and 27.7,
+// 590x590 39.8 and 35.4. As strips, the launches alone: 1024x1024 84.8 and 76.9,
+// 2048x2048 249.5 and 240.3 in calls back to back.
+constexpr int NT_A = 448, NT_B = 384;
+static_assert(NT_A >= (TX + 4) * (TY + 4) && NT_B >= (TX + 2) * (TY + 2), "a ring is one turn");
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... Args>
+static int launch_pdl(void (*kernel)(Args...), dim3 grid, unsigned block, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    TPT_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+    TPT_LAUNCHED();
+    return TPT_OK;
+}
+
 // Pass A of one tile, staged by plain loads (the caller's grids may have any
 // row length, so no TMA).
-__global__ void __launch_bounds__(NT) k_pressure_velocity(const AirInst I) {
+__global__ void __launch_bounds__(NT_A) k_pressure_velocity(const AirInst I) {
     __shared__ LayoutA1 S;
+    pdl_wait();
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
-    stage_flag<3>(S.b, I.bair, 0xFFFFFFFFu, I, x0, y0);
-    stage<float, 2>(S.vx, I.vx, I, x0, y0);
-    stage<float, 2>(S.vy, I.vy, I, x0, y0);
-    stage<float, 1>(S.pv, I.pv, I, x0, y0);
+    stage_flag<3, NT_A>(S.b, I.bair, 0xFFFFFFFFu, I, x0, y0);
+    stage<float, 2, NT_A>(S.vx, I.vx, I, x0, y0);
+    stage<float, 2, NT_A>(S.vy, I.vy, I, x0, y0);
+    stage<float, 1, NT_A>(S.pv, I.pv, I, x0, y0);
     __syncthreads();
-    pass_a(I, x0, y0, S);
+    pass_a<NT_A>(I, x0, y0, S);
 }
 
 // Pass B of one tile.
-__global__ void __launch_bounds__(NT) k_advect_heat(const AirInst I) {
+__global__ void __launch_bounds__(NT_B) k_advect_heat(const AirInst I) {
     __shared__ LayoutB1 S;
+    pdl_wait();
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
     if (I.air_mode != 4u) {
-        stage_flag<3>(S.b, I.bair, 0xFFFFFFFFu, I, x0, y0);
-        stage<float, 3>(S.ovx, I.ovx, I, x0, y0);
-        stage<float, 3>(S.ovy, I.ovy, I, x0, y0);
-        stage<float, 2>(S.opv, I.opv, I, x0, y0);
+        stage_flag<3, NT_B>(S.b, I.bair, 0xFFFFFFFFu, I, x0, y0);
+        stage<float, 3, NT_B>(S.ovx, I.ovx, I, x0, y0);
+        stage<float, 3, NT_B>(S.ovy, I.ovy, I, x0, y0);
+        stage<float, 2, NT_B>(S.opv, I.opv, I, x0, y0);
     } else {
-        stage<float, 1>(S.nvx, I.vx, I, x0, y0);
-        stage<float, 1>(S.nvy, I.vy, I, x0, y0);
+        stage<float, 1, NT_B>(S.nvx, I.vx, I, x0, y0);
+        stage<float, 1, NT_B>(S.nvy, I.vy, I, x0, y0);
     }
     if (I.aheat) {
-        stage_flag<1>(S.bh, I.bairh, 0x8u, I, x0, y0);
-        stage<float, 1>(S.hv, I.hv, I, x0, y0);
+        stage_flag<1, NT_B>(S.bh, I.bairh, 0x8u, I, x0, y0);
+        stage<float, 1, NT_B>(S.hv, I.hv, I, x0, y0);
     }
     __syncthreads();
-    pass_b(I, x0, y0, S);
+    pdl_release();
+    pass_b<NT_B>(I, x0, y0, S);
 }
 
 // The same tick as warp strips (air_strip.cuh): warp w takes strip w % strips of
@@ -62,15 +103,18 @@ __device__ __forceinline__ bool strip_of(const OneGrid &G, int width, int &x0, i
     return y0 < (int)G.I.Y;
 }
 __global__ void __launch_bounds__(STRIP_WARPS * 32, 8) k_strip_velocity(const __grid_constant__ OneGrid G) {
+    pdl_wait();
     int x0, y0, y1;
     if (strip_of(G, strip_width(PASS_VELOCITY), x0, y0, y1)) strip_a(G.P, G.I, 0u, x0, y0, y1);
 }
 __global__ void __launch_bounds__(STRIP_WARPS * 32, 6) k_strip_advect(const __grid_constant__ OneGrid G) {
+    pdl_wait();
     int x0, y0, y1;
     // into vx / vy, free since the velocity pass read them
     if (strip_of(G, strip_width(PASS_ADVECT), x0, y0, y1)) strip_advect(G.P, G.I, G.P.vx, G.P.vy, 0u, x0, y0, y1);
 }
 __global__ void __launch_bounds__(STRIP_WARPS * 32, 6) k_strip_heat(const __grid_constant__ OneGrid G) {
+    pdl_wait();
     int x0, y0, y1;
     // from vx / vy into ovx / ovy; the settle pass copies them back
     if (strip_of(G, strip_width(PASS_HEAT), x0, y0, y1))
@@ -82,6 +126,7 @@ __global__ void __launch_bounds__(STRIP_WARPS * 32, 6) k_strip_heat(const __grid
 // HotAir pass (settle.rs:118-161). The grid is dense here (pitch == X).
 __global__ void k_settle(const AirInst I, const uint32_t *__restrict__ pmap, const uint32_t *__restrict__ props,
                          uint32_t nprops, uint32_t xres, uint32_t yres, bool copy_v) {
+    pdl_wait();
     const size_t n = (size_t)I.X * I.Y;
     for (size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x; g < n; g += (size_t)gridDim.x * blockDim.x) {
         if (I.aheat) {
@@ -144,9 +189,7 @@ int launch_single(const AirInst &I, const uint32_t *pmap, const uint32_t *props,
             const size_t fit = (size_t)G.strips * I.Y / (3 * 148 * 24);
             G.rows = (uint32_t)std::min<size_t>(32, std::max<size_t>(4, fit));
             const uint32_t warps = G.strips * ((I.Y + G.rows - 1) / G.rows);
-            kernel<<<(warps + STRIP_WARPS - 1) / STRIP_WARPS, STRIP_WARPS * 32, 0, st>>>(G);
-            TPT_LAUNCHED();
-            return TPT_OK;
+            return launch_pdl(kernel, dim3((warps + STRIP_WARPS - 1) / STRIP_WARPS), STRIP_WARPS * 32, st, (const OneGrid)G);
         };
         int rc = TPT_OK;
         if (I.air_mode != 4u) {
@@ -157,19 +200,14 @@ int launch_single(const AirInst &I, const uint32_t *pmap, const uint32_t *props,
         if (rc) return rc;
     } else {
         dim3 grid((I.X + TX - 1) / TX, (I.Y + TY - 1) / TY);
-        if (I.air_mode != 4u) {
-            k_pressure_velocity<<<grid, NT, 0, st>>>(I);
-            TPT_LAUNCHED();
-        }
-        if (I.air_mode != 4u || I.aheat) {
-            k_advect_heat<<<grid, NT, 0, st>>>(I);
-            TPT_LAUNCHED();
-        }
+        int rc = TPT_OK;
+        if (I.air_mode != 4u) rc = launch_pdl(k_pressure_velocity, grid, NT_A, st, (const AirInst)I);
+        if (rc == TPT_OK && (I.air_mode != 4u || I.aheat)) rc = launch_pdl(k_advect_heat, grid, NT_B, st, (const AirInst)I);
+        if (rc) return rc;
     }
     unsigned blocks = (unsigned)std::min<size_t>((n + 255) / 256, 148 * 16);
-    k_settle<<<blocks, 256, 0, st>>>(I, pmap, props, nprops, xres, yres, I.aheat && (strips || I.air_mode == 4u));
-    TPT_LAUNCHED();
-    return TPT_OK;
+    return launch_pdl(k_settle, dim3(blocks), 256, st, (const AirInst)I, pmap, props, nprops, xres, yres,
+                      I.aheat && (strips || I.air_mode == 4u));
 }
 
 // ---- air step with library-owned scratch (no allocation) ------------------

@@ -193,18 +193,18 @@ struct LayoutB2 {
 };
 
 // ---- staging by loads (single-grid path) -------------------------------------
-template <typename T, int H>
+template <typename T, int H, int THREADS = NT>
 __device__ __forceinline__ void stage(T *s, const T *g, const AirInst &I, int x0, int y0) {
-    for (int i = threadIdx.x; i < Reg<H>::N; i += NT) {
+    for (int i = threadIdx.x; i < Reg<H>::N; i += THREADS) {
         int ly = i / Reg<H>::W, lx = i - ly * Reg<H>::W;
         int gx = x0 - H + lx, gy = y0 - H + ly;
         s[i] = in_grid(gx, gy, I) ? __ldg(g + (size_t)gy * I.pitch + gx) : T(0);
     }
 }
-template <int H>
+template <int H, int THREADS = NT>
 __device__ __forceinline__ void stage_flag(uint8_t *s, const uint32_t *g, uint32_t bitmask, const AirInst &I, int x0,
                                            int y0) {
-    for (int i = threadIdx.x; i < Reg<H>::N; i += NT) {
+    for (int i = threadIdx.x; i < Reg<H>::N; i += THREADS) {
         int ly = i / Reg<H>::W, lx = i - ly * Reg<H>::W;
         int gx = x0 - H + lx, gy = y0 - H + ly;
         s[i] = in_grid(gx, gy, I) ? ((__ldg(g + (size_t)gy * I.pitch + gx) & bitmask) != 0u) : 0;
@@ -213,10 +213,10 @@ __device__ __forceinline__ void stage_flag(uint8_t *s, const uint32_t *g, uint32
 
 // Calls f(gx, gy) for every in-grid cell of the tile's +R ring (R = 0: the
 // tile), spread over the block's threads.
-template <int R, typename F>
+template <int R, int THREADS = NT, typename F>
 __device__ __forceinline__ void for_ring(const AirInst &I, int x0, int y0, F &&f) {
     constexpr int W = TX + 2 * R, N = W * (TY + 2 * R);
-    for (int i = threadIdx.x; i < N; i += NT) {
+    for (int i = threadIdx.x; i < N; i += THREADS) {
         int ly = i / W, lx = i - ly * W;
         int gx = x0 - R + lx, gy = y0 - R + ly;
         if (in_grid(gx, gy, I)) f(gx, gy);
@@ -247,13 +247,14 @@ __device__ __forceinline__ bool wall_cleared_vy(const L &S, uint32_t x, uint32_t
 }
 
 // The compute of pass A once the tile is staged in S. Writes opv, ovx, ovy.
-template <class L> __device__ __forceinline__ void pass_a(const AirInst &I, int x0, int y0, L &S) {
+template <int THREADS = NT, class L>
+__device__ __forceinline__ void pass_a(const AirInst &I, int x0, int y0, L &S) {
     const uint32_t X = I.X, Y = I.Y;
     // effective_vx/vy (pressure.rs:119-157) on the +2 ring, in place; this
     // is also the velocity pass's pre-gradient value (pressure.rs:265-276).
     // Every thread reads only its own cells' velocities, so no barrier is
     // needed between the reads and the in-place writes.
-    for_ring<2>(I, x0, y0, [&](int gx, int gy) {
+    for_ring<2, THREADS>(I, x0, y0, [&](int gx, int gy) {
         float vx = S.VX(gx, gy, x0, y0), vy = S.VY(gx, gy, x0, y0);
         if (in_border(gx, gy, X, Y)) {
             vx = I.evx + (vx - I.evx) * 0.9f;
@@ -266,7 +267,7 @@ template <class L> __device__ __forceinline__ void pass_a(const AirInst &I, int 
     });
     __syncthreads();
     // air_pressure_kernel (pressure.rs:186-237) on the +1 ring.
-    for_ring<1>(I, x0, y0, [&](int gx, int gy) {
+    for_ring<1, THREADS>(I, x0, y0, [&](int gx, int gy) {
         float cur = S.PV(gx, gy, x0, y0);
         if (in_border(gx, gy, X, Y)) cur = I.ep + (cur - I.ep) * 0.8f;
         float next = cur;
@@ -280,7 +281,7 @@ template <class L> __device__ __forceinline__ void pass_a(const AirInst &I, int 
     __syncthreads();
     // air_velocity_kernel (pressure.rs:260-298) on the tile.
     const int gx = x0 + (int)(threadIdx.x % TX), gy = y0 + (int)(threadIdx.x / TX);
-    if (in_grid(gx, gy, I)) {
+    if ((THREADS == NT || threadIdx.x < NT) && in_grid(gx, gy, I)) {
         float nx = S.VX(gx, gy, x0, y0), ny = S.VY(gx, gy, x0, y0);
         if (interior(gx, gy, X, Y)) {
             float dx = S.OPV(gx - 1, gy, x0, y0) - S.OPV(gx + 1, gy, x0, y0);
@@ -629,18 +630,19 @@ __device__ __forceinline__ float heat_cell(const AirInst &I, L &S, int x, int y,
 // NVY already hold the stored vx/vy (staged by the caller); the convected
 // velocity then goes to ovx/ovy (unused scratch in that mode) so that no CTA
 // writes a vx/vy cell another CTA may still stage.
-template <class L> __device__ __forceinline__ void pass_b(const AirInst &I, int x0, int y0, L &S) {
+template <int THREADS = NT, class L>
+__device__ __forceinline__ void pass_b(const AirInst &I, int x0, int y0, L &S) {
     const uint32_t X = I.X, Y = I.Y;
     const bool update = I.air_mode != 4u;
     if (update) {
         if (I.vcoef > 0.0f) {
-            for_ring<2>(I, x0, y0,
+            for_ring<2, THREADS>(I, x0, y0,
                         [&](int gx, int gy) { S.VORT(gx, gy, x0, y0) = vorticity_bmap(S, gx, gy, X, Y, x0, y0); });
             __syncthreads();
         }
         // the +1 ring outside the tile is needed only as heat-smoothing taps
         if (I.aheat) {
-            for_ring<1>(I, x0, y0, [&](int gx, int gy) {
+            for_ring<1, THREADS>(I, x0, y0, [&](int gx, int gy) {
                 float a, b, c;
                 smooth_advect_cell(I, S, gx, gy, x0, y0, a, b, c);
                 S.NVX(gx, gy, x0, y0) = a;
@@ -648,7 +650,7 @@ template <class L> __device__ __forceinline__ void pass_b(const AirInst &I, int 
                 S.NPV(gx, gy, x0, y0) = c;
             });
         } else {
-            for_ring<0>(I, x0, y0, [&](int gx, int gy) {
+            for_ring<0, THREADS>(I, x0, y0, [&](int gx, int gy) {
                 float a, b, c;
                 smooth_advect_cell(I, S, gx, gy, x0, y0, a, b, c);
                 S.NVX(gx, gy, x0, y0) = a;
@@ -659,7 +661,7 @@ template <class L> __device__ __forceinline__ void pass_b(const AirInst &I, int 
         __syncthreads();
     }
     const int gx = x0 + (int)(threadIdx.x % TX), gy = y0 + (int)(threadIdx.x / TX);
-    if (!in_grid(gx, gy, I)) return;
+    if ((THREADS != NT && threadIdx.x >= NT) || !in_grid(gx, gy, I)) return;
     const size_t g = (size_t)gy * I.pitch + gx;
     float vx = S.NVX(gx, gy, x0, y0), vy = S.NVY(gx, gy, x0, y0);
     if (I.aheat) {
