@@ -20,7 +20,9 @@ from __future__ import annotations
 
 import ctypes
 import dataclasses
+import operator
 import os
+import struct
 import subprocess
 
 import numpy as np
@@ -292,6 +294,14 @@ def _ptr(t) -> ctypes.c_void_p | None:
     return ctypes.c_void_p(t.data_ptr())
 
 
+def _addr(t) -> int:
+    """The address of a tensor or array (0 for None), for a structure that
+    holds no reference to it."""
+    if t is None:
+        return 0
+    return t.ctypes.data if isinstance(t, np.ndarray) else t.data_ptr()
+
+
 def _stream(stream) -> ctypes.c_void_p | None:
     if stream is None:
         import torch
@@ -415,21 +425,29 @@ class SimBuffers:
         return out
 
 
+_air_grids = operator.attrgetter(
+    "air_pv", "air_vx", "air_vy", "air_hv", "air_opv", "air_ovx", "air_ovy", "air_ohv", "block_air", "block_airh",
+    "wall_bmap", "wall_emap", "elem_block_air", "elem_block_airh", "fan_vx", "fan_vy")
+
+
+_air_pack = struct.Struct("@18P3I4x").pack  # AirBufs
+assert len(_air_pack(*[0] * 21)) == ctypes.sizeof(AirBufs)
+
+
 def air_bufs(b: SimBuffers) -> AirBufs:
-    x = AirBufs()
-    for name, attr in (("pv", "air_pv"), ("vx", "air_vx"), ("vy", "air_vy"), ("hv", "air_hv"), ("opv", "air_opv"),
-                       ("ovx", "air_ovx"), ("ovy", "air_ovy"), ("ohv", "air_ohv"), ("block_air", "block_air"),
-                       ("block_airh", "block_airh"), ("wall_bmap", "wall_bmap"), ("wall_emap", "wall_emap"),
-                       ("elem_block_air", "elem_block_air"), ("elem_block_airh", "elem_block_airh"),
-                       ("fan_vx", "fan_vx"), ("fan_vy", "fan_vy")):
-        setattr(x, name, _ptr(getattr(b, attr)))
+    # A call on a small canvas is bound by its host work: one pass over the
+    # grids in AirBufs' order and one packed structure (2.6 us) instead of a
+    # ctypes pointer and a field assignment each (6.4 us).
+    pmap = props = xres = yres = n_elements = 0
     if b.pmap is not None:
-        x.pmap = _ptr(b.pmap)
-        x.elem_props = _ptr(b.elem_props)
-        x.xres = b.config.xres
-        x.yres = b.config.yres
-        x.n_elements = b.elem_props.numel() // 32
-    return x
+        pmap, props = _addr(b.pmap), _addr(b.elem_props)
+        xres, yres, n_elements = b.config.xres, b.config.yres, b.elem_props.numel() // 32
+    grids = _air_grids(b)
+    try:
+        ptrs = [t.data_ptr() for t in grids]
+    except AttributeError:  # an absent optional grid
+        ptrs = [_addr(t) for t in grids]
+    return AirBufs.from_buffer_copy(_air_pack(*ptrs, pmap, props, xres, yres, n_elements))
 
 
 def step_air_gpu(bufs: SimBuffers, stream=None) -> None:
