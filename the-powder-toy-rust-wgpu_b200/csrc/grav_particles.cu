@@ -43,9 +43,31 @@ __device__ __forceinline__ float clampf(float v, float lo, float hi) {
     return out;
 }
 
+// The kernels of a gravity tick are programmatic dependent launches: each waits
+// for the one before it to complete before it touches memory.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename... Args>
+int launch_pdl(void (*kernel)(Args...), uint32_t blocks, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    TPT_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+    TPT_LAUNCHED();
+    return TPT_OK;
+}
+
 // seed_gravity_tool_mass_kernel (:241-262) then seed_gravity_mass_kernel
 // (:217-229, whose tool word the first step has already consumed).
 __global__ void k_seed(GravGrids G, uint32_t cells) {
+    pdl_release();
+    pdl_wait();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= cells) return;
     if (G.tool) {
@@ -61,6 +83,8 @@ __global__ void k_seed(GravGrids G, uint32_t cells) {
 // apply_gravity_kernel (:434-516) and build_gravity_mass_kernel (:275-376),
 // one thread per slot.
 __global__ void k_particles(GravGrids G, Parts P) {
+    pdl_release();
+    pdl_wait();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
     const uint32_t ty = P.ty[i];
@@ -144,6 +168,8 @@ __global__ void k_particles(GravGrids G, Parts P) {
 
 // apply_grav_mass_override_kernel (:379-391) then copy_gravity_mass_kernel (:518-527).
 __global__ void k_finish(GravGrids G, uint32_t cells) {
+    pdl_release();
+    pdl_wait();
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= cells) return;
     int32_t m = G.mass[c];
@@ -156,20 +182,16 @@ __global__ void k_finish(GravGrids G, uint32_t cells) {
 
 int launch_seed(const GravGrids &G, cudaStream_t st) {
     const uint32_t cells = G.xcells * G.ycells;
-    k_seed<<<(cells + 255) / 256, 256, 0, st>>>(G, cells);
-    TPT_LAUNCHED();
-    return TPT_OK;
+    return launch_pdl(k_seed, (cells + 255) / 256, st, G, cells);
 }
 
 int launch_particles_and_finish(const GravGrids &G, const Parts &P, cudaStream_t st) {
     if (P.n) {
-        k_particles<<<(P.n + 255) / 256, 256, 0, st>>>(G, P);
-        TPT_LAUNCHED();
+        const int rc = launch_pdl(k_particles, (P.n + 255) / 256, st, G, P);
+        if (rc) return rc;
     }
     const uint32_t cells = G.xcells * G.ycells;
-    k_finish<<<(cells + 255) / 256, 256, 0, st>>>(G, cells);
-    TPT_LAUNCHED();
-    return TPT_OK;
+    return launch_pdl(k_finish, (cells + 255) / 256, st, G, cells);
 }
 
 }  // namespace gp
