@@ -62,8 +62,11 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 template <int R, bool INV> __device__ __noinline__ void row_step2(const Axis &A, uint32_t cnt) {
     step2<R, INV>(fft_smem, A, RowSeq{}, cnt);
 }
-template <int R, bool INV> __device__ __noinline__ void col_step2(float2 *S, const Axis &A, uint32_t lc) {
-    step2<R, INV>(S, A, ColSeq{lc}, 1u << lc);
+template <int R> __device__ __noinline__ void col_step2(const Axis &A, uint32_t lc) {
+    step2<R, false>(fft_smem, A, ColSeq{lc}, 1u << lc);
+}
+template <int R> __device__ __noinline__ void pair_step2(const Axis &A, uint32_t lc) {
+    step2<R, true>(fft_smem, A, PairSeq{lc, A.sz << lc}, 2u << lc);
 }
 
 // Row pairs y = 2 p, 2 p + 1 (p0 <= p < p0 + cnt) as z = m[2p] + i m[2p+1].
@@ -195,13 +198,15 @@ template <int R> __device__ __noinline__ void cols_products(const Job &J, uint32
         }
     }
 }
-template <int R> __device__ __noinline__ void cols_store(const Job &J, uint32_t h0, uint32_t lc, float2 *S, float2 *out) {
-    const uint32_t Y = J.Y, nhp = J.nhp, left = J.nh - h0, m = J.ay.m;
-    const size_t stride = (size_t)m * nhp;
-    out += h0;
-    unstep1<R>(S, J.ay, ColSeq{lc}, 1u << lc, [&](uint32_t c, uint32_t j, const float2(&v)[R]) {
-        float2 *p = out + (size_t)j * nhp + c;
-        const uint32_t rows = c < left ? Y : 0u;
+template <int R> __device__ __noinline__ void cols_store(const Job &J, uint32_t h0, uint32_t lc) {
+    const Axis &A = J.ay;
+    const uint32_t Y = J.Y, nhp = J.nhp, left = J.nh - h0, m = A.m;
+    const size_t stride = (size_t)m * nhp, second = (size_t)Y * nhp;
+    float2 *out = J.spec + h0;
+    unstep1<R>(fft_smem, A, PairSeq{lc, A.sz << lc}, 2u << lc, [&](uint32_t c, uint32_t j, const float2(&v)[R]) {
+        const uint32_t f = c >> lc, col = c - (f << lc);
+        float2 *p = out + (f ? second : 0) + (size_t)j * nhp + col;
+        const uint32_t rows = col < left ? Y : 0u;
 #pragma unroll
         for (int a = 0; a < R; ++a)
             if (j + m * a < rows) p[a * stride] = v[a];
@@ -221,22 +226,16 @@ __global__ void __launch_bounds__(NT_LARGE, MIN_BLOCKS) k_columns(const Job *job
     with_radix(A.r1, [&](auto R) { cols_load<decltype(R)::value>(J, h0, lc); });
     __syncthreads();
     if (A.r2 > 1) {
-        with_radix(A.r2, [&](auto R) { col_step2<decltype(R)::value, false>(fft_smem, A, lc); });
+        with_radix(A.r2, [&](auto R) { col_step2<decltype(R)::value>(A, lc); });
         __syncthreads();
     }
     with_radix(A.r3, [&](auto R) { cols_products<decltype(R)::value>(J, h0, lc, S2); });
     __syncthreads();
     if (A.r2 > 1) {
-#pragma unroll 1
-        for (int f = 0; f < 2; ++f)
-            with_radix(A.r2, [&](auto R) { col_step2<decltype(R)::value, true>(f ? fft_smem : S2, A, lc); });
+        with_radix(A.r2, [&](auto R) { pair_step2<decltype(R)::value>(A, lc); });
         __syncthreads();
     }
-#pragma unroll 1
-    for (int f = 0; f < 2; ++f)
-        with_radix(A.r1, [&](auto R) {
-            cols_store<decltype(R)::value>(J, h0, lc, f ? fft_smem : S2, J.spec + (f ? (size_t)J.Y * J.nhp : 0));
-        });
+    with_radix(A.r1, [&](auto R) { cols_store<decltype(R)::value>(J, h0, lc); });
 }
 
 template <int R> __device__ __noinline__ void rows_first(const Job &J, uint32_t y0, uint32_t cnt) {
@@ -383,7 +382,13 @@ __global__ void spectrum_cols_f64(const double2 *rows, uint32_t n1, uint32_t n2,
 // convolution, 2 cells - 1, as a product of two radices or else of three.
 // Neighbouring lengths lie within 1.25 of each other (1.07 on average above
 // 256), where padding to a power of two costs up to 2 in each direction.
-static bool axis_for(uint32_t cells, Axis *out) {
+//
+// Of the factorings of that length a batch takes two radices before three:
+// fewer steps. One grid is a serial chain instead, with fewer work items than
+// threads, and takes the smallest radices. Measured on B200, us per solve of
+// one grid, two radices and smallest: 153x96 19.2 and 14.8, 300x64 17.4 and
+// 14.2, 400x225 (no factoring in two) 19.5; 256 grids 0.402 and 0.439 ms.
+static bool axis_for(uint32_t cells, bool one_grid, Axis *out) {
     const uint32_t need = std::max<uint32_t>(2 * cells - 1, 32u);
     Axis best{};
     for (uint32_t r1 : kRadices)
@@ -392,10 +397,12 @@ static bool axis_for(uint32_t cells, Axis *out) {
             for (uint32_t r3 : kRadices) {
                 const uint32_t n = r1 * r2 * r3;
                 if (r3 > r1 || n < need || n % 2) continue;
-                // ties: two radices before three, then the smallest sum
-                const bool better = best.n == 0 || n < best.n ||
-                                    (n == best.n && ((r2 == 1) != (best.r2 == 1) ? r2 == 1
-                                                                                 : r1 + r2 + r3 < best.r1 + best.r2 + best.r3));
+                bool better = best.n == 0 || n < best.n;
+                if (n == best.n) {  // r1 is the largest
+                    if (one_grid && r1 != best.r1) better = r1 < best.r1;
+                    else if (!one_grid && (r2 == 1) != (best.r2 == 1)) better = r2 == 1;
+                    else better = r1 + r2 + r3 < best.r1 + best.r2 + best.r3;
+                }
                 if (better) {
                     best.n = n;
                     best.r1 = r1;
@@ -509,7 +516,7 @@ int FftSet::create(const std::vector<JobShape> &shapes) {
     };
     for (size_t j = 0; j < nj; ++j) {
         Job &J = jobs_host[j];
-        if (!axis_for(shapes[j].X, &J.ax) || !axis_for(shapes[j].Y, &J.ay))
+        if (!axis_for(shapes[j].X, nj == 1, &J.ax) || !axis_for(shapes[j].Y, nj == 1, &J.ay))
             TPT_FAIL(TPT_ERR_INVALID_DIMS, "gravity grid %ux%u exceeds the longest transform", shapes[j].X, shapes[j].Y);
         J.X = J.pitch = shapes[j].X;
         J.Y = shapes[j].Y;

@@ -230,6 +230,21 @@ struct ColSeq {
     }
     __device__ __forceinline__ uint32_t step(uint32_t stride) const { return stride << lc; }
 };
+// The columns of both fields: field 0's lie `off` behind field 1's, and its
+// items come first. Column c of field f is c + (f << lc).
+struct PairSeq {
+    uint32_t lc, off;
+    __device__ __forceinline__ void split(uint32_t it, uint32_t items, uint32_t, uint32_t &c, uint32_t &e) const {
+        const uint32_t half = items << lc, f = it >= half ? 1u : 0u;
+        it -= f ? half : 0u;
+        c = (it & ((1u << lc) - 1u)) | (f << lc);
+        e = it >> lc;
+    }
+    __device__ __forceinline__ float2 *at(float2 *S, const Axis &, uint32_t c, uint32_t pos) const {
+        return S + (pos << lc) + (c & ((1u << lc) - 1u)) + (c >> lc ? 0u : off);
+    }
+    __device__ __forceinline__ uint32_t step(uint32_t stride) const { return stride << lc; }
+};
 struct RowSeq {
     __device__ __forceinline__ void split(uint32_t it, uint32_t items, uint32_t magic, uint32_t &c, uint32_t &e) const {
         c = fast_div(it, magic);
