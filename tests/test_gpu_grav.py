@@ -133,3 +133,10 @@ def test_fp32_plan_lengths(cuda, tf, oracle, X, Y):
     scale = max(np.abs(dx).max(), np.abs(dy).max(), 1e-30)
     assert np.abs(gx - dx).max() <= TOL * scale and np.abs(gy - dy).max() <= TOL * scale
     assert np.all(gx[mask == 0] == 0) and np.all(gy[mask == 0] == 0)
+
+
+@pytest.mark.parametrize("n", [16, 48, 67, 200, 512])
+def test_fp32_square_plans(cuda, tf, oracle, n):
+    """Both axes of one length, each with a factoring of its own (and, at 67,
+    of three radices); the bar is the solve's."""
+    test_fp32_plan_lengths(cuda, tf, oracle, n, n)

@@ -388,7 +388,13 @@ __global__ void spectrum_cols_f64(const double2 *rows, uint32_t n1, uint32_t n2,
 // threads, and takes the smallest radices. Measured on B200, us per solve of
 // one grid, two radices and smallest: 153x96 19.2 and 14.8, 300x64 17.4 and
 // 14.2, 400x225 (no factoring in two) 19.5; 256 grids 0.402 and 0.439 ms.
-static bool axis_for(uint32_t cells, bool one_grid, Axis *out) {
+//
+// The largest radix r1 loads a column and r3, which has the most work items,
+// inverts its two products. Rows have it the other way round: their loading
+// step takes two rows of masses and masks per item, and is the longest with a
+// large radix. 16x16 10.1 -> 8.7 us, 600x400 30.2 -> 26.6, 256 grids 0.402 ->
+// 0.392 ms (columns the same way: 1000x900 64.2 -> 69.4 us).
+static bool axis_for(uint32_t cells, bool one_grid, bool rows, Axis *out) {
     const uint32_t need = std::max<uint32_t>(2 * cells - 1, 32u);
     Axis best{};
     for (uint32_t r1 : kRadices)
@@ -412,6 +418,7 @@ static bool axis_for(uint32_t cells, bool one_grid, Axis *out) {
             }
         }
     if (best.n == 0) return false;
+    if (rows) std::swap(best.r1, best.r3);
     auto magic = [](uint32_t d) { return (uint32_t)(((1ull << 32) + d - 1) / d); };
     best.m = best.r2 * best.r3;
     best.q = best.r1 * best.r2;
@@ -425,6 +432,11 @@ static bool axis_for(uint32_t cells, bool one_grid, Axis *out) {
     best.div_13 = magic(best.r1 * best.r3);
     *out = best;
     return true;
+}
+
+// The fewest work items that a transform has in one step.
+static uint32_t fewest_items(const Axis &a) {
+    return std::min(std::min(a.m, a.q), a.r2 > 1 ? a.r1 * a.r3 : a.m);
 }
 
 // The axis's twiddles (layout: Axis::tw), evaluated in double.
@@ -505,18 +517,23 @@ int FftSet::create(const std::vector<JobShape> &shapes) {
         size_t off;
     };
     std::vector<Size> sizes;     // distinct kernels: the spectra depend on the lengths only
-    std::vector<uint32_t> lens;  // distinct lengths, their twiddle tables
-    std::vector<size_t> lens_off;
+    std::vector<Axis> axes;      // distinct factorings, their twiddle tables
+    std::vector<size_t> axes_off;
     std::vector<float2> twh;
+    auto axis_index = [&](const Axis &a) {
+        return (size_t)(std::find_if(axes.begin(), axes.end(), [&](const Axis &b) {
+                            return a.r1 == b.r1 && a.r2 == b.r2 && a.r3 == b.r3;
+                        }) - axes.begin());
+    };
     auto table = [&](const Axis &a) {
-        if (std::find(lens.begin(), lens.end(), a.n) != lens.end()) return;
-        lens.push_back(a.n);
-        lens_off.push_back(twh.size());
+        if (axis_index(a) < axes.size()) return;
+        axes.push_back(a);
+        axes_off.push_back(twh.size());
         fill_twiddles(a, twh);
     };
     for (size_t j = 0; j < nj; ++j) {
         Job &J = jobs_host[j];
-        if (!axis_for(shapes[j].X, nj == 1, &J.ax) || !axis_for(shapes[j].Y, nj == 1, &J.ay))
+        if (!axis_for(shapes[j].X, nj == 1, true, &J.ax) || !axis_for(shapes[j].Y, nj == 1, false, &J.ay))
             TPT_FAIL(TPT_ERR_INVALID_DIMS, "gravity grid %ux%u exceeds the longest transform", shapes[j].X, shapes[j].Y);
         J.X = J.pitch = shapes[j].X;
         J.Y = shapes[j].Y;
@@ -549,7 +566,7 @@ int FftSet::create(const std::vector<JobShape> &shapes) {
         rc = build_spectra(s.n1, s.n2, (s.n1 / 2 + 1 + 7) / 8 * 8, kern + s.off);
         if (rc) return rc;
     }
-    auto tw_of = [&](uint32_t n) { return tw + lens_off[std::find(lens.begin(), lens.end(), n) - lens.begin()]; };
+    auto tw_of = [&](const Axis &a) { return tw + axes_off[axis_index(a)]; };
     // Per block about `per` points of rows and twice that of columns (two to
     // four work items per thread in each step: the job's staging and the code
     // fetched serve all of them), fewer while that leaves SMs idle.
@@ -564,14 +581,18 @@ int FftSet::create(const std::vector<JobShape> &shapes) {
         J.work = work + woff[j];
         J.spec = spec + 2 * woff[j];
         J.kern = kern + koff[j];
-        J.ax.tw = tw_of(J.ax.n);
-        J.ay.tw = tw_of(J.ay.n);
+        J.ax.tw = tw_of(J.ax);
+        J.ay.tw = tw_of(J.ay);
         J.rows_f = J.rows_i = std::max<uint32_t>(1u, per / J.ax.n);
         // columns: at least 4 (32-byte pieces of the rows), 2 when there are
-        // few blocks or their two buffers would leave one block per SM
+        // few blocks or their two buffers would leave one block per SM (two, for
+        // one grid: 1200x701 62.5 -> 52.8 us), and 1 when even those would
+        // (1500x1500 181 -> 157 us)
         J.lc = 2;
         while (J.lc < 5 && (J.ay.n << (J.lc + 1)) <= 2 * per) ++J.lc;
-        while (J.lc > 1 && (points / per < 2 * 148 || ((size_t)J.ay.sz << J.lc) * 2 * sizeof(float2) > 100 * 1024)) --J.lc;
+        auto col_smem = [&J]() { return ((size_t)J.ay.sz << J.lc) * 2 * sizeof(float2); };
+        while (J.lc > 1 && (points / per < 2 * 148 || col_smem() > (nj == 1 ? 72u : 100u) * 1024)) --J.lc;
+        if (col_smem() > 100 * 1024) J.lc = 0;
         for (uint32_t p = 0; p < (J.Y + 1) / 2; p += J.rows_f) list[0].push_back({(uint32_t)j, p});
         const size_t csm = ((size_t)J.ay.sz << J.lc) * 2 * sizeof(float2);
         const int pc = csm <= COL_SMEM_SMALL ? 1 : 3;
@@ -592,7 +613,10 @@ int FftSet::create(const std::vector<JobShape> &shapes) {
         passes[p]->first = (uint32_t)all.size();
         passes[p]->blocks = (uint32_t)list[p].size();
         passes[p]->smem = smem[p];
-        passes[p]->threads = p == 3 ? NT_LARGE : NT;
+        // the first pass of one grid has few blocks, of a pair of rows each when
+        // they are long: a thread for every item (1200x701 67.4 -> 62.5 us)
+        const bool few = p == 0 && nj == 1 && list[p].size() < 3 * 148 && fewest_items(jobs_host[0].ax) > NT;
+        passes[p]->threads = p == 3 || few ? NT_LARGE : NT;
         all.insert(all.end(), list[p].begin(), list[p].end());
     }
     TPT_CUDA(cudaMalloc(&jobs, std::max<size_t>(nj, 1) * sizeof(Job)));
