@@ -106,10 +106,14 @@ struct Group {
     uint32_t MpT;                        // T: row length of aRiT (G * Yp rounded up to 32)
     uint32_t SR, sbox, snb;              // T: strip rows per (f, kx); TMA box rows; boxes per strip
     uint32_t wR, wRI;                    // N tile widths of R (complex columns) and R^-1 (multiples of 16)
+    // The y DFT's slots: kh = Y rounded up to 32; slot ky < Y is the cosine of
+    // ky, slot kh + ky its sine, and slot kh, where the sine of 0 would be, the
+    // cosine of ky = Y = N2/2.
+    uint32_t kh;
     uint32_t wC;                         // N tile width of C and C^-1 (complex columns; 128, 64 or 32)
     bf16 *aR, *bC, *bCi, *aRi;           // data operands (planes stacked), DFT form
     bf16 *bT, *aRiT;                     // T's A operand [plane][kx][inst][re/im][y]; R^-1's A [plane][f][kx][m']
-    const float *kxs, *kys;              // imaginary parts of the kernel spectra, [kx][ky]
+    const float *kxs, *kys;              // imaginary parts of the kernel spectra, [kx][slot] (spectra_y)
 };
 
 struct InstIO {
@@ -171,19 +175,19 @@ __global__ void __launch_bounds__(THREADS, 1)
     // [kx of Re C | kx of Im C] against [G1r ; -G1i]: each K tile loads one
     // hi/lo plane pair of A and of B, and its N tiles are 256 wide. T's B
     // (the Toeplitz strip) lives outside the ring.
-    constexpr bool A_COMPLEX = STAGE == ST_C || STAGE == ST_CI;
+    constexpr bool Y_DFT = STAGE == ST_C || STAGE == ST_CI;
     constexpr bool B_COMPLEX = STAGE == ST_R || STAGE == ST_C || STAGE == ST_CI;
     constexpr bool OUT_COMPLEX = B_COMPLEX;
     constexpr bool WIDE = STAGE == ST_RI || STAGE == ST_T;         // real N tiles of 256
     constexpr uint32_t NTS = WIDE ? 2 * NT : NT;                     // N tile (complex columns if complex)
-    constexpr uint32_t A_PLANES = A_COMPLEX ? 4 : 2;
+    constexpr uint32_t A_PLANES = 2;
     constexpr uint32_t B_PLANES = STAGE == ST_T ? 0 : (B_COMPLEX ? 4 : 2);
     constexpr uint32_t BPB = STAGE == ST_RI ? 2 * TILE_BYTES : TILE_BYTES;  // bytes of one B plane
     constexpr uint32_t SBYTES = A_PLANES * TILE_BYTES + B_PLANES * BPB;   // one stage
     constexpr uint32_t RING = STAGE == ST_T                       ? T_RING_BYTES
                               : (STAGE == ST_R || STAGE == ST_RI) ? RING_R_BYTES
                                                                   : RING_BYTES;
-    constexpr uint32_t NSTG = RING / SBYTES < MAX_STAGES ? RING / SBYTES : MAX_STAGES;  // 3 (C, C^-1), 4, 6 (T)
+    constexpr uint32_t NSTG = RING / SBYTES < MAX_STAGES ? RING / SBYTES : MAX_STAGES;  // 3 (R, R^-1), 4 (C, C^-1), 6 (T)
     constexpr uint32_t B_OFF = A_PLANES * TILE_BYTES;
     constexpr uint32_t BLO = (B_COMPLEX ? 2 : 1) * BPB;  // B lo block from B hi block
     static_assert(NSTG >= 3, "stage ring");
@@ -236,7 +240,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 // tiles are the group's N width (little padding of N1h or X; narrow for few tiles)
                 const uint32_t wN = STAGE == ST_R    ? groups[P.group].wR
                                     : STAGE == ST_RI ? groups[P.group].wRI
-                                    : A_COMPLEX      ? groups[P.group].wC
+                                    : Y_DFT          ? groups[P.group].wC
                                                      : NTS;
                 const int32_t n0 = T.nt * wN;
                 const uint32_t tx = STAGE == ST_T ? SBYTES : A_PLANES * TILE_BYTES + B_PLANES * wN * KT * 2;
@@ -316,9 +320,9 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const bool amn = STAGE == ST_RI && P.a_mn != 0;
                 const uint32_t nmma = STAGE == ST_T ? groups[P.group].nTy : 128u;
                 const uint32_t kpT = STAGE == ST_T ? groups[P.group].kpC : 0u;
-                const uint32_t wC = A_COMPLEX ? groups[P.group].wC : 128u;
+                const uint32_t wC = Y_DFT ? groups[P.group].wC : 128u;
                 const uint32_t IT = tc::idesc_bf16(128, nmma, false, amn);
-                const uint32_t IC = tc::idesc_bf16(128, wC), ICN = tc::idesc_bf16(128, wC, true);
+                const uint32_t IC = tc::idesc_bf16(128, wC);
                 const uint32_t wRI = STAGE == ST_RI ? groups[P.group].wRI : 256u;
                 const uint32_t IRI = tc::idesc_bf16(128, wRI, false, amn), IRIN = tc::idesc_bf16(128, wRI, true, amn);
                 const uint32_t IR = tc::idesc_bf16(128, STAGE == ST_R ? groups[P.group].wR : 128u);
@@ -377,7 +381,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                             tc::mma_bf16(d + 128, arl, tc::sdesc_k64(bhi + TILE_BYTES + o), IR, 1);
                         } else {
                             if (wC == 128u) {
-                                // [Dr | Di] += Ar * [Br | Bi]
+                                // [Dr | Di] += A * [Br | Bi]
                                 tc::mma_bf16(d, arh, tc::sdesc_k64(bhi + o), I256, first);
                                 tc::mma_bf16(d, arh, tc::sdesc_k64(blo + o), I256, 1);
                                 tc::mma_bf16(d, arl, tc::sdesc_k64(bhi + o), I256, 1);
@@ -388,16 +392,6 @@ __global__ void __launch_bounds__(THREADS, 1)
                                 tc::mma_bf16(d + 128, arh, tc::sdesc_k64(bhi + TILE_BYTES + o), IC, first);
                                 tc::mma_bf16(d + 128, arh, tc::sdesc_k64(blo + TILE_BYTES + o), IC, 1);
                                 tc::mma_bf16(d + 128, arl, tc::sdesc_k64(bhi + TILE_BYTES + o), IC, 1);
-                            }
-                            if (A_COMPLEX) {
-                                const uint64_t aih = ad(2), ail = ad(3);
-                                // Dr -= Ai * Bi ; Di += Ai * Br
-                                tc::mma_bf16(d, aih, tc::sdesc_k64(bhi + TILE_BYTES + o), ICN, 1);
-                                tc::mma_bf16(d, aih, tc::sdesc_k64(blo + TILE_BYTES + o), ICN, 1);
-                                tc::mma_bf16(d, ail, tc::sdesc_k64(bhi + TILE_BYTES + o), ICN, 1);
-                                tc::mma_bf16(d + 128, aih, tc::sdesc_k64(bhi + o), IC, 1);
-                                tc::mma_bf16(d + 128, aih, tc::sdesc_k64(blo + o), IC, 1);
-                                tc::mma_bf16(d + 128, ail, tc::sdesc_k64(bhi + o), IC, 1);
                             }
                         }
                     }
@@ -437,19 +431,24 @@ __global__ void __launch_bounds__(THREADS, 1)
             const uint32_t mrow0 = T.mt * MT + q * 32;  // first row of this warp
             const uint32_t m = mrow0 + lane;            // this thread's row
             const uint32_t d = tmem + acc * 256 + ((q * 32u) << 16);
-            const uint32_t wN = STAGE == ST_R ? Gp.wR : STAGE == ST_RI ? Gp.wRI : A_COMPLEX ? Gp.wC : NTS;
+            const uint32_t wN = STAGE == ST_R ? Gp.wR : STAGE == ST_RI ? Gp.wRI : Y_DFT ? Gp.wC : NTS;
             for (uint32_t c0 = half * 32; c0 < wN; c0 += 64) {
                 const uint32_t nb = T.nt * wN + c0, jmax = wN - c0;  // columns j < jmax belong to the tile
                 const bool row_ok = m < P.M;
                 if constexpr (STAGE == ST_C) {
-                    // row m = ky ; col = (inst, kx) -> B operand of C^-1: row (inst, f, kx), k = ky.
-                    // S_f = B * i Ks_f: real = -Bi Ks, imag = Br Ks. Each part is
+                    // row m = slot ; col = (inst, kx) -> B operand of C^-1: row
+                    // (inst, f, kx), k = slot. With U the cosine row and V the
+                    // sine row of ky, and Kx even and Ky odd in ky:
+                    //   field x: cosine slot  i Kx U, sine slot -i Kx V
+                    //   field y: cosine slot   -Ky V, sine slot   -Ky U
+                    // so x keeps its slot and y changes it. Each part is
                     // transposed through shared memory so each lane writes one
-                    // destination row's 32 consecutive ky as 16-byte stores.
+                    // destination row's 32 consecutive slots as 16-byte stores.
                     const uint32_t il = nb / Gp.N1hp, kx0 = nb - il * Gp.N1hp;
                     if (mrow0 >= P.M || il >= Gp.G) continue;  // warp-uniform
                     const size_t plane = (size_t)Gp.rowsCi * Gp.kpCi;
                     const uint32_t kx = kx0 + lane;  // after the transpose
+                    const bool sine = mrow0 >= Gp.kh;  // kh is a multiple of 32
                     // Each field's 32 spectrum values are loaded once (one round
                     // trip) and serve both parts.
 #pragma unroll 1
@@ -458,17 +457,19 @@ __global__ void __launch_bounds__(THREADS, 1)
                         float kv[32];
 #pragma unroll
                         for (int j = 0; j < 32; ++j)
-                            kv[j] = (row_ok && kx0 + j < Gp.N1h) ? __ldg(ks + (size_t)(kx0 + j) * Gp.N2 + m) : 0.0f;
+                            kv[j] = kx0 + j < Gp.N1h ? __ldg(ks + (size_t)(kx0 + j) * 2 * Gp.kh + m) : 0.0f;
+                        const uint32_t k0 = f == 0 ? mrow0 : sine ? mrow0 - Gp.kh : mrow0 + Gp.kh;
 #pragma unroll 1
                         for (int part = 0; part < 2; ++part) {
                             float v[32];
-                            tc::tmem_ld32(d + (part ? 0u : 128u) + c0, v);  // part 0 needs Bi, part 1 Br
-                            const float sgn = part ? 1.0f : -1.0f;
+                            // x takes the other part (times i), y the same
+                            tc::tmem_ld32(d + (part != f ? 0u : 128u) + c0, v);
+                            const float sgn = f == 0 && (part == 1) != sine ? 1.0f : -1.0f;
 #pragma unroll
                             for (int j = 0; j < 32; ++j) xbuf[lane * 33 + j] = sgn * v[j] * kv[j];
                             __syncwarp();
                             if (kx < Gp.N1h) {
-                                bf16 *o = Gp.bCi + (size_t)((il * 2 + f) * Gp.N1hp + kx) * Gp.kpCi + mrow0 +
+                                bf16 *o = Gp.bCi + (size_t)((il * 2 + f) * Gp.N1hp + kx) * Gp.kpCi + k0 +
                                           (size_t)(2 * part) * plane;
                                 uint32_t hw[16], lw[16];
 #pragma unroll
@@ -723,6 +724,26 @@ __global__ void dft_matrix(bf16 *out, uint32_t rows, uint32_t kvalid, uint32_t k
     split_store_d(out + 2 * plane + e, out + 3 * plane + e, w * (double)sign * s);
 }
 
+// The y DFT's real matrices into 2 planes, for the 2 kh slots described at
+// Group::kh: forward, a slot per row and k = y, the sines negated; inverse,
+// rows y and k = slot. Slots that no frequency takes stay zero.
+__global__ void half_dft_matrix(bf16 *out, uint32_t kh, uint32_t pitch, uint32_t n, int inverse) {
+    const uint32_t Y = n / 2;
+    const size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= (size_t)(Y + 1) * Y) return;
+    const uint32_t ky = (uint32_t)(id / Y), y = (uint32_t)(id - (size_t)ky * Y);
+    const uint64_t t = ((uint64_t)ky * y) % n;
+    double s, c;
+    sincospi(2.0 * (double)t / (double)n, &s, &c);
+    const size_t plane = (size_t)(inverse ? Y : 2 * kh) * pitch;
+    auto put = [&](uint32_t slot, double v) {
+        const size_t e = inverse ? (size_t)y * pitch + slot : (size_t)slot * pitch + y;
+        split_store_d(out + e, out + plane + e, v);
+    };
+    put(ky < Y ? ky : kh, c);
+    if (ky > 0 && ky < Y) put(kh + ky, inverse ? s : -s);
+}
+
 // Imaginary parts of the x/y kernel spectra, first over x:
 // tx[j][kx] = sum_dx Kx(dx, dy_j) sin(2 pi kx dx / N1), ty = sum_dx Ky cos(..),
 // with K(d) = scale * d / |d|^3, d folded into (-N/2, N/2) (the +N/2 offset
@@ -755,10 +776,15 @@ __global__ void spectra_x(double *tx, double *ty, uint32_t N1, uint32_t N2, uint
     ty[id] = sy;
 }
 
-// then over y: kxs = -sum_j tx[j] cos(2 pi ky j / N2), kys = -sum_j ty[j] sin(..)
-__global__ void spectra_y(const double *tx, const double *ty, float *kxs, float *kys, uint32_t N2, uint32_t N1h) {
+// then over y, for each slot: Kx = -sum_j tx[j] cos(2 pi ky j / N2), Ky = -sum_j
+// ty[j] sin(..), even and odd in ky, twice where ky stands for -ky too. The slot
+// of ky = N2/2 is a cosine among the sines, whose signs are opposite in x; Ky
+// is zero at 0 and N2/2.
+__global__ void spectra_y(const double *tx, const double *ty, float *kxs, float *kys, uint32_t N2, uint32_t N1h,
+                          uint32_t kh) {
+    const uint32_t Y = N2 / 2;
     size_t id = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= (size_t)N2 * N1h) return;
+    if (id >= (size_t)(Y + 1) * N1h) return;
     uint32_t ky = (uint32_t)(id / N1h), kx = (uint32_t)(id - (size_t)ky * N1h);
     double ax = 0.0, ay = 0.0;
     for (uint32_t j = 0; j < N2; ++j) {
@@ -768,8 +794,15 @@ __global__ void spectra_y(const double *tx, const double *ty, float *kxs, float 
         ax += tx[(size_t)j * N1h + kx] * c;
         ay += ty[(size_t)j * N1h + kx] * s;
     }
-    kxs[(size_t)kx * N2 + ky] = (float)(-ax);
-    kys[(size_t)kx * N2 + ky] = (float)(-ay);
+    float *x = kxs + (size_t)kx * 2 * kh, *y = kys + (size_t)kx * 2 * kh;
+    if (ky == 0) {
+        x[0] = (float)-ax;
+    } else if (ky == Y) {
+        x[kh] = (float)ax;
+    } else {
+        x[ky] = x[kh + ky] = (float)(-2.0 * ax);
+        y[ky] = y[kh + ky] = (float)(-2.0 * ay);
+    }
 }
 
 // Toeplitz strips of the y stage, into 2 planes: row (f * N1h + kx) * SR + r,
@@ -1006,7 +1039,8 @@ int DftSet::create(const std::vector<JobShape> &shapes) {
         inst0 += g.G;
         g.kpR = round_up(g.X, KT);
         g.kpC = round_up(g.Y, KT);
-        g.kpCi = round_up(g.N2, KT);
+        g.kh = round_up(g.Y, KT);
+        g.kpCi = 2 * g.kh;
         g.kpRi = round_up(g.N1h, KT);
         g.rowsR = g.G * g.Y;
         g.rowsC = g.G * g.N1hp;
@@ -1026,14 +1060,14 @@ int DftSet::create(const std::vector<JobShape> &shapes) {
         g.snb = (g.SR + T_NMAX - 1) / T_NMAX;                    // TMA boxes per strip (box rows <= 256)
         g.sbox = round_up((g.SR + g.snb - 1) / g.snb, 8);        // box rows, 512-byte multiples
         H.kpF1 = g.kpR;   // F1: N1h rows, K = x
-        H.kpF2 = g.kpC;   // F2: N2 rows, K = y
-        H.kpG2 = g.kpCi;  // G2: Y rows, K = ky
+        H.kpF2 = g.kpC;   // F2: slots, K = y
+        H.kpG2 = g.kpCi;  // G2: Y rows, K = slot
         H.kpG1 = g.kpRi;  // G1: X rows, K = kx
         // executed tensor flops (3-term split, padded tiles) of both y forms
         auto tiles_of = [](uint32_t v, uint32_t t) { return (double)((v + t - 1) / t) * t; };
         const double fR = 2.0 * tiles_of(g.rowsR, MT) * tiles_of(g.N1h, g.wR) * 2 * g.kpR * 3;
-        const double fC = 2.0 * tiles_of(g.N2, MT) * tiles_of(g.rowsC, g.wC) * 4 * g.kpC * 3;
-        const double fCi = 2.0 * tiles_of(g.Y, MT) * tiles_of(g.rowsCi, g.wC) * 4 * g.kpCi * 3;
+        const double fC = 2.0 * tiles_of(2 * g.kh, MT) * tiles_of(g.rowsC, g.wC) * 2 * g.kpC * 3;
+        const double fCi = 2.0 * tiles_of(g.Y, MT) * tiles_of(g.rowsCi, g.wC) * 2 * g.kpCi * 3;
         const double fRi = 2.0 * tiles_of(g.rowsRi, MT) * tiles_of(g.X, g.wRI) * 2 * g.kpRi * 3;
         const double fT = 2.0 * 2 * g.N1h * tiles_of(2 * g.G, MT) * g.nTy * g.kpC * 3;
         const double fRiT = 2.0 * 2 * tiles_of(g.G * g.Yp, MT) * tiles_of(g.X, g.wRI) * 2 * g.kpRi * 3;
@@ -1059,11 +1093,11 @@ int DftSet::create(const std::vector<JobShape> &shapes) {
             if ((rc = I->alloc(&g.bC, (size_t)4 * g.rowsC * g.kpC))) return rc;
             if ((rc = I->alloc(&g.bCi, (size_t)4 * g.rowsCi * g.kpCi))) return rc;
             if ((rc = I->alloc(&g.aRi, (size_t)4 * g.rowsRi * g.kpRi))) return rc;
-            if ((rc = I->alloc(&H.f2, (size_t)4 * g.N2 * H.kpF2))) return rc;
-            if ((rc = I->alloc(&H.g2, (size_t)4 * g.Y * H.kpG2))) return rc;
-            if ((rc = I->alloc(&H.kxs, (size_t)2 * g.N2 * g.N1h))) return rc;
+            if ((rc = I->alloc(&H.f2, (size_t)2 * 2 * g.kh * H.kpF2))) return rc;
+            if ((rc = I->alloc(&H.g2, (size_t)2 * g.Y * H.kpG2))) return rc;
+            if ((rc = I->alloc(&H.kxs, (size_t)2 * 2 * g.kh * g.N1h))) return rc;
             g.kxs = H.kxs;
-            g.kys = H.kxs + (size_t)g.N2 * g.N1h;
+            g.kys = H.kxs + (size_t)2 * g.kh * g.N1h;
         }
         // constants in FP64, rounded once to the hi/lo planes
         auto blocks = [](size_t cnt) { return (unsigned)((cnt + 255) / 256); };
@@ -1080,14 +1114,14 @@ int DftSet::create(const std::vector<JobShape> &shapes) {
             spectra_x<<<blocks((size_t)g.N2 * g.N1h), 256>>>(tx, ty, g.N1, g.N2, g.N1h, scale);
             toeplitz_strip<<<blocks((size_t)2 * g.N1h * g.SR * KT), 256>>>(tx, ty, H.ts, g.SR, g.N2, g.N1h, g.kpC);
         } else {
-            dft_matrix<<<blocks((size_t)g.N2 * g.Y), 256>>>(H.f2, g.N2, g.Y, H.kpF2, g.N2, -1, 0);
-            dft_matrix<<<blocks((size_t)g.Y * g.N2), 256>>>(H.g2, g.Y, g.N2, H.kpG2, g.N2, +1, 0);
+            half_dft_matrix<<<blocks((size_t)(g.Y + 1) * g.Y), 256>>>(H.f2, g.kh, H.kpF2, g.N2, 0);
+            half_dft_matrix<<<blocks((size_t)(g.Y + 1) * g.Y), 256>>>(H.g2, g.kh, H.kpG2, g.N2, 1);
             count_launch();
             count_launch();
             const double scale = -(double)6.673e-1f / ((double)g.N1 * (double)g.N2);
             spectra_x<<<blocks((size_t)g.N2 * g.N1h), 256>>>(tx, ty, g.N1, g.N2, g.N1h, scale);
-            spectra_y<<<blocks((size_t)g.N2 * g.N1h), 256>>>(tx, ty, H.kxs, H.kxs + (size_t)g.N2 * g.N1h, g.N2,
-                                                             g.N1h);
+            spectra_y<<<blocks((size_t)(g.Y + 1) * g.N1h), 256>>>(tx, ty, H.kxs, H.kxs + (size_t)2 * g.kh * g.N1h,
+                                                                  g.N2, g.N1h, g.kh);
         }
         count_launch();
         count_launch();
@@ -1165,14 +1199,14 @@ int DftSet::create(const std::vector<JobShape> &shapes) {
             }
         } else {
             // stage C: A = F2, B = bC
-            if ((rc = make_tmap(&tmh[2], H.f2, H.kpF2, 4 * g.N2))) return rc;
+            if ((rc = make_tmap(&tmh[2], H.f2, H.kpF2, 2 * 2 * g.kh))) return rc;
             if ((rc = make_tmap(&tmh[3], g.bC, g.kpC, 4 * g.rowsC, g.wC))) return rc;
             // stage C^-1: A = G2, B = bCi
-            if ((rc = make_tmap(&tmh[4], H.g2, H.kpG2, 4 * g.Y))) return rc;
+            if ((rc = make_tmap(&tmh[4], H.g2, H.kpG2, 2 * g.Y))) return rc;
             if ((rc = make_tmap(&tmh[5], g.bCi, g.kpCi, 4 * g.rowsCi, g.wC))) return rc;
             // stage R^-1: A = aRi, B = G1
             if ((rc = make_tmap(&tmh[6], g.aRi, g.kpRi, 4 * g.rowsRi))) return rc;
-            pr.push_back({tmd + 2, tmd + 3, gi32, g.N2, g.rowsC, g.kpC / KT, g.N2, g.rowsC, 0});
+            pr.push_back({tmd + 2, tmd + 3, gi32, 2 * g.kh, g.rowsC, g.kpC / KT, 2 * g.kh, g.rowsC, 0});
             add_tiles(ST_C, (uint32_t)pr.size() - 1, true);
             pr.push_back({tmd + 4, tmd + 5, gi32, g.Y, g.rowsCi, g.kpCi / KT, g.Y, g.rowsCi, 0});
             add_tiles(ST_CI, (uint32_t)pr.size() - 1, true);
