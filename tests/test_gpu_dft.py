@@ -263,3 +263,25 @@ def test_split_bf16_tile_widths(cuda, tf, oracle, shapes):
             emax, el2 = errors(got[k], d)
             assert emax <= TOL and el2 <= TOL, (i, k, emax, el2)
     b.close()
+
+
+@pytest.mark.parametrize("X,Y", [(5, 1), (40, 2), (9, 31), (33, 32), (20, 33), (64, 63), (31, 64), (8, 65), (600, 500)])
+def test_split_bf16_y_slots(cuda, tf, oracle, X, Y):
+    """The y DFT's cosine and sine slots at the edges of their 32-slot chunks
+    (Y of 1 has no sine at all), and a grid whose y stages take wider tiles
+    than R; the FP64 bars."""
+    rng = np.random.default_rng(100 * X + Y)
+    mass = (rng.uniform(-1.0, 3.0, X * Y) * (rng.random(X * Y) < 0.3)).astype(np.float32)
+    mass[0] = 1.0
+    b = tf.SimBuffers(tf.SimulationConfig(xres=4 * X, yres=4 * Y, newton_grav=True))
+    b.grav_mask.fill_(-1)
+    s = tf.GravityFft(tf.PRECISION_SPLIT_BF16)
+    s.solve(b, cuda.from_numpy(mass).cuda())
+    cuda.cuda.synchronize()
+    check_clean(tf)
+    dx, dy = oracle.grav_solve(X, Y, np.full(X * Y, 0xFFFFFFFF, np.uint32), mass_f32=mass, dtype=np.float64)
+    for got, d in ((b.grav_fx, dx), (b.grav_fy, dy)):
+        if np.abs(d).max() > 1e-6 * max(np.abs(dx).max(), np.abs(dy).max()):
+            emax, el2 = errors(got.cpu().numpy(), d)
+            assert emax <= TOL and el2 <= TOL, (emax, el2)
+    s.close()

@@ -985,6 +985,31 @@ static uint32_t tile_width(const std::vector<JobShape> &shapes) {
     return 32;
 }
 
+// The N tile of C and C^-1 for few grids. They have two to four times R's tiles,
+// so R's width can give them two rounds of narrow tiles where one round of
+// wider ones is cheaper: a K tile loads 64 + w units of 256 bytes (A's 128 rows,
+// B's w columns), and a stage lasts as many of those as its rounds. Measured on
+// B200 at 32 and 64 columns, one solve: 256x256 48.7 and 55.3 us, 512x512 74.3
+// and 80.8, 700x700 134 and 105.
+static uint32_t y_tile_width(const std::vector<JobShape> &shapes, uint32_t width) {
+    uint32_t best = width;
+    size_t least = SIZE_MAX;
+    for (uint32_t w = NT; w >= 32 && width < (uint32_t)NT; w /= 2) {
+        size_t c = 0, ci = 0;
+        for (const JobShape &s : shapes) {
+            const size_t cols = ((size_t)s.X + 1 + 31) / 32 * 32, slots = ((size_t)s.Y + KT - 1) / KT * KT * 2;
+            c += (slots + MT - 1) / MT * ((cols + w - 1) / w);
+            ci += ((size_t)s.Y + MT - 1) / MT * ((2 * cols + w - 1) / w);
+        }
+        const size_t cost = ((c + 147) / 148 + 2 * ((ci + 147) / 148)) * (64 + w);  // C^-1: twice the K
+        if (cost < least) {
+            least = cost;
+            best = w;
+        }
+    }
+    return best;
+}
+
 int DftSet::create(const std::vector<JobShape> &shapes) {
     destroy();
     int rc = init_attrs();
@@ -1019,6 +1044,7 @@ int DftSet::create(const std::vector<JobShape> &shapes) {
     I->inst_local.resize(n);
     I->hg.resize(members.size());
     const uint32_t width = tile_width(shapes);
+    const uint32_t y_width = y_tile_width(shapes, width);
     I->dependent = width < (uint32_t)NT;
     uint32_t inst0 = 0;
     for (size_t gi = 0; gi < members.size(); ++gi) {
@@ -1056,7 +1082,7 @@ int DftSet::create(const std::vector<JobShape> &shapes) {
         const uint32_t ntR = (g.N1h + width - 1) / width, ntRI = (g.X + 2 * width - 1) / (2 * width);
         g.wR = round_up((g.N1h + ntR - 1) / ntR, 16);
         g.wRI = round_up((g.X + ntRI - 1) / ntRI, 16);
-        g.wC = width;
+        g.wC = y_width;
         g.snb = (g.SR + T_NMAX - 1) / T_NMAX;                    // TMA boxes per strip (box rows <= 256)
         g.sbox = round_up((g.SR + g.snb - 1) / g.snb, 8);        // box rows, 512-byte multiples
         H.kpF1 = g.kpR;   // F1: N1h rows, K = x
