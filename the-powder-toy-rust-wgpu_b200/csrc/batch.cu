@@ -976,7 +976,7 @@ int tpt_batch_profile_phases(tpt_batch *b, uint32_t ticks, tpt_stream_t stream, 
     // form: pass A + pass B, which is two launches as strips (+ a settle pass
     // when an instance is NoUpdate with ambient heat)
     out->air_launches_per_tick = b->sweep_form() ? 2 : (b->use_strips ? 3 : 2) + (b->any_noupdate_heat ? 1 : 0);
-    out->grav_launches_per_tick = b->any_grav ? (b->precision == TPT_PRECISION_FP32 ? 3 : b->dft.launches()) : 0;
+    out->grav_launches_per_tick = b->any_grav ? (b->precision == TPT_PRECISION_FP32 ? b->fft.launches() : b->dft.launches()) : 0;
     out->grav_flops_per_tick = b->any_grav && b->precision != TPT_PRECISION_FP32 ? b->dft.flops() : 0.0;
     cudaEvent_t e0, e1, e2;
     TPT_CUDA(cudaEventCreate(&e0));

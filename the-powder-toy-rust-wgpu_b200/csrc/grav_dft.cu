@@ -640,10 +640,13 @@ struct PrepRef {
     uint32_t group, row;  // row = inst_local * Y + y
 };
 
-__global__ void prep_mass(const Group *__restrict__ groups, const PrepRef *__restrict__ refs,
+constexpr uint32_t PREP_ROWS = 4, PREP_LANES = 64;  // rows per block, threads per row
+__global__ void prep_mass(const Group *__restrict__ groups, const PrepRef *__restrict__ refs, uint32_t nrefs,
                           const InstIO *__restrict__ ios, InstIO io0, int io0_active) {
     pdl_release();
-    const PrepRef r = refs[blockIdx.x];
+    const uint32_t ref = blockIdx.x * PREP_ROWS + threadIdx.x / PREP_LANES, lane = threadIdx.x % PREP_LANES;
+    if (ref >= nrefs) return;
+    const PrepRef r = refs[ref];
     const Group Gp = groups[r.group];
     const uint32_t il = r.row / Gp.Y, y = r.row - il * Gp.Y, inst = Gp.inst0 + il;
     const InstIO io = (io0_active && inst == 0) ? io0 : ios[inst];
@@ -656,7 +659,7 @@ __global__ void prep_mass(const Group *__restrict__ groups, const PrepRef *__res
     // the aR row is 64-byte aligned and padded to a multiple of 32.
     const bool vec = (io.pitch & 7u) == 0u &&
                      ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(io.mask + c0)) & 15u) == 0u;
-    for (uint32_t x0 = threadIdx.x * 8; x0 < Gp.X; x0 += blockDim.x * 8) {
+    for (uint32_t x0 = lane * 8; x0 < Gp.X; x0 += PREP_LANES * 8) {
         float v[8];
         if (vec) {
             const uint4 *mk = reinterpret_cast<const uint4 *>(io.mask + c0 + x0);
@@ -1333,7 +1336,8 @@ int DftSet::launch(cudaStream_t st, const SolveIO *io) const {
         io0 = InstIO{io->mass_i, io->mass_f, io->mask, io->gx, io->gy, io->mass_scale_inv, io->pitch};
         act = 1;
     }
-    prep_mass<<<I->nprep, 64, 0, st>>>(I->groups, I->prep, I->ios, io0, act);
+    prep_mass<<<(I->nprep + PREP_ROWS - 1) / PREP_ROWS, PREP_ROWS * PREP_LANES, 0, st>>>(I->groups, I->prep, I->nprep,
+                                                                                         I->ios, io0, act);
     TPT_LAUNCHED();
     int rc;
     if (!split_active()) {

@@ -17,9 +17,9 @@ namespace gfft {
 // of loads (job, grid, twiddles), barriers and instruction fetch, at 24 warps
 // per SM and 16 to 55% of the issue slots; DRAM stays below 15% of its rate.
 // Measured on B200, solve of 256 grids (8.1 M cells, sides 32 to 512):
-// 0.407 ms (0.988 ms with one warp per transform, padded to powers of two and
-// exchanged by lane shuffles); one 400x225 grid 22.6 us (55.3); one 1200x701
-// grid 90 us (698 us with radix-2 passes in shared memory). Blocks of about
+// 0.392 ms (0.988 ms with one warp per transform, padded to powers of two and
+// exchanged by lane shuffles); one 400x225 grid 20.2 us (55.3); one 1200x701
+// grid 63.5 us (698 us with radix-2 passes in shared memory). Blocks of about
 // 2048 row points and 4096 column points: 1024 and 1024 took 0.554 ms, 2048
 // and 2048 0.479, 4096 and 4096 0.464, 8192 and 4096 0.509 (before the grid
 // addresses were hoisted out of the radix loops, at 0.456).

@@ -35,6 +35,12 @@ struct FftSet {
     int upload_jobs();
     // io != null: a one-job set solving on per-call pointers.
     int launch(cudaStream_t st, const JobIO *io = nullptr) const;
+    // Launches of one solve.
+    uint32_t launches() const {
+        uint32_t n = 0;
+        for (const Pass *p : {&rows, &cols[0], &cols[1], &inv}) n += p->blocks > 0 ? 1u : 0u;
+        return n;
+    }
     void destroy();
     ~FftSet() { destroy(); }
 };
