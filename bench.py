@@ -44,12 +44,12 @@ import numpy as np  # noqa: E402
 
 B_AIR = 52  # algorithmic bytes per cell-tick of the air step (reference layout)
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one air tick
-# (both tile-form launches) and of one gravity solve of the whole batch (the
+# (its three strip launches) and of one gravity solve of the whole batch (the
 # GEMM launches), from ncu captures; workloads without a capture report null.
-# Air: 74.7 bytes per cell-tick measured on the first 32 instances of the
+# Air: 85.1 bytes per cell-tick measured on the first 32 instances of the
 # 128-instance batch (2.88 M cells, well above L2) after 900 ticks, scaled by
 # its 6,121,601 cells (traffic grows with the cells staged).
-MEASURED_DRAM_BYTES = {5: {"air_tick": 457.3e6, "grav_solve": 418.4e6}}
+MEASURED_DRAM_BYTES = {5: {"air_tick": 521.2e6, "grav_solve": 400.7e6}}
 WORKLOAD_NAMES = {
     1: "C1 plain FP32 air+gravity, 153x96 cells (612x384 canvas)",
     2: "C2 plain FP32 air+gravity, 400x225 cells (1600x900 canvas)",
@@ -664,7 +664,7 @@ def run_voxel3d(args, rank, world, local):
     b_grav = 4 * W.VOX_VOXELS + 4 * nonempty + 8 * W.VOX_CELLS
     gbs_air = b_air / (phase["air_gather"] / 1e3) / 1e9
     gbs_grav = b_grav / (phase["grav_gather"] / 1e3) / 1e9
-    roof_grav = {"kernel": "gravity gather (k_brick_mult + k_grav_gather_rows)", "bound": "hbm",
+    roof_grav = {"kernel": "gravity gather (k_grav_gather_list + k_grav_gather_rows)", "bound": "hbm",
                  "achieved": round(gbs_grav, 1), "peak": hbm,
                  "unit": "GB/s", "frac": round(gbs_grav / hbm, 4), "peak_source": peak_src,
                  "algorithmic_bytes_per_launch": b_grav, "avg_launch_ms": round(phase["grav_gather"], 5),
