@@ -498,8 +498,8 @@ def run_ours(args, rank, world, local):
 
 # -------------------------------------------------------------- 3-D ----
 # ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_grav_gather_rows
-# launch on the bench's world with every brick listed (134.3 MB + 4.0 MB)
-VOX_GRAV_GATHER_DRAM_BYTES = 138.3e6
+# launch on the bench's world with every brick listed (134.3 MB + 0.3 MB)
+VOX_GRAV_GATHER_DRAM_BYTES = 134.6e6
 VOX_NAME = ("3-D sandbox field step, 64^3 cells per world over 256^3 voxels with every brick active: air gather, "
             "air solve (12 Jacobi sweeps), gravity solve (24 sweeps), clear mass, gravity gather")
 
