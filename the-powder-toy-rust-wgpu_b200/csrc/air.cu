@@ -24,12 +24,10 @@ namespace air {
 // launches) and now: 16x16 10.9 and 8.1, 64x48 16.3 and 11.4, 153x96 18.5 and
 // 13.4, 300x200 18.6 and 14.3, 401x225 20.2 and 16.7, 512x512 32.0 and 27.7,
 // 590x590 39.8 and 35.4; as strips, launches alone: 1024x1024 84.8 and 76.9,
-// 2048x2048 249.5 and 240.3 in calls back to back.
+// 2048x2048 249.5 and 244.7 in calls back to back.
 constexpr int NT_A = 448, NT_B = 384;
 static_assert(NT_A >= (TX + 4) * (TY + 4) && NT_B >= (TX + 2) * (TY + 2), "a ring is one turn");
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... Args>
 static int launch_pdl(void (*kernel)(Args...), dim3 grid, unsigned block, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
@@ -88,7 +86,7 @@ __global__ void __launch_bounds__(NT_B) k_advect_heat(const AirInst I) {
 // walks its rows one after the other: below about 300,000 cells the tiles, a
 // thread per cell, are done sooner. Measured on B200, us per tick, tiles and
 // strips: 401x225 16.4 and 24.1, 512x512 27.8 and 28.8, 590x590 35.7 and 33.7,
-// 700x600 40.3 and 37.8, 1024x1024 87.1 and 76.5, 2048x2048 360 and 240.
+// 700x600 40.3 and 37.8, 1024x1024 87.1 and 76.5, 2048x2048 360 and 245.
 constexpr size_t STRIP_MIN_CELLS = 300000;
 struct OneGrid {
     StripGrids P;

@@ -36,6 +36,7 @@
 
 #include "common.cuh"
 #include "exact_div.cuh"
+#include "pdl.cuh"
 
 #ifndef AIR_TILE_X
 #define AIR_TILE_X AIR_TX
@@ -198,7 +199,7 @@ __device__ __forceinline__ void stage(T *s, const T *g, const AirInst &I, int x0
     for (int i = threadIdx.x; i < Reg<H>::N; i += THREADS) {
         int ly = i / Reg<H>::W, lx = i - ly * Reg<H>::W;
         int gx = x0 - H + lx, gy = y0 - H + ly;
-        s[i] = in_grid(gx, gy, I) ? __ldg(g + (size_t)gy * I.pitch + gx) : T(0);
+        s[i] = in_grid(gx, gy, I) ? load_after_wait(g + (size_t)gy * I.pitch + gx) : T(0);
     }
 }
 template <int H, int THREADS = NT>
@@ -207,7 +208,7 @@ __device__ __forceinline__ void stage_flag(uint8_t *s, const uint32_t *g, uint32
     for (int i = threadIdx.x; i < Reg<H>::N; i += THREADS) {
         int ly = i / Reg<H>::W, lx = i - ly * Reg<H>::W;
         int gx = x0 - H + lx, gy = y0 - H + ly;
-        s[i] = in_grid(gx, gy, I) ? ((__ldg(g + (size_t)gy * I.pitch + gx) & bitmask) != 0u) : 0;
+        s[i] = in_grid(gx, gy, I) ? ((load_after_wait(g + (size_t)gy * I.pitch + gx) & bitmask) != 0u) : 0;
     }
 }
 
@@ -425,7 +426,7 @@ __device__ __forceinline__ void smooth_advect_cell(const AirInst &I, L &S, int x
         x, y, nvx, nvy,
         [&](int cx, int cy) -> bool {
             if (S.has3(cx, cy, x0, y0)) return S.blk(cx, cy, x0, y0);
-            return __ldg(I.bair + (size_t)cy * I.pitch + cx) != 0u;
+            return load_after_wait(I.bair + (size_t)cy * I.pitch + cx) != 0u;
         },
         X, Y, tx0, ty0);
     int i0 = (int)tx0, j0 = (int)ty0;
@@ -447,14 +448,14 @@ __device__ __forceinline__ void smooth_advect_cell(const AirInst &I, L &S, int x
             b11 = S.OVY(i0 + 1, j0 + 1, x0, y0);
         } else {
             size_t r0 = (size_t)j0 * I.pitch + i0, r1 = r0 + I.pitch;
-            a00 = __ldg(I.ovx + r0);
-            a10 = __ldg(I.ovx + r0 + 1);
-            a01 = __ldg(I.ovx + r1);
-            a11 = __ldg(I.ovx + r1 + 1);
-            b00 = __ldg(I.ovy + r0);
-            b10 = __ldg(I.ovy + r0 + 1);
-            b01 = __ldg(I.ovy + r1);
-            b11 = __ldg(I.ovy + r1 + 1);
+            a00 = load_after_wait(I.ovx + r0);
+            a10 = load_after_wait(I.ovx + r0 + 1);
+            a01 = load_after_wait(I.ovx + r1);
+            a11 = load_after_wait(I.ovx + r1 + 1);
+            b00 = load_after_wait(I.ovy + r0);
+            b10 = load_after_wait(I.ovy + r0 + 1);
+            b01 = load_after_wait(I.ovy + r1);
+            b11 = load_after_wait(I.ovy + r1 + 1);
         }
         nvx = nvx * 0.7f + 0.3f * (a00 * w00 + a10 * w10 + a01 * w01 + a11 * w11);
         nvy = nvy * 0.7f + 0.3f * (b00 * w00 + b10 * w10 + b01 * w01 + b11 * w11);
@@ -478,9 +479,9 @@ __device__ __forceinline__ void smooth_advect_cell(const AirInst &I, L &S, int x
         nvy += k * (0.0f - dwx) / (norm + 0.001f) * w;
     }
     size_t g = (size_t)y * I.pitch + x;
-    if (__ldg(I.wall + g) == 5u) {  // WL_FAN, advect.rs:331-334
-        nvx += __ldg(I.fvx + g);
-        nvy += __ldg(I.fvy + g);
+    if (load_after_wait(I.wall + g) == 5u) {  // WL_FAN, advect.rs:331-334
+        nvx += load_after_wait(I.fvx + g);
+        nvy += load_after_wait(I.fvy + g);
     }
     nvx = clampf(nvx, -256.0f, 256.0f);
     nvy = clampf(nvy, -256.0f, 256.0f);
@@ -549,7 +550,7 @@ __device__ __forceinline__ float heat_cell(const AirInst &I, L &S, int x, int y,
         x, y, svx, svy,
         [&](int cx, int cy) -> bool {
             if (S.hasH(cx, cy, x0, y0)) return S.hblk(cx, cy, x0, y0);
-            return (__ldg(I.bairh + (size_t)cy * I.pitch + cx) & 0x8u) != 0u;
+            return (load_after_wait(I.bairh + (size_t)cy * I.pitch + cx) & 0x8u) != 0u;
         },
         X, Y, tx, ty);
     int i0 = (int)tx, j0 = (int)ty;
@@ -564,10 +565,10 @@ __device__ __forceinline__ float heat_cell(const AirInst &I, L &S, int x, int y,
             s11 = S.hblk(i0 + 1, j0 + 1, x0, y0) ? dh : S.HV(i0 + 1, j0 + 1, x0, y0);
         } else {
             size_t r0 = (size_t)j0 * I.pitch + i0, r1 = r0 + I.pitch;
-            s00 = (__ldg(I.bairh + r0) & 0x8u) ? dh : __ldg(I.hv + r0);
-            s10 = (__ldg(I.bairh + r0 + 1) & 0x8u) ? dh : __ldg(I.hv + r0 + 1);
-            s01 = (__ldg(I.bairh + r1) & 0x8u) ? dh : __ldg(I.hv + r1);
-            s11 = (__ldg(I.bairh + r1 + 1) & 0x8u) ? dh : __ldg(I.hv + r1 + 1);
+            s00 = (load_after_wait(I.bairh + r0) & 0x8u) ? dh : load_after_wait(I.hv + r0);
+            s10 = (load_after_wait(I.bairh + r0 + 1) & 0x8u) ? dh : load_after_wait(I.hv + r0 + 1);
+            s01 = (load_after_wait(I.bairh + r1) & 0x8u) ? dh : load_after_wait(I.hv + r1);
+            s11 = (load_after_wait(I.bairh + r1 + 1) & 0x8u) ? dh : load_after_wait(I.hv + r1 + 1);
         }
         float w00 = (1.0f - fx) * (1.0f - fy);
         float w10 = fx * (1.0f - fy);
@@ -709,7 +710,7 @@ __device__ __forceinline__ void masks_cell(const AirInst &I, size_t g, uint32_t 
     const uint32_t raw = emap_seen(stored, lag);
     const uint32_t next = raw != 0u ? raw - 1u : 0u;
     if (next != stored) I.emap[g] = next;
-    masks_of(__ldg(I.wall + g), raw, I.eair ? __ldg(I.eair + g) : 0u, I.eairh ? __ldg(I.eairh + g) : 0u, bair, bairh);
+    masks_of(load_after_wait(I.wall + g), raw, I.eair ? load_after_wait(I.eair + g) : 0u, I.eairh ? load_after_wait(I.eairh + g) : 0u, bair, bairh);
 }
 
 }  // namespace AIR_SHAPE_NS

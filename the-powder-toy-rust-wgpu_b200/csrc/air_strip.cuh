@@ -86,10 +86,10 @@ __device__ __forceinline__ void strip_a(const StripGrids &P, const AirInst &I, u
     uint32_t nb = 0u;
     auto load = [&](int r, uint32_t e) {  // the next row's loads are in flight during a step
         const bool ok = C.in && r >= 0 && r < Y;
-        nvx = ok ? __ldg(P.vx + e) : 0.f;
-        nvy = ok ? __ldg(P.vy + e) : 0.f;
-        npv = ok ? __ldg(P.pv + e) : 0.f;
-        nb = ok ? __ldg(P.bair + e) : 0u;
+        nvx = ok ? load_after_wait(P.vx + e) : 0.f;
+        nvy = ok ? load_after_wait(P.vy + e) : 0.f;
+        npv = ok ? load_after_wait(P.pv + e) : 0.f;
+        nb = ok ? load_after_wait(P.bair + e) : 0u;
     };
     load(y0 - 3, o);
 #pragma unroll 1
@@ -386,11 +386,11 @@ __device__ __forceinline__ void strip_advect(const StripGrids &P, const AirInst 
     uint32_t nb = 0u, nw = 0u;
     auto load = [&](int r, uint32_t e) {  // the next step's loads are in flight during a step
         const bool ok = C.in && r >= 0 && r < Y, okw = out && r - 2 >= 0 && r - 2 < Y;
-        nvx = ok ? __ldg(P.ovx + e) : 0.f;
-        nvy = ok ? __ldg(P.ovy + e) : 0.f;
-        npv = ok ? __ldg(P.opv + e) : 0.f;
-        nb = ok ? __ldg(P.bair + e) : 0u;
-        nw = okw ? __ldg(P.wall + (e - 2u * pitch)) : 0u;
+        nvx = ok ? load_after_wait(P.ovx + e) : 0.f;
+        nvy = ok ? load_after_wait(P.ovy + e) : 0.f;
+        npv = ok ? load_after_wait(P.opv + e) : 0.f;
+        nb = ok ? load_after_wait(P.bair + e) : 0u;
+        nw = okw ? load_after_wait(P.wall + (e - 2u * pitch)) : 0u;
     };
     load(y0 - 2, o);
 #pragma unroll 1
@@ -409,14 +409,14 @@ __device__ __forceinline__ void strip_advect(const StripGrids &P, const AirInst 
         if (mine)
             far_target(xf, (float)a, nx, ny, limx, limy,
                        [&](int cx, int cy) -> bool {
-                           return __ldg(P.bair + (off + (uint32_t)cy * pitch + (uint32_t)cx)) != 0u;
+                           return load_after_wait(P.bair + (off + (uint32_t)cy * pitch + (uint32_t)cx)) != 0u;
                        },
                        tx, ty);
         const Landing q(tx, ty, 2.0f, limx - 1.0f, limy - 1.0f, off, pitch, mine && !(bk2 & 2u));
         // both rows of the sample: cells of the grid in any case (it has two rows and columns)
         const float *q0 = P.ovx + q.g, *q1 = P.ovy + q.g;
-        const float a00 = __ldg(q0), a10 = __ldg(q0 + 1), a01 = __ldg(q0 + pitch), a11 = __ldg(q0 + pitch + 1);
-        const float b00 = __ldg(q1), b10 = __ldg(q1 + 1), b01 = __ldg(q1 + pitch), b11 = __ldg(q1 + pitch + 1);
+        const float a00 = load_after_wait(q0), a10 = load_after_wait(q0 + 1), a01 = load_after_wait(q0 + pitch), a11 = load_after_wait(q0 + pitch + 1);
+        const float b00 = load_after_wait(q1), b10 = load_after_wait(q1 + 1), b01 = load_after_wait(q1 + pitch), b11 = load_after_wait(q1 + pitch + 1);
         // the means of row r - 1 get this row's taps, row r's begin (advect.rs:192-253)
         const uint32_t cl0 = around(row0 | C.not_inner | (r < 1 || r + 1 >= Y ? ~0u : 0u), lane);
         const Closed k0(cl0), k1(cl1);
@@ -450,8 +450,8 @@ __device__ __forceinline__ void strip_advect(const StripGrids &P, const AirInst 
             }
             const uint32_t w = o - 2u * pitch;
             if (wall2 == 5u) {  // WL_FAN, advect.rs:331-334
-                nx += __ldg(P.fvx + w);
-                ny += __ldg(P.fvy + w);
+                nx += load_after_wait(P.fvx + w);
+                ny += load_after_wait(P.fvy + w);
             }
             nx = clamp_speed(nx);
             ny = clamp_speed(ny);
@@ -506,10 +506,10 @@ __device__ __forceinline__ void strip_heat(const StripGrids &P, const AirInst &I
     uint32_t nbh = 0u;
     auto load = [&](int r, uint32_t e) {  // the next step's loads are in flight during a step
         const bool ok = C.in && r >= 0 && r < Y;
-        nu = ok ? __ldg((STORED ? P.vx : iu) + e) : 0.f;
-        nv = ok ? __ldg((STORED ? P.vy : iv) + e) : 0.f;
-        nh = ok ? __ldg(P.hv + e) : 0.f;
-        nbh = ok ? __ldg(P.bairh + e) : 0u;
+        nu = ok ? load_after_wait((STORED ? P.vx : iu) + e) : 0.f;
+        nv = ok ? load_after_wait((STORED ? P.vy : iv) + e) : 0.f;
+        nh = ok ? load_after_wait(P.hv + e) : 0.f;
+        nbh = ok ? load_after_wait(P.bairh + e) : 0u;
     };
     load(y0 - 1, o);
 #pragma unroll 1
@@ -524,14 +524,14 @@ __device__ __forceinline__ void strip_heat(const StripGrids &P, const AirInst &I
         float h2 = 0.f, nx = 0.f, ny = 0.f;
         uint32_t mw = 0u, me = 0u, ma = 0u, mb = 0u;  // the mask rebuild's
         if (mine) {
-            h2 = __ldg(P.hv + w);
-            nx = __ldg((STORED ? P.vx : iu) + w);
-            ny = __ldg((STORED ? P.vy : iv) + w);
+            h2 = load_after_wait(P.hv + w);
+            nx = load_after_wait((STORED ? P.vx : iu) + w);
+            ny = load_after_wait((STORED ? P.vy : iv) + w);
             if (MASKS) {
-                mw = __ldg(P.wall + w);
+                mw = load_after_wait(P.wall + w);
                 me = P.emap[w];
-                ma = __ldg(P.eair + w);
-                mb = __ldg(P.eairh + w);
+                ma = load_after_wait(P.eair + w);
+                mb = load_after_wait(P.eairh + w);
             }
         }
         // backtrace of row h (heat.rs:105-130)
@@ -542,15 +542,15 @@ __device__ __forceinline__ void strip_heat(const StripGrids &P, const AirInst &I
         if (mine)
             far_target(xf, (float)h, svx, svy, limx, limy,
                        [&](int cx, int cy) -> bool {
-                           return (__ldg(P.bairh + (off + (uint32_t)cy * pitch + (uint32_t)cx)) & 0x8u) != 0u;
+                           return (load_after_wait(P.bairh + (off + (uint32_t)cy * pitch + (uint32_t)cx)) & 0x8u) != 0u;
                        },
                        tx, ty);
         const bool here = (hb2 & 2u) != 0u;
         const Landing q(tx, ty, 0.0f, limx + 1.0f, limy + 1.0f, off, pitch, mine && !here);
         const float *q0 = P.hv + q.g;
         const uint32_t *qb = P.bairh + q.g;
-        const float t00 = __ldg(q0), t10 = __ldg(q0 + 1), t01 = __ldg(q0 + pitch), t11 = __ldg(q0 + pitch + 1);
-        const uint32_t c00 = __ldg(qb), c10 = __ldg(qb + 1), c01 = __ldg(qb + pitch), c11 = __ldg(qb + pitch + 1);
+        const float t00 = load_after_wait(q0), t10 = load_after_wait(q0 + 1), t01 = load_after_wait(q0 + pitch), t11 = load_after_wait(q0 + pitch + 1);
+        const uint32_t c00 = load_after_wait(qb), c10 = load_after_wait(qb + 1), c01 = load_after_wait(qb + pitch), c11 = load_after_wait(qb + pitch + 1);
         // the means of row r - 1 get this row's taps, row r's begin (heat.rs:46-104)
         const uint32_t hc0 = around(row0 | C.not_inner | (r < 1 || r + 1 >= Y ? ~0u : 0u), lane);
         const Closed k0(hc0), k1(hc1);
@@ -574,9 +574,9 @@ __device__ __forceinline__ void strip_heat(const StripGrids &P, const AirInst &I
                 if (radial) convection_dir(I, C.x, h, convx, convy);
                 if (I.conv == 1u) {
                     const float weight =
-                        div_by_const((h2 - __ldg(P.hv + (w - 1u))) * convx + (h2 - __ldg(P.hv + (w - pitch))) * convy,
+                        div_by_const((h2 - load_after_wait(P.hv + (w - 1u))) * convx + (h2 - load_after_wait(P.hv + (w - pitch))) * convy,
                                      kConvLegacy, kConvLegacyRcp);
-                    if (weight > 0.0f && !(__ldg(P.bairh + (w - pitch)) & 0x8u)) {
+                    if (weight > 0.0f && !(load_after_wait(P.bairh + (w - pitch)) & 0x8u)) {
                         nx += weight * convx;
                         ny += weight * convy;
                     }
@@ -616,7 +616,7 @@ __device__ __forceinline__ void strip_masks(const StripGrids &P, const AirInst &
         const uint32_t raw = emap_seen(me, lag), next = raw != 0u ? raw - 1u : 0u;
         if (next != me) P.emap[w] = next;
         uint32_t ba, bh;
-        masks_of(__ldg(P.wall + w), raw, __ldg(P.eair + w), __ldg(P.eairh + w), ba, bh);
+        masks_of(load_after_wait(P.wall + w), raw, load_after_wait(P.eair + w), load_after_wait(P.eairh + w), ba, bh);
         P.bair_out[w] = ba;
         P.bairh_out[w] = bh;
     }

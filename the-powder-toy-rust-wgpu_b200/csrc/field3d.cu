@@ -28,6 +28,7 @@
 
 #include "field3d.hpp"
 #include "field3d_cell.cuh"
+#include "pdl.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -42,9 +43,6 @@ constexpr int PLANE = N * N;      // floats per plane
 constexpr int SLAB = PL * PLANE;  // floats per CTA slab
 constexpr size_t CLUSTER_SMEM = 3 * SLAB * sizeof(float);
 static_assert(ROWS * PL * 4 <= 32, "a thread's cells fit one 32-bit mask");
-
-__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ------------------------------------------------------------- gathers ----
 // One warp per listed brick, persistent warps taking the list in order. Lane

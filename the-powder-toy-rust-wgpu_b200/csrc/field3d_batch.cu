@@ -29,6 +29,7 @@
 // the sweeps.
 #include "field3d.hpp"
 #include "field3d_cell.cuh"
+#include "pdl.cuh"
 
 namespace tpt {
 namespace vox {
@@ -41,9 +42,6 @@ constexpr int PBLOCKS = QUADS / PBLOCK;
 // Worlds from which a sweep's thread takes two quads (see k_b_sweep).
 constexpr uint32_t MANY_WORLDS = 4;
 static_assert(TPT_VOX_GRAV_ITERATIONS % 2 == 0, "an even sweep count leaves the last sweep in grav_potential");
-
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Which field block z of a launch works on: bit f of `fields` (f = 0 air,
 // 1 gravity) marks the fields in the grid, in that order.
@@ -89,7 +87,7 @@ __device__ __forceinline__ Quad load_quad(const float *a, int i0, int y, int z) 
 
 __global__ void __launch_bounds__(PBLOCK) k_b_prep(const __grid_constant__ Batch B) {
     pdl_wait();
-    pdl_launch_dependents();
+    pdl_release();
     const BWorld &w = B.w[blockIdx.y];
     const int f = field_of(B.fields, blockIdx.z);
     const int q = blockIdx.x * PBLOCK + threadIdx.x;
@@ -181,7 +179,7 @@ __global__ void __launch_bounds__(THREADS) k_b_sweep(const __grid_constant__ Bat
     };
     if (s > 0) load_source();  // the first sweep's predecessor is the pass that writes it
     pdl_wait();
-    pdl_launch_dependents();
+    pdl_release();
     if (s == 0) load_source();
     c[0] = y0 > 0 ? ld4(S + i0 - SY) : zero4();
 #pragma unroll
@@ -226,7 +224,7 @@ __global__ void __launch_bounds__(PBLOCK) k_b_finish(const __grid_constant__ Bat
     const int i0 = 4 * (int)(blockIdx.x * PBLOCK + threadIdx.x), x0 = i0 & 63, z = (i0 >> 6) & 63, y = i0 >> 12;
     if (f == 1) {
         pdl_wait();
-        pdl_launch_dependents();
+        pdl_release();
         // gravity_force_kernel (gravity.rs:199-224) on the last sweep, then
         // gravity_clear_kernel (gravity.rs:112-118) when asked
         const Quad u = load_quad(w.pot, i0, y, z);
@@ -257,7 +255,7 @@ __global__ void __launch_bounds__(PBLOCK) k_b_finish(const __grid_constant__ Bat
         f4set(buoy, k, (lt - kAmbient) * kBuoyancy);
     }
     pdl_wait();
-    pdl_launch_dependents();
+    pdl_release();
     const Quad p = load_quad((B.air_iters & 1u) ? w.p_tmp : w.p, i0, y, z);  // the last sweep's buffer
 #pragma unroll
     for (int a = 0; a < 3; ++a) {

@@ -53,6 +53,7 @@
 #include <vector>
 
 #include "grav_dft.hpp"
+#include "pdl.cuh"
 #include "tc.cuh"
 
 namespace tpt {
@@ -157,15 +158,12 @@ __device__ __forceinline__ void split_pack32(const float (&v)[32], float sgn, ui
     }
 }
 
-// Programmatic dependent launch, used where a solve's launches are too small to
-// fill the GPU: a stage's CTAs start on idle SMs, set up their barriers and
-// TMEM and fetch their first tile's description while the stage before runs,
-// and wait here for its results. Without the launch attribute the wait returns
-// at once.
-__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // ---- the GEMM kernel ---------------------------------------------------------
+// Where a solve's launches are too small to fill the GPU they are programmatic
+// dependent launches: a stage's CTAs start on idle SMs, set up their barriers
+// and TMEM and fetch their first tile's description while the stage before
+// runs, and wait for its results. Without the launch attribute the wait returns
+// at once.
 template <int STAGE>
 __global__ void __launch_bounds__(THREADS, 1)
     dft_gemm(const Problem *__restrict__ probs, const Tile *__restrict__ tiles, uint32_t ntiles,

@@ -8,6 +8,7 @@
 #include "grav_fft.cuh"
 #include "grav_fft_mixed.cuh"
 #include "grav_plan.hpp"
+#include "pdl.cuh"
 
 namespace tpt {
 namespace gfft {
@@ -52,12 +53,10 @@ __device__ __forceinline__ const Job &stage_job(const Job *jobs, const BlockRef 
     return *reinterpret_cast<const Job *>(words);
 }
 
-// Programmatic dependent launch: the next pass's blocks are launched as this
-// one's drain, stage their job, and wait here for its results.
-__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // ---- the three passes ------------------------------------------------------------
+// Programmatic dependent launches: the next pass's blocks are launched as this
+// one's drain, stage their job, and wait for its results.
+//
 // One function per radix and step: blocks of all lengths share them.
 template <int R, bool INV> __device__ __noinline__ void row_step2(const Axis &A, uint32_t cnt) {
     step2<R, INV>(fft_smem, A, RowSeq{}, cnt);
@@ -85,10 +84,10 @@ template <int R> __device__ __noinline__ void rows_load(const Job &J, uint32_t p
 #pragma unroll
         for (int a = 0; a < R; ++a) {
             const bool in = j + m * a < X;
-            on[a] = in ? __ldg(mk + m * a) : 0u;
-            raw[a] = in ? __ldg(ms + m * a) : 0u;
-            on1[a] = in && two ? __ldg(mk1 + m * a) : 0u;
-            raw1[a] = in ? __ldg(ms1 + m * a) : 0u;
+            on[a] = in ? load_after_wait(mk + m * a) : 0u;
+            raw[a] = in ? load_after_wait(ms + m * a) : 0u;
+            on1[a] = in && two ? load_after_wait(mk1 + m * a) : 0u;
+            raw1[a] = in ? load_after_wait(ms1 + m * a) : 0u;
         }
 #pragma unroll
         for (int a = 0; a < R; ++a) {
@@ -160,7 +159,7 @@ template <int R> __device__ __noinline__ void cols_load(const Job &J, uint32_t h
         const float2 *p = work + (size_t)j * nhp + c;
         const uint32_t rows = c < left ? Y : 0u;
 #pragma unroll
-        for (int a = 0; a < R; ++a) v[a] = j + m * a < rows ? __ldg(p + a * stride) : make_float2(0.0f, 0.0f);
+        for (int a = 0; a < R; ++a) v[a] = j + m * a < rows ? load_after_wait(p + a * stride) : make_float2(0.0f, 0.0f);
     });
 }
 // Step 3, the two products and the inverses' first step. The spectrum of a
@@ -253,7 +252,7 @@ template <int R> __device__ __noinline__ void rows_first(const Job &J, uint32_t 
 #pragma unroll
         for (int i = 0; i < R; ++i) {
             const bool direct = R % 2 == 1 && i == R / 2 ? 2u * (q + A.q * i) <= A.n : i < (R + 1) / 2;
-            w[i] = __ldg(direct ? lo + A.q * i : hi - A.q * i);
+            w[i] = load_after_wait(direct ? lo + A.q * i : hi - A.q * i);
             if (!direct) w[i].y = -w[i].y;
         }
         unstep3<R>(o, 1, t, w);
@@ -269,7 +268,7 @@ template <int R> __device__ __noinline__ void rows_store(const Job &J, uint32_t 
         float *px = gx + r, *py = gy + r;
         uint32_t on[R];
 #pragma unroll
-        for (int a = 0; a < R; ++a) on[a] = j + m * a < X ? __ldg(mk + m * a) : 0u;
+        for (int a = 0; a < R; ++a) on[a] = j + m * a < X ? load_after_wait(mk + m * a) : 0u;
 #pragma unroll
         for (int a = 0; a < R; ++a)
             if (j + m * a < X) {

@@ -13,6 +13,7 @@
 // positions and element state, never the velocity the force writes), and the
 // override joins the snapshot copy: three launches plus the solve.
 #include "grav_particles.hpp"
+#include "pdl.cuh"
 
 namespace tpt {
 namespace gp {
@@ -45,8 +46,6 @@ __device__ __forceinline__ float clampf(float v, float lo, float hi) {
 
 // The kernels of a gravity tick are programmatic dependent launches: each waits
 // for the one before it to complete before it touches memory.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... Args>
 int launch_pdl(void (*kernel)(Args...), uint32_t blocks, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
@@ -103,7 +102,8 @@ __global__ void k_particles(GravGrids G, Parts P) {
         if (eligible) {
             cell = ((uint32_t)yi / CELL) * G.xcells + (uint32_t)xi / CELL;
             // unpowered stasis wall freezes the particle
-            if (__ldg(G.wall + cell) == WL_STASIS && (__ldg(G.emap + cell) & 0xFFu) < 8u) eligible = false;
+            if (load_after_wait(G.wall + cell) == WL_STASIS && (load_after_wait(G.emap + cell) & 0xFFu) < 8u)
+                eligible = false;
         }
         if (eligible) {
             const uint32_t *rec = P.lut + (size_t)ty * LUT_WORDS;
@@ -115,8 +115,8 @@ __global__ void k_particles(GravGrids G, Parts P) {
                 vy *= loss;
             }
             if ((props & TYPE_SOLID) == 0u) {
-                vx += G.newton * __ldg(G.gx + cell);
-                vy += G.newton * __ldg(G.gy + cell);
+                vx += G.newton * load_after_wait(G.gx + cell);
+                vy += G.newton * load_after_wait(G.gy + cell);
             }
             P.vx[i] = vx;
             P.vy[i] = vy;
@@ -158,7 +158,7 @@ __global__ void k_particles(GravGrids G, Parts P) {
         const uint32_t cx = (uint32_t)xi / CELL, cy = (uint32_t)yi / CELL;
         if (cx < G.xcells && cy < G.ycells) {
             const uint32_t cell = cy * G.xcells + cx;
-            if (__ldg(G.mask + cell) != 0u) {
+            if (load_after_wait(G.mask + cell) != 0u) {
                 const int32_t q = to_fixed(mass);
                 if (q != 0) atomicAdd(G.mass + cell, q);
             }
