@@ -518,7 +518,8 @@ typedef struct tpt_vox_plan tpt_vox_plan;
  * its kernel. The plan owns the forms' scratch (the reference's velocity
  * snapshot, air.rs:78-79, and the batched form's per-world source fields,
  * about 5 MiB per world for 16 worlds) and the gravity gather's table of
- * per-brick list counts (128 KiB); no entry point below allocates.
+ * per-brick list counts (128 KiB), which is zero between calls and carries
+ * over from one gather to the next; no entry point below allocates.
  */
 int tpt_vox_plan_create(int form, tpt_vox_plan **out);
 int tpt_vox_plan_destroy(tpt_vox_plan *plan);

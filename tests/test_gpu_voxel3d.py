@@ -130,6 +130,32 @@ def test_grav_gather_list_lengths(cuda, oracle, plans, world, n):
     _same(V.download(bufs, air), d, ("grav_mass",))
 
 
+def test_gravity_gathers_of_two_worlds_in_turn(cuda, oracle, plans, world):
+    """Two worlds share a plan's table of counts, with list lengths on both
+    sides of the half that the gather's two forms part at, one call behind the
+    other: no call leaves counts to the next."""
+    import voxel3d as V
+    import workloads as W
+
+    rng = np.random.default_rng(23)
+    half = W.VOX_BRICKS // 2
+    hosts = [_copy(world), _copy(world)]
+    hosts[1]["voxel"] = np.roll(hosts[1]["voxel"], 8 * 4097)
+    devs = [V.upload(d) for d in hosts]
+    lengths = [W.VOX_BRICKS, half, 0, half + 1, 1, half + 1, half, W.VOX_BRICKS]
+    lists = [rng.integers(0, W.VOX_BRICKS, W.VOX_BRICKS).astype(np.uint32) for _ in lengths]
+    on_device = [cuda.from_numpy(a.view(np.int32)).cuda() for a in lists]
+    for k, n in enumerate(lengths):
+        d, (bufs, _) = hosts[k % 2], devs[k % 2]
+        d["sim_list"], d["sim_count"] = lists[k], np.array([n, 1, 1], np.uint32)
+        bufs.sim_list.copy_(on_device[k])
+        bufs.sim_count.copy_(cuda.tensor([n, 1, 1], dtype=cuda.int32))
+        V.gravity_gather(plans["batched"], bufs)
+        oracle.vox_grav_gather(d)
+    for d, (bufs, air) in zip(hosts, devs):
+        _same(V.download(bufs, air), d, ("grav_mass",))
+
+
 @pytest.mark.parametrize("form", sorted(FORMS))
 @pytest.mark.parametrize("iterations", [0, 1, 2, 3, 12])
 def test_air_solve(cuda, oracle, plans, world, form, iterations):

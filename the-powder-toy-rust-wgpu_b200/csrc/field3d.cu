@@ -201,10 +201,12 @@ __device__ __forceinline__ void gather_brick(const uint32_t *__restrict__ voxel,
 //                      per listed brick;
 //   above              it counts how often each brick is listed, and
 //                      k_grav_gather_rows, launched behind it in any case,
-//                      takes the bricks in memory order: a block owns a row
-//                      of 32 bricks along x and its warps the row's listed
-//                      ones in turn, and it clears the row's counts for the
-//                      next call.
+//                      takes the counted bricks in memory order: a block owns
+//                      a row of 32 bricks along x and its warps the row's
+//                      counted ones in turn, and it clears the row's counts
+//                      for the next call. It goes by the counts alone and
+//                      takes every one it finds, so that none can stay
+//                      whatever becomes of the list's length meanwhile.
 //
 // Measured on B200, us per world over eight worlds in turn (1 GB of voxels and
 // aux_tmp), both launches, list against rows: 30% of the bricks listed 22.5 /
@@ -235,12 +237,10 @@ __global__ void __launch_bounds__(GATHER_WARPS * 32) k_grav_gather_list(
 }
 
 __global__ void __launch_bounds__(GATHER_WARPS * 32) k_grav_gather_rows(
-    const uint32_t *__restrict__ voxel, const int32_t *__restrict__ aux, const uint32_t *__restrict__ count,
-    uint32_t *mult, int32_t *__restrict__ mass) {
+    const uint32_t *__restrict__ voxel, const int32_t *__restrict__ aux, uint32_t *mult, int32_t *__restrict__ mass) {
     __shared__ uint2 queue[GATHER_WARPS][512];
     __shared__ uint32_t part[GATHER_WARPS][32];
     pdl_wait();
-    if (__ldg(count) <= LIST_BRICKS) return;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t bbase = blockIdx.x << 5;
     part[warp][lane] = 0u;
@@ -756,8 +756,7 @@ int launch_grav_gather(const World &w, uint32_t *brick_mult, cudaStream_t st) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, k_grav_gather_rows, (const uint32_t *)w.voxel,
-                                             (const int32_t *)w.aux_tmp, (const uint32_t *)w.sim_count, brick_mult,
-                                             w.grav_mass);
+                                             (const int32_t *)w.aux_tmp, brick_mult, w.grav_mass);
     if (e != cudaSuccess) {
         // the counts must not stay for the next call
         cudaMemsetAsync(brick_mult, 0, TPT_VOX_BRICKS * sizeof(uint32_t), st);
