@@ -383,6 +383,27 @@ def test_batch_whole_field_io_then_step(cuda, tf, oracle):
     b.close()
 
 
+@pytest.mark.parametrize("form", [0, 1])
+def test_refused_tuning_leaves_the_batch_as_it_was(cuda, tf, oracle, form):
+    """A tuning that is refused for its last field after an earlier one asked
+    for another shape: the graphs that were captured before it still have
+    their work lists, and the batch steps on."""
+    insts = mixed_instances()
+    b = tf.Batch(insts)
+    set_form(tf, b, form)
+    b.step(3)
+    before = b.tuning_dict()
+    with pytest.raises(tf.TptError, match="ctas_per_sm"):
+        set_form(tf, b, tf.AIR_FORM_SWEEP, tile_x=256, tile_y=32, ctas_per_sm=32)
+    with pytest.raises(tf.TptError, match="grav_side_ctas"):
+        set_form(tf, b, tf.AIR_FORM_TILES, tile_x=64, tile_y=16, grav_side_ctas=10000)
+    assert b.tuning_dict() == before
+    b.step(3)
+    cuda.cuda.synchronize()
+    check_against_oracle(tf, oracle, b, insts, 6, f"form {form}")
+    b.close()
+
+
 @pytest.mark.parametrize("queue,ticks", [(1, 3), (0, 2)])
 def test_large_batch_strips_match_oracle(cuda, tf, oracle, queue, ticks):
     """A batch large enough for the warp strips (2 million cells): grids one

@@ -934,13 +934,22 @@ int tpt_batch_set_tuning(tpt_batch *b, const tpt_batch_tuning *t) {
     const bool split = b->any_grav && b->precision == TPT_PRECISION_SPLIT_BF16 && b->dft.can_split();
     if (t->grav_side_ctas && !split)
         TPT_FAIL(TPT_ERR_INVALID_ARG, "grav_side_ctas must be 0: the batch's gravity has one kind of y stage");
+    if (split && t->grav_side_ctas > b->dft.max_side_ctas())
+        TPT_FAIL(TPT_ERR_INVALID_ARG, "grav_side_ctas %u above %u", t->grav_side_ctas, b->dft.max_side_ctas());
+    if (sweep) {
+        int fit = 0;
+        int rc = air::sweep_max_ctas_per_sm(t->tile_x, &fit);
+        if (rc) return rc;
+        if (t->ctas_per_sm > (uint32_t)fit)
+            TPT_FAIL(TPT_ERR_INVALID_ARG, "ctas_per_sm %u exceeds the %d sweep CTAs of %u lanes that fit an SM",
+                     t->ctas_per_sm, fit, t->tile_x);
+    }
+    // The arguments are good. The graphs go before the lists that they name.
+    b->drop_graphs();
     if (sweep && (t->tile_x != b->sweep_lanes || t->tile_y != b->sweep_rows)) {
         int rc = set_sweep_shape(b, t->tile_x, t->tile_y);
         if (rc) return rc;
     }
-    if (sweep && t->ctas_per_sm > (uint32_t)b->sweep_occupancy)
-        TPT_FAIL(TPT_ERR_INVALID_ARG, "ctas_per_sm %u exceeds the %d sweep CTAs of %u lanes that fit an SM",
-                 t->ctas_per_sm, b->sweep_occupancy, t->tile_x);
     if (!sweep && sh != b->shape) {
         int rc = set_tile_shape(b, sh);
         if (rc) return rc;
@@ -953,7 +962,6 @@ int tpt_batch_set_tuning(tpt_batch *b, const tpt_batch_tuning *t) {
         int rc = b->dft.set_side_ctas(t->grav_side_ctas);
         if (rc) return rc;
     }
-    b->drop_graphs();
     b->tuning = *t;
     return TPT_OK;
 }
