@@ -420,9 +420,9 @@ int tpt_batch_step(tpt_batch *batch, uint32_t ticks, tpt_stream_t stream);
  * for batches with gravity, the whole step (air and gravity together) for
  * the best few air settings and every gravity branch split. The choice is cached in
  * the process per batch composition -- the instances' (xcells, ycells)
- * buckets (powers of two) with their counts, and the gravity precision -- so
- * tuning a batch of the same composition again only applies the cached
- * settings. Synchronous. */
+ * buckets (powers of two) with their counts, the gravity precision, and
+ * whether the tile form runs strips -- so tuning a batch of the same
+ * composition again only applies the cached settings. Synchronous. */
 int tpt_batch_tune(tpt_batch *batch, tpt_stream_t stream);
 int tpt_batch_get_tuning(const tpt_batch *batch, tpt_batch_tuning *out);
 int tpt_batch_set_tuning(tpt_batch *batch, const tpt_batch_tuning *tuning);

@@ -383,6 +383,24 @@ def test_batch_whole_field_io_then_step(cuda, tf, oracle):
     b.close()
 
 
+def test_tiles_and_strips_are_tuned_separately(cuda, tf):
+    """Two batches whose grids fall in the same size buckets, on either side
+    of 2 million cells (tiles and strips): the second is timed, not given the
+    first one's settings."""
+    import workloads as W
+
+    launches = []
+    for side in (300, 500):
+        inst = W.make_instance(side, side, side, config=W.AirConfig(newton_grav=0))
+        b = tf.Batch([inst] * 12)
+        assert (b.total_cells >= 2000000) == (side == 500)
+        n0 = tf.launch_count()
+        b.tune()
+        launches.append(tf.launch_count() - n0)
+        b.close()
+    assert launches[0] > 0 and launches[1] > 0
+
+
 @pytest.mark.parametrize("form", [0, 1])
 def test_refused_tuning_leaves_the_batch_as_it_was(cuda, tf, oracle, form):
     """A tuning that is refused for its last field after an earlier one asked

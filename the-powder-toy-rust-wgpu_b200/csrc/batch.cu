@@ -27,6 +27,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <vector>
 
 #include "air_launch.hpp"
@@ -1009,14 +1010,17 @@ int tpt_batch_profile_phases(tpt_batch *b, uint32_t ticks, tpt_stream_t stream, 
 }
 
 // Tuned settings per batch composition: the shapes' (W, H) buckets
-// (powers of two) with their counts, and the gravity precision. A batch whose
+// (powers of two) with their counts, the gravity precision, and whether the
+// tile form runs strips (the settings that are fast for tiles need not be: two
+// CTAs of a 64x16 tile fill an SM, two of four strips do not). A batch whose
 // instances fall in the same buckets reuses the tuned settings without
 // timing.
 struct TuneKey {
     int precision;
+    bool strips;
     std::vector<std::pair<uint32_t, uint32_t>> buckets;  // (log2 W << 8 | log2 H, count), sorted
     bool operator<(const TuneKey &o) const {
-        return precision != o.precision ? precision < o.precision : buckets < o.buckets;
+        return std::tie(precision, strips, buckets) < std::tie(o.precision, o.strips, o.buckets);
     }
 };
 static std::mutex g_tune_mu;
@@ -1033,6 +1037,7 @@ static TuneKey tune_key(const tpt_batch *b) {
     for (const auto &d : b->descs) ++h[log2_bucket(d.air.xcells) << 8 | log2_bucket(d.air.ycells)];
     TuneKey k;
     k.precision = b->any_grav ? b->precision : -1;
+    k.strips = b->use_strips;
     k.buckets.assign(h.begin(), h.end());
     return k;
 }
