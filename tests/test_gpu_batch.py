@@ -401,6 +401,21 @@ def test_tiles_and_strips_are_tuned_separately(cuda, tf):
     assert launches[0] > 0 and launches[1] > 0
 
 
+def test_tuning_times_each_strip_layout_once(cuda, tf):
+    """At 2.2 million cells every tile shape stands for the same strips, and no
+    temporal depth is tried: 8 settings of the strips (CTAs per SM and queue)
+    and 3 of the sweep, 2 x 20 ticks each of 3 and 2 launches."""
+    import workloads as W
+
+    inst = W.make_instance(400, 225, 1, config=W.AirConfig(newton_grav=0))
+    b = tf.Batch([inst] * 24)
+    n0 = tf.launch_count()
+    b.tune()
+    assert 0 < tf.launch_count() - n0 <= 8 * 40 * 3 + 3 * 40 * 2
+    assert b.tuning().temporal_depth == 1
+    b.close()
+
+
 @pytest.mark.parametrize("form", [0, 1])
 def test_refused_tuning_leaves_the_batch_as_it_was(cuda, tf, oracle, form):
     """A tuning that is refused for its last field after an earlier one asked

@@ -98,9 +98,10 @@ constexpr int TILE_SHAPES = 4;
 // The offered shapes, 32x8 first; tile_shape(tx, ty) is null for any other.
 const TileShape *const *tile_shapes();
 const TileShape *tile_shape(uint32_t tx, uint32_t ty);
-// Appends a pass's strips of every instance (X, Y): about `rows` rows each,
-// `resident` warps working on them.
-void plan_strips(int pass, const std::vector<std::pair<uint32_t, uint32_t>> &grids, uint32_t rows, uint32_t resident,
+// The rows per strip of a pass over instances (X, Y) for a shape's rows and
+// `resident` warps, and the strips of about that many rows, appended.
+uint32_t strip_rows(int pass, const std::vector<std::pair<uint32_t, uint32_t>> &grids, uint32_t rows, uint32_t resident);
+void plan_strips(int pass, const std::vector<std::pair<uint32_t, uint32_t>> &grids, uint32_t rows,
                  std::vector<StripRef> &out);
 // resident CTAs per SM, per pass
 int strip_occupancy(int occupancy[STRIP_PASSES]);

@@ -115,19 +115,31 @@ int read_errors(uint32_t *out) {  // the strips and the sweep form have no waits
     return TPT_OK;
 }
 
-// Rows per strip. A strip of h rows takes h + 3 to h + 6 steps, so tall strips
-// spend the least on their halo, but a launch's last strips must be short for
-// its warps to end together: the first half of the cells is cut into strips of
-// twice the shape's rows, the last quarter into half its rows. Where that makes
-// fewer than three strips per resident warp, shorter ones throughout, down to
-// 4 rows (a small batch is bound by how long one warp walks).
-void plan_strips(int pass, const std::vector<std::pair<uint32_t, uint32_t>> &grids, uint32_t rows, uint32_t resident,
+// Rows of all strips across the grids.
+static uint64_t strip_rows_total(const std::vector<std::pair<uint32_t, uint32_t>> &grids, uint32_t w) {
+    uint64_t total = 0;
+    for (const auto &g : grids) total += (uint64_t)((g.first + w - 1) / w) * g.second;
+    return total;
+}
+
+// Rows per strip: the shape's, or what makes three strips per resident warp
+// where that is less, down to 4 (a small batch is bound by how long one warp
+// walks).
+uint32_t strip_rows(int pass, const std::vector<std::pair<uint32_t, uint32_t>> &grids, uint32_t rows,
+                    uint32_t resident) {
+    const uint64_t fit = strip_rows_total(grids, (uint32_t)strip_width(pass)) / (3ull * std::max<uint32_t>(resident, 1u));
+    return std::max<uint32_t>(4u, (uint32_t)std::min<uint64_t>(fit, rows));
+}
+
+// A strip of h rows takes h + 3 to h + 6 steps, so tall strips spend the least
+// on their halo, but a launch's last strips must be short for its warps to end
+// together: the first half of the cells is cut into strips of twice `rows`, the
+// last quarter into half of them.
+void plan_strips(int pass, const std::vector<std::pair<uint32_t, uint32_t>> &grids, uint32_t rows,
                  std::vector<StripRef> &out) {
     const uint32_t w = (uint32_t)strip_width(pass);
-    uint64_t total = 0, done = 0;
-    for (const auto &g : grids) total += (uint64_t)((g.first + w - 1) / w) * g.second;
-    const uint64_t fit = total / (3ull * std::max<uint32_t>(resident, 1u));
-    rows = std::max<uint32_t>(4u, std::min<uint32_t>(rows, (uint32_t)std::min<uint64_t>(fit, rows)));
+    const uint64_t total = strip_rows_total(grids, w);
+    uint64_t done = 0;
     for (uint32_t i = 0; i < (uint32_t)grids.size(); ++i) {
         const uint32_t X = grids[i].first, Y = grids[i].second;
         const uint32_t h = 2 * done < total ? 2 * rows : 4 * done < 3 * total ? rows : std::max<uint32_t>(4u, rows / 2);

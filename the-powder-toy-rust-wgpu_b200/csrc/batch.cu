@@ -25,8 +25,10 @@
 #include <string.h>
 
 #include <algorithm>
+#include <array>
 #include <map>
 #include <mutex>
+#include <set>
 #include <tuple>
 #include <vector>
 
@@ -528,6 +530,21 @@ static int upload_tile_maps(const std::vector<CUtensorMap> &tm, const std::vecto
     return TPT_OK;
 }
 
+// The rows of a shape's strips, per pass: shapes of equal rows have the same
+// strips.
+static int shape_strip_rows(const tpt_batch *b, const air::TileShape *sh, std::array<uint32_t, air::STRIP_PASSES> &rows,
+                            int occ[air::STRIP_PASSES], std::vector<std::pair<uint32_t, uint32_t>> &grids) {
+    int rc = air::strip_occupancy(occ);
+    if (rc) return rc;
+    grids.clear();
+    for (const auto &d : b->descs) grids.push_back({d.air.xcells, d.air.ycells});
+    for (int k = 0; k < air::STRIP_PASSES; ++k) {
+        if (occ[k] < 1) TPT_FAIL(TPT_ERR_UNSUPPORTED, "strip pass %d does not fit an SM", k);
+        rows[k] = air::strip_rows(k, grids, sh->strip_rows, (uint32_t)(b->sms * occ[k] * air::STRIP_WARPS));
+    }
+    return TPT_OK;
+}
+
 // Plans the tile form for shape `sh` and uploads it: the tile list and the
 // tensor maps (boxes of the tile plus a 4-cell x and 3-cell y halo), or the
 // strips.
@@ -551,16 +568,15 @@ static int set_tile_shape(tpt_batch *b, const air::TileShape *sh) {
         return TPT_OK;
     }
     int occ[air::STRIP_PASSES] = {};
-    int rc = air::strip_occupancy(occ);
+    std::array<uint32_t, air::STRIP_PASSES> rows;
+    std::vector<std::pair<uint32_t, uint32_t>> grids;
+    int rc = shape_strip_rows(b, sh, rows, occ, grids);
     if (rc) return rc;
     std::vector<air::StripRef> list;
     uint32_t count[air::STRIP_PASSES];
-    std::vector<std::pair<uint32_t, uint32_t>> grids;
-    for (const auto &d : b->descs) grids.push_back({d.air.xcells, d.air.ycells});
     for (int k = 0; k < air::STRIP_PASSES; ++k) {
-        if (occ[k] < 1) TPT_FAIL(TPT_ERR_UNSUPPORTED, "the %ux%u tile kernels do not fit an SM", sh->tx, sh->ty);
         const size_t before = list.size();
-        air::plan_strips(k, grids, sh->strip_rows, (uint32_t)(b->sms * occ[k] * air::STRIP_WARPS), list);
+        air::plan_strips(k, grids, rows[k], list);
         count[k] = (uint32_t)(list.size() - before);
     }
     air::StripRef *d = nullptr;
@@ -1064,8 +1080,17 @@ int tpt_batch_tune(tpt_batch *b, tpt_stream_t stream) {
         uint32_t form, x, y, per_sm, queue;
     };
     std::vector<Cand> cands;
+    std::set<std::array<uint32_t, air::STRIP_PASSES>> seen;
     for (int k = 0; k < air::TILE_SHAPES; ++k) {
         const air::TileShape *sh = air::tile_shapes()[k];
+        if (b->use_strips) {  // a shape whose strips are an earlier one's is that candidate
+            int occ[air::STRIP_PASSES] = {};
+            std::array<uint32_t, air::STRIP_PASSES> rows;
+            std::vector<std::pair<uint32_t, uint32_t>> grids;
+            const int rrc = shape_strip_rows(b, sh, rows, occ, grids);
+            if (rrc) return rrc;
+            if (!seen.insert(rows).second) continue;
+        }
         const bool base = sh->tx == DEFAULT_TILE_X && sh->ty == DEFAULT_TILE_Y;
         for (uint32_t q : {1u, 0u})
             for (uint32_t c : base ? std::vector<uint32_t>{0u, 4u, 6u, 8u} : std::vector<uint32_t>{0u, 2u})
@@ -1108,8 +1133,12 @@ int tpt_batch_tune(tpt_batch *b, tpt_stream_t stream) {
     }
     // Phase 1b, for the tile form at the chosen layout, on the same 20 ticks:
     // the temporal depth (ticks per block of fused B(t) + A(t + 1) launches).
+    // Not as strips: there a block's middle launches are tiles, and every
+    // depth is slower (air us per tick at depths 1, 2, 4, 10 and 20: 2.2 M
+    // cells in 24 grids 179, 205, 216, 224, 226; 6.1 M in 128 414, 540, 602, 641,
+    // 653; 8.1 M in 256 549, 750, 850, 911, 931).
     for (uint32_t depth : {2u, 4u, 10u, 20u}) {
-        if (rc || best.air_form != TPT_AIR_FORM_TILES) break;
+        if (rc || best.air_form != TPT_AIR_FORM_TILES || b->use_strips) break;
         tpt_batch_tuning t = best;
         t.temporal_depth = depth;
         rc = tpt_batch_set_tuning(b, &t);
