@@ -347,9 +347,10 @@ enum {
     /* Two launches per tick over tiles (32x8, 64x8, 32x16 or 64x16 cells),
      * halos staged by TMA: pass A (pressure, velocity) writes opv/ovx/ovy,
      * pass B (smoothing, advection, vorticity, fans, heat, convection, masks)
-     * reads them. A batch of 2 million cells or more runs the same passes as
-     * strips, one per warp, of 26 to 30 columns and a number of rows that goes
-     * with the tile shape (24, 32, 16 and 40 on average), B as two launches. */
+     * reads them. A batch of 2 million cells or more (6 million where nearly
+     * all grids are 31 or 32 cells wide) runs the same passes as strips, one
+     * per warp, of 26 to 30 columns and a number of rows that goes with the
+     * tile shape (24, 32, 16 and 40 on average), B as two launches. */
     TPT_AIR_FORM_TILES = 0,
     /* One fused launch per tick: CTAs sweep down column strips with every
      * stage pipelined over the rows (no intermediate grid in memory), plus a
@@ -433,10 +434,10 @@ typedef struct tpt_batch_profile {
     float grav_ms;             /* `ticks` gravity solves alone             */
     uint32_t ticks;
     /* Air launches per tick without temporal blocking: 2, or 3 in the tile
-     * form of a batch of 2 million cells or more (one more in the tile form
-     * with a NoUpdate + heat instance: its settle). At temporal depth k, a
-     * block of n <= k ticks makes n - 1 launches more than one tick (plus the
-     * n settles). */
+     * form of a batch that runs strips (one more in the tile form with a
+     * NoUpdate + heat instance: its settle). At temporal depth k, a block of
+     * n <= k ticks makes n - 1 launches more than one tick (plus the n
+     * settles). */
     uint32_t air_launches_per_tick;
     uint32_t grav_launches_per_tick;
     uint64_t cells;            /* sum of xcells*ycells over instances      */

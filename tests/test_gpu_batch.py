@@ -416,6 +416,20 @@ def test_tuning_times_each_strip_layout_once(cuda, tf):
     b.close()
 
 
+@pytest.mark.parametrize("side,n,launches", [((32, 256), 245, 2), ((31, 256), 253, 2), ((32, 256), 733, 3),
+                                             ((30, 256), 261, 3), ((33, 256), 237, 3), ((64, 256), 123, 3),
+                                             ((64, 256), 122, 2)])
+def test_which_batches_run_strips(cuda, tf, side, n, launches):
+    """Strips (three launches a tick) from 2 million cells, and from 6 million
+    where every grid is one tile wide but two strips."""
+    import workloads as W
+
+    inst = W.make_instance(*side, 3, config=W.AirConfig(newton_grav=0))
+    b = tf.Batch([inst] * n)
+    assert b.profile_phases(2).air_launches_per_tick == launches
+    b.close()
+
+
 @pytest.mark.parametrize("form", [0, 1])
 def test_refused_tuning_leaves_the_batch_as_it_was(cuda, tf, oracle, form):
     """A tuning that is refused for its last field after an earlier one asked

@@ -84,9 +84,32 @@ constexpr uint32_t DEFAULT_TILE_X = 32, DEFAULT_TILE_Y = 8;
 // tick, fewer instructions per cell) instead of tiles (two launches, every cell
 // a thread). Measured on B200 with FP32 gravity beside, us per tick, tiles and
 // strips: 0.55 M cells 77.6 and 82.2, 1.15 M 142.6 and 146.7, 1.81 M 238 and
-// 222 (but 33 first ticks of 1.68 M 280 and 283, the walks long), 2.26 M 263 and 241, 3.9 M 500 and 442, 6.1 M 677 and 596, 8.1 M 1003 and
-// 861 (air alone 613 and 454).
+// 222 (33 first ticks of 1.68 M, whose walks are long, 280 and 283), 2.26 M 263
+// and 241, 3.9 M 500 and 442, 6.1 M 677 and 596, 8.1 M 1003 and 861 (air alone
+// 613 and 454).
+//
+// Grids of 31 or 32 cells are one tile wide but two strips, the second nearly
+// empty: such a batch, of nearly twice as many rows of strips as rows of
+// tiles, runs strips from three times the cells. Air alone, tiles and strips:
+// 32x32 2.0 M 246 and 250, 3.0 M 351 and 346, 6.0 M 669 and 636; 32x512 2.0 M
+// 216 and 241, 4.0 M 399 and 416, 6.0 M 583 and 574; 32x2048 2.0 M 194 and 242,
+// 6.0 M 515 and 532. Widths with fewer idle lanes keep the line: 30x512 2.0 M
+// 230 and 215, 60x512 214 and 195, 64x64 236 and 216, 64x512 204 and 203 (but
+// 64x2048 186 and 206), 96x512 185 and 173, 400x225 173 and 167.
 constexpr size_t STRIP_MIN_CELLS = 2000000;
+static bool runs_strips(uint32_t n, const tpt_instance_desc *descs) {
+    uint64_t cells = 0, strip_rows = 0, tile_rows = 0;
+    for (uint32_t i = 0; i < n; ++i) {
+        const uint32_t X = descs[i].air.xcells, Y = descs[i].air.ycells;
+        cells += (uint64_t)X * Y;
+        for (int k = 0; k < air::STRIP_PASSES; ++k) {
+            const uint32_t w = (uint32_t)air::strip_width(k);
+            strip_rows += (uint64_t)((X + w - 1) / w) * Y;
+            tile_rows += (uint64_t)((X + DEFAULT_TILE_X - 1) / DEFAULT_TILE_X) * Y;
+        }
+    }
+    return cells >= (10 * strip_rows < 18 * tile_rows ? 1 : 3) * STRIP_MIN_CELLS;
+}
 
 // Splits every instance into column strips of at most lanes - 2 * SW_H
 // columns and row strips of about `rows` rows (sizes balanced within an
@@ -179,7 +202,7 @@ struct tpt_batch {
     uint32_t nform_tiles = 0;
     CUtensorMap *tmaps = nullptr;
     int tile_occupancy_a = 1, tile_occupancy_b = 1;
-    // a large one: its strips and their passes' resident CTAs per SM
+    // a large one (runs_strips): its strips and their passes' resident CTAs per SM
     bool use_strips = false;
     air::StripRef *strips = nullptr;  // the passes' lists one after the other
     uint32_t nstrips[air::STRIP_PASSES] = {};
@@ -748,9 +771,7 @@ int tpt_batch_create(uint32_t n, const tpt_instance_desc *descs, int precision, 
         return bail(TPT_ERR_CUDA);
     }
     b->want = b->ctl + 1;
-    size_t cells = 0;
-    for (uint32_t i = 0; i < n; ++i) cells += (size_t)descs[i].air.xcells * descs[i].air.ycells;
-    b->use_strips = cells >= STRIP_MIN_CELLS;
+    b->use_strips = runs_strips(n, descs);
     rc = set_tile_shape(b, air::tile_shape(DEFAULT_TILE_X, DEFAULT_TILE_Y));
     if (rc) return bail(rc);
     rc = set_sweep_shape(b, DEFAULT_LANES, DEFAULT_ROWS);
