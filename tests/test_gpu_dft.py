@@ -285,3 +285,26 @@ def test_split_bf16_y_slots(cuda, tf, oracle, X, Y):
             emax, el2 = errors(got.cpu().numpy(), d)
             assert emax <= TOL and el2 <= TOL, (emax, el2)
     s.close()
+
+
+@pytest.mark.parametrize("X,Y,n,launches", [(64, 64, 7, 5), (64, 64, 8, 4), (160, 160, 12, 4), (400, 225, 12, 4),
+                                            (256, 256, 9, 4), (40, 257, 9, 5)])
+def test_split_bf16_groups_take_the_toeplitz_stage(cuda, tf, oracle, X, Y, n, launches):
+    """From 8 grids of one shape of up to 256 rows the y stage is the one
+    Toeplitz launch (prep, R, T, R^-1) instead of the y DFT's two; the FP64
+    bars on the group's first and last grid."""
+    import workloads as W
+
+    insts = [W.make_instance(X, Y, 50 + i, mass_density=0.03) for i in range(n)]
+    b = tf.Batch(insts, precision=tf.PRECISION_SPLIT_BF16)
+    assert b.profile_phases(2).grav_launches_per_tick == launches
+    b.step(1)
+    cuda.cuda.synchronize()
+    check_clean(tf)
+    for i in (0, n - 1):
+        got = b.state(i)
+        dx, dy = oracle.grav_solve(X, Y, insts[i].gmask, mass_fx=insts[i].mass_fx, dtype=np.float64)
+        for k, d in (("gx", dx), ("gy", dy)):
+            emax, el2 = errors(got[k], d)
+            assert emax <= TOL and el2 <= TOL, (i, k, emax, el2)
+    b.close()

@@ -949,7 +949,16 @@ static int init_attrs() {
     return TPT_OK;
 }
 
-// Smallest group that takes the Toeplitz y stage by default.
+// Smallest group that takes the Toeplitz y stage by default (where Y fits its
+// tile). T is one launch that reads and writes the spectra once, the y DFT two
+// that pass twice the planes on, so from 8 instances T is the faster one
+// whatever the products: measured on B200, us per solve of DFT and T, at 8
+// instances 64x64 30.4 and 19.2, 160x160 51.6 and 32.7, 256x256 66.8 and 56.4,
+// 1000x100 112 and 106, 1500x250 342 and 308 (each at its best tile width); at
+// 12 400x225 142 and 103; at 16 256x256 111 and 75, 512x256 182 and 140; at 24
+// 2048x33 268 and 212. A rule on the executed products, of which T has up to
+// 1.9 times as many there, had chosen the DFT in all of these. Below 8 T's M
+// tile of 2G instance rows is mostly padding.
 constexpr uint32_t kToeMinGroup = 8;
 enum YMode { YMODE_AUTO = 0, YMODE_DFT = 1, YMODE_TOEPLITZ = 2 };
 
@@ -1099,16 +1108,12 @@ int DftSet::create(const std::vector<JobShape> &shapes) {
         const double fT = 2.0 * 2 * g.N1h * tiles_of(2 * g.G, MT) * g.nTy * g.kpC * 3;
         const double fRiT = 2.0 * 2 * tiles_of(g.G * g.Yp, MT) * tiles_of(g.X, g.wRI) * 2 * g.kpRi * 3;
         // Form of the y stage: Toeplitz when the group has at least
-        // kToeMinGroup instances (below that, T's M tile of 2G instance rows
-        // is mostly padding, and a lone instance's y DFT pair is cheaper:
-        // measured on B200 with single-instance groups of 32..512 cells), Y
-        // fits one T tile, and T executes fewer tensor flops than the y DFT pair.
+        // kToeMinGroup instances and Y fits one T tile.
         const bool toe_ok = g.Y <= (uint32_t)T_NMAX;
-        const bool toe_cheaper = g.G >= kToeMinGroup && fT + fRiT < fC + fCi + fRi;
         g.toe = !toe_ok                   ? 0u
                 : ymode == YMODE_TOEPLITZ ? (g.G >= toe_min_group ? 1u : 0u)
                 : ymode == YMODE_DFT      ? 0u
-                                          : (toe_cheaper ? 1u : 0u);
+                                          : (g.G >= kToeMinGroup ? 1u : 0u);
         if ((rc = I->alloc(&g.aR, (size_t)2 * g.rowsR * g.kpR))) return rc;
         if ((rc = I->alloc(&H.f1, (size_t)4 * g.N1h * H.kpF1))) return rc;
         if ((rc = I->alloc(&H.g1, (size_t)4 * g.X * H.kpG1))) return rc;
