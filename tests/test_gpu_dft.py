@@ -308,3 +308,48 @@ def test_split_bf16_groups_take_the_toeplitz_stage(cuda, tf, oracle, X, Y, n, la
             emax, el2 = errors(got[k], d)
             assert emax <= TOL and el2 <= TOL, (i, k, emax, el2)
     b.close()
+
+
+def executed_flops(X, Y, n, w, wy, toeplitz):
+    """The split-BF16 solve's tensor products for n grids of X x Y at N tiles of
+    w (R, R^-1) and wy (C, C^-1) complex columns, padding included."""
+    def up(v, m):
+        return -(-v // m) * m
+
+    def stage(rows, cols, col_tile, k):
+        return 2.0 * up(rows, 128) * up(cols, col_tile) * k * 3
+
+    def even(cols, widest):  # the tile of the fewest tiles, a multiple of 16
+        return up(-(-cols // -(-cols // widest)), 16)
+
+    nh, kx, ky = X + 1, up(X + 1, 32), up(Y, 32)
+    r, ri = even(nh, w), even(X, 2 * w)
+    first = stage(n * Y, nh, r, 2 * up(X, 32))
+    if toeplitz:
+        t = 2.0 * 2 * nh * up(2 * n, 128) * min(256, up(Y, 16)) * ky * 3
+        return first + t + 2 * stage(n * up(Y, 8), X, ri, 2 * kx)
+    return (first + stage(2 * ky, n * kx, wy, 2 * ky) + stage(Y, 2 * n * kx, wy, 4 * ky)
+            + stage(2 * n * Y, X, ri, 2 * kx))
+
+
+@pytest.mark.parametrize("X,Y,n,w,wy,toeplitz", [(512, 512, 1, 32, 32, False), (1200, 700, 1, 64, 128, False),
+                                                 (1500, 250, 2, 64, 128, False), (1300, 250, 4, 128, 128, False),
+                                                 (400, 225, 16, 128, 0, True)])
+def test_split_bf16_tiles_fill_whole_rounds(cuda, tf, oracle, X, Y, n, w, wy, toeplitz):
+    """The N tile is narrow only as far as its tiles go over the SMs without
+    another round, with the rows of equal grids taken together: seen by the
+    padding in the executed products; the FP64 bars."""
+    import workloads as W
+
+    insts = [W.make_instance(X, Y, 90 + i, mass_density=0.03) for i in range(n)]
+    b = tf.Batch(insts, precision=tf.PRECISION_SPLIT_BF16)
+    assert b.profile_phases(2).grav_flops_per_tick == executed_flops(X, Y, n, w, wy, toeplitz)
+    b.step(1)
+    cuda.cuda.synchronize()
+    check_clean(tf)
+    got = b.state(n - 1)
+    dx, dy = oracle.grav_solve(X, Y, insts[-1].gmask, mass_fx=insts[-1].mass_fx, dtype=np.float64)
+    for k, d in (("gx", dx), ("gy", dy)):
+        emax, el2 = errors(got[k], d)
+        assert emax <= TOL and el2 <= TOL, (k, emax, el2)
+    b.close()

@@ -979,39 +979,70 @@ static YMode y_mode_from_env(uint32_t *min_group) {
     return YMODE_AUTO;
 }
 
-// The widest N tile (128, 64 or 32 complex columns) at which R, the stage with
-// the fewest tiles, gives every SM one. With few grids a stage makes so few
-// tiles of 128 columns that most SMs idle while the others run its K loops and
-// epilogues; narrow tiles load A more often, which the idle SMs have time for.
-// Measured on B200, one solve: 512x512 148 us at 128 columns, 110 at 32, and 98
-// with the stages as programmatic dependents (`dependent`, taken with them);
-// 51x104 65.6, 51.1 and 41.0 us. The sums over K are the same: same bits.
-static uint32_t tile_width(const std::vector<JobShape> &shapes) {
-    for (uint32_t w = NT; w > 32; w /= 2) {
-        size_t tiles = 0;
-        for (const JobShape &s : shapes) tiles += (size_t)((s.Y + MT - 1) / MT) * ((s.X + 1 + w - 1) / w);
-        if (tiles >= 148) return w;
+// Instances of one shape: their rows follow each other in the stages' operands.
+struct ShapeGroup {
+    uint32_t X, Y, G;
+    bool toe;
+};
+static size_t tiles_across(size_t v, size_t t) { return (v + t - 1) / t; }
+// What a stage's tiles of w columns cost: a K tile loads 64 + w units of 256
+// bytes (A's 128 rows, B's w columns), a round of tiles over the SMs lasts as
+// many of those, and its start and epilogue about 64 more.
+static size_t stage_cost(size_t tiles, uint32_t w) { return tiles_across(tiles, 148) * (128 + w); }
+// Tiles of R at N tiles of w complex columns, and of R^-1 at twice that in
+// real ones.
+static size_t r_tiles(const std::vector<ShapeGroup> &groups, uint32_t w) {
+    size_t n = 0;
+    for (const ShapeGroup &s : groups) n += tiles_across((size_t)s.G * s.Y, MT) * tiles_across(s.X + 1, w);
+    return n;
+}
+static size_t ri_tiles(const std::vector<ShapeGroup> &groups, uint32_t w) {
+    size_t n = 0;
+    for (const ShapeGroup &s : groups) {
+        const size_t rows = s.toe ? 2 * tiles_across((size_t)s.G * round_up(s.Y, 8), MT)  // a problem per field
+                                  : tiles_across((size_t)2 * s.G * s.Y, MT);
+        n += rows * tiles_across(s.X, 2 * w);
     }
-    return 32;
+    return n;
 }
 
-// The N tile of C and C^-1 for few grids. They have two to four times R's tiles,
-// so R's width can give them two rounds of narrow tiles where one round of
-// wider ones is cheaper: a K tile loads 64 + w units of 256 bytes (A's 128 rows,
-// B's w columns), and a stage lasts as many of those as its rounds. Measured on
-// B200 at 32 and 64 columns, one solve: 256x256 48.7 and 55.3 us, 512x512 74.3
-// and 80.8, 700x700 134 and 105.
-static uint32_t y_tile_width(const std::vector<JobShape> &shapes, uint32_t width) {
+// The N tile of R and R^-1 (128, 64 or 32 complex columns). With few grids tiles
+// of 128 columns leave most SMs idle while the others run their K loops and
+// epilogues, but a width whose tiles need a second round costs more than it
+// spreads. R^-1 has twice R's K. Measured on B200, us per solve at 128, 64 and
+// 32 columns, the chosen width in brackets: one 512x512 100, 78, [76]; one
+// 1200x700 167, [150], 195; four 512x512 119, [117], 133; six 1000x100 118,
+// [105], 138; eight 400x225 81, [79], 85; sixteen 400x225 [107], 116, 128;
+// sixteen 1000x100 [140], 165, 202; two 1500x250 162, [143], 193; four 1500x250
+// [203], 247, 296; 64 of 160x160 [84], 92, 92. The sums over K are the same:
+// same bits.
+static uint32_t tile_width(const std::vector<ShapeGroup> &groups) {
+    uint32_t best = NT;
+    size_t least = SIZE_MAX;
+    for (uint32_t w = NT; w >= 32; w /= 2) {
+        const size_t cost = stage_cost(r_tiles(groups, w), w) + 2 * stage_cost(ri_tiles(groups, w), w);
+        if (cost < least) {
+            least = cost;
+            best = w;
+        }
+    }
+    return best;
+}
+
+// The N tile of C and C^-1 where R takes a narrow one, by the same count: they
+// have two to four times R's tiles. Measured on B200 at 32 and 64 columns, one
+// solve: 256x256 48.7 and 55.3 us, 512x512 74.3 and 80.8, 700x700 134 and 105.
+static uint32_t y_tile_width(const std::vector<ShapeGroup> &groups, uint32_t width) {
     uint32_t best = width;
     size_t least = SIZE_MAX;
     for (uint32_t w = NT; w >= 32 && width < (uint32_t)NT; w /= 2) {
         size_t c = 0, ci = 0;
-        for (const JobShape &s : shapes) {
-            const size_t cols = ((size_t)s.X + 1 + 31) / 32 * 32, slots = ((size_t)s.Y + KT - 1) / KT * KT * 2;
-            c += (slots + MT - 1) / MT * ((cols + w - 1) / w);
-            ci += ((size_t)s.Y + MT - 1) / MT * ((2 * cols + w - 1) / w);
+        for (const ShapeGroup &s : groups) {
+            const size_t cols = (size_t)s.G * round_up(s.X + 1, 32), slots = 2 * (size_t)round_up(s.Y, KT);
+            c += tiles_across(slots, MT) * tiles_across(cols, w);
+            ci += tiles_across(s.Y, MT) * tiles_across(2 * cols, w);
         }
-        const size_t cost = ((c + 147) / 148 + 2 * ((ci + 147) / 148)) * (64 + w);  // C^-1: twice the K
+        const size_t cost = stage_cost(c, w) + 2 * stage_cost(ci, w);  // C^-1: twice the K
         if (cost < least) {
             least = cost;
             best = w;
@@ -1053,9 +1084,22 @@ int DftSet::create(const std::vector<JobShape> &shapes) {
     I->inst_group.resize(n);
     I->inst_local.resize(n);
     I->hg.resize(members.size());
-    const uint32_t width = tile_width(shapes);
-    const uint32_t y_width = y_tile_width(shapes, width);
-    I->dependent = width < (uint32_t)NT;
+    // Form of a group's y stage: Toeplitz when it has at least kToeMinGroup
+    // instances and Y fits one T tile.
+    auto takes_toeplitz = [&](uint32_t Y, uint32_t G) {
+        return Y <= (uint32_t)T_NMAX && ymode != YMODE_DFT &&
+               G >= (ymode == YMODE_TOEPLITZ ? toe_min_group : kToeMinGroup);
+    };
+    std::vector<ShapeGroup> counts;
+    for (const auto &mv : members) {
+        const JobShape &s = shapes[mv[0]];
+        counts.push_back({s.X, s.Y, (uint32_t)mv.size(), takes_toeplitz(s.Y, (uint32_t)mv.size())});
+    }
+    const uint32_t width = tile_width(counts);
+    const uint32_t y_width = y_tile_width(counts, width);
+    // Programmatic dependent launches where a stage leaves SMs idle: one
+    // 512x512 103 -> 100 us at 128 columns, 79 -> 76 at 32, and 51x104 51 -> 41.
+    I->dependent = r_tiles(counts, NT) < 148;
     uint32_t inst0 = 0;
     for (size_t gi = 0; gi < members.size(); ++gi) {
         HostGroup &H = I->hg[gi];
@@ -1107,13 +1151,7 @@ int DftSet::create(const std::vector<JobShape> &shapes) {
         const double fRi = 2.0 * tiles_of(g.rowsRi, MT) * tiles_of(g.X, g.wRI) * 2 * g.kpRi * 3;
         const double fT = 2.0 * 2 * g.N1h * tiles_of(2 * g.G, MT) * g.nTy * g.kpC * 3;
         const double fRiT = 2.0 * 2 * tiles_of(g.G * g.Yp, MT) * tiles_of(g.X, g.wRI) * 2 * g.kpRi * 3;
-        // Form of the y stage: Toeplitz when the group has at least
-        // kToeMinGroup instances and Y fits one T tile.
-        const bool toe_ok = g.Y <= (uint32_t)T_NMAX;
-        g.toe = !toe_ok                   ? 0u
-                : ymode == YMODE_TOEPLITZ ? (g.G >= toe_min_group ? 1u : 0u)
-                : ymode == YMODE_DFT      ? 0u
-                                          : (g.G >= kToeMinGroup ? 1u : 0u);
+        g.toe = takes_toeplitz(g.Y, g.G) ? 1u : 0u;
         if ((rc = I->alloc(&g.aR, (size_t)2 * g.rowsR * g.kpR))) return rc;
         if ((rc = I->alloc(&H.f1, (size_t)4 * g.N1h * H.kpF1))) return rc;
         if ((rc = I->alloc(&H.g1, (size_t)4 * g.X * H.kpG1))) return rc;
