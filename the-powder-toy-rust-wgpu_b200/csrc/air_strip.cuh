@@ -606,21 +606,5 @@ __device__ __forceinline__ void strip_heat(const StripGrids &P, const AirInst &I
     }
 }
 
-// The masks of an instance without ambient heat.
-__device__ __forceinline__ void strip_masks(const StripGrids &P, const AirInst &I, uint32_t off, int x0, int y0, int y1,
-                                            uint32_t lag) {
-    const StripCols C(I, x0, HEAT_HALO);
-    if (!C.output(HEAT_HALO)) return;
-    for (int y = y0; y < y1; ++y) {
-        const uint32_t w = off + (uint32_t)y * I.pitch + (uint32_t)C.x, me = P.emap[w];
-        const uint32_t raw = emap_seen(me, lag), next = raw != 0u ? raw - 1u : 0u;
-        if (next != me) P.emap[w] = next;
-        uint32_t ba, bh;
-        masks_of(load_after_wait(P.wall + w), raw, load_after_wait(P.eair + w), load_after_wait(P.eairh + w), ba, bh);
-        P.bair_out[w] = ba;
-        P.bairh_out[w] = bh;
-    }
-}
-
 }  // namespace air
 }  // namespace tpt

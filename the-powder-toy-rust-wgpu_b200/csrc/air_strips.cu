@@ -51,6 +51,25 @@ __global__ void __launch_bounds__(STRIP_WARPS * 32, 6)
     }
 }
 
+// The masks of an instance without ambient heat. The batch's launches are
+// ordinary ones, and nothing writes what they read this way: as ordinary loads,
+// which stay behind the row before's stores, the step of 64 grids of 400x225
+// without heat took 255 us where it takes 234.
+__device__ __forceinline__ void strip_masks(const StripGrids &P, const AirInst &I, uint32_t off, int x0, int y0, int y1,
+                                            uint32_t lag) {
+    const StripCols C(I, x0, HEAT_HALO);
+    if (!C.output(HEAT_HALO)) return;
+    for (int y = y0; y < y1; ++y) {
+        const uint32_t w = off + (uint32_t)y * I.pitch + (uint32_t)C.x, me = P.emap[w];
+        const uint32_t raw = emap_seen(me, lag), next = raw != 0u ? raw - 1u : 0u;
+        if (next != me) P.emap[w] = next;
+        uint32_t ba, bh;
+        masks_of(__ldg(P.wall + w), raw, __ldg(P.eair + w), __ldg(P.eairh + w), ba, bh);
+        P.bair_out[w] = ba;
+        P.bairh_out[w] = bh;
+    }
+}
+
 __global__ void __launch_bounds__(STRIP_WARPS * 32, 6)
     kb_heat_masks(const __grid_constant__ StripGrids P, const float *su, const float *sv,
                   const AirInst *__restrict__ insts, const StripRef *__restrict__ strips, uint32_t nstrips,
