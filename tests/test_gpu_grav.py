@@ -140,3 +140,33 @@ def test_fp32_square_plans(cuda, tf, oracle, n):
     """Both axes of one length, each with a factoring of its own (and, at 67,
     of three radices); the bar is the solve's."""
     test_fp32_plan_lengths(cuda, tf, oracle, n, n)
+
+
+@pytest.mark.parametrize("X,Y,dims", [(25, 30, (50, 60)), (24, 31, (48, 64)), (33, 36, (80, 80)), (64, 65, (128, 144)),
+                                      (17, 50, (36, 100)), (100, 121, (200, 250))])
+def test_fp32_short_axes_of_one_grid_take_small_radices(cuda, tf, oracle, X, Y, dims):
+    """One grid's transforms of up to 128 points have no radix above 10, at the
+    price of a longer one (72 -> 80 points); the solve's bar."""
+    solver = tf.GravityFft()
+    solver._ensure(X, Y)
+    assert solver.padded_dims() == dims
+    solver.close()
+    test_fp32_plan_lengths(cuda, tf, oracle, X, Y)
+
+
+@pytest.mark.parametrize("X,Y,n", [(33, 36, 4), (48, 25, 16), (64, 64, 37), (64, 64, 38), (153, 96, 10), (153, 96, 11)])
+def test_fp32_batches_of_few_points(cuda, tf, oracle, X, Y, n):
+    """Batches on both sides of the line (303,104 points) up to which they
+    take one grid's radices; the solve's bar on the first and last grid."""
+    import workloads as W
+
+    insts = [W.make_instance(X, Y, 300 + i, mass_density=0.03) for i in range(n)]
+    b = tf.Batch(insts)
+    b.step(1)
+    cuda.cuda.synchronize()
+    for i in (0, n - 1):
+        got = b.state(i)
+        dx, dy = oracle.grav_solve(X, Y, insts[i].gmask, mass_fx=insts[i].mass_fx, dtype=np.float64)
+        scale = max(np.abs(dx).max(), np.abs(dy).max(), 1e-30)
+        assert np.abs(got["gx"] - dx).max() <= TOL * scale and np.abs(got["gy"] - dy).max() <= TOL * scale
+    b.close()

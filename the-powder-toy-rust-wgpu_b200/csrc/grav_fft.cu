@@ -377,35 +377,50 @@ __global__ void spectrum_cols_f64(const double2 *rows, uint32_t n1, uint32_t n2,
 }
 
 // ---- lengths and tables --------------------------------------------------------
+// Points of a set's row transforms up to which the set is as a single grid
+// (see axis_for): two blocks of 1024 points per SM.
+constexpr size_t FEW_POINTS = 2 * 148 * 1024;
+
 // The axis of `cells` cells: the shortest even length that holds the linear
 // convolution, 2 cells - 1, as a product of two radices or else of three.
 // Neighbouring lengths lie within 1.25 of each other (1.07 on average above
 // 256), where padding to a power of two costs up to 2 in each direction.
 //
 // Of the factorings of that length a batch takes two radices before three:
-// fewer steps. One grid is a serial chain instead, with fewer work items than
-// threads, and takes the smallest radices. Measured on B200, us per solve of
-// one grid, two radices and smallest: 153x96 19.2 and 14.8, 300x64 17.4 and
-// 14.2, 400x225 (no factoring in two) 19.5; 256 grids 0.402 and 0.439 ms.
+// fewer steps. A set of few points -- one grid, or a batch below FEW_POINTS --
+// is a serial chain instead, with fewer work items than threads, and takes the
+// smallest radices. Measured on B200, us per solve of one grid, two radices and
+// smallest: 153x96 19.2 and 14.8, 300x64 17.4 and 14.2, 400x225 (no factoring in
+// two) 19.5; of 16 grids 153x96 26.7 and 22.6, 64x64 22.2 and 16.4, of 4 20.5 and
+// 14.4; 64 of 48x48 20.5 and 18.5, 64 of 64x64 (0.5 million points) 24.5 and 22.6;
+// 256 of 32x32 (as many) 22.5 and 28.7, 256 of 48x48 35.0 and 41.0, the mixed 256
+// grids 402 and 439.
+//
+// For the same reason such a set takes no radix above 10 in a short transform,
+// even where another length is the price: 72 points are 12 x 6, 80 are 5 x 4 x 4.
+// One 33x33 grid (72 and 80 points) 14.3 and 11.2 us per solve, 27.4 and 24.0 with
+// the air's launches before it, at errors against 64 bits of 1.14e-7 and 0.97e-7.
+// (Radix 10 stays: 64 points instead of its 60 gain 0.8 us and lose a third of
+// the precision, 1.01e-7 and 1.35e-7.)
 //
 // The largest radix r1 loads a column and r3, which has the most work items,
 // inverts its two products. Rows have it the other way round: their loading
 // step takes two rows of masses and masks per item, and is the longest with a
 // large radix. 16x16 10.1 -> 8.7 us, 600x400 30.2 -> 26.6, 256 grids 0.402 ->
 // 0.392 ms (columns the same way: 1000x900 64.2 -> 69.4 us).
-static bool axis_for(uint32_t cells, bool one_grid, bool rows, Axis *out) {
-    const uint32_t need = std::max<uint32_t>(2 * cells - 1, 32u);
+static bool axis_for(uint32_t cells, bool few, bool rows, Axis *out) {
+    const uint32_t need = std::max<uint32_t>(2 * cells - 1, 32u), largest = few && need <= 128 ? 10u : 16u;
     Axis best{};
     for (uint32_t r1 : kRadices)
         for (uint32_t r2 = 1; r2 <= r1; ++r2) {
             if (r2 > 1 && std::find(std::begin(kRadices), std::end(kRadices), r2) == std::end(kRadices)) continue;
             for (uint32_t r3 : kRadices) {
                 const uint32_t n = r1 * r2 * r3;
-                if (r3 > r1 || n < need || n % 2) continue;
+                if (r1 > largest || r3 > r1 || n < need || n % 2) continue;
                 bool better = best.n == 0 || n < best.n;
                 if (n == best.n) {  // r1 is the largest
-                    if (one_grid && r1 != best.r1) better = r1 < best.r1;
-                    else if (!one_grid && (r2 == 1) != (best.r2 == 1)) better = r2 == 1;
+                    if (few && r1 != best.r1) better = r1 < best.r1;
+                    else if (!few && (r2 == 1) != (best.r2 == 1)) better = r2 == 1;
                     else better = r1 + r2 + r3 < best.r1 + best.r2 + best.r3;
                 }
                 if (better) {
@@ -530,9 +545,12 @@ int FftSet::create(const std::vector<JobShape> &shapes) {
         axes_off.push_back(twh.size());
         fill_twiddles(a, twh);
     };
+    size_t least = 0;  // points of the row transforms, without padding
+    for (const JobShape &s : shapes) least += (size_t)s.Y * (2 * s.X - 1);
+    const bool few = nj == 1 || least < FEW_POINTS;
     for (size_t j = 0; j < nj; ++j) {
         Job &J = jobs_host[j];
-        if (!axis_for(shapes[j].X, nj == 1, true, &J.ax) || !axis_for(shapes[j].Y, nj == 1, false, &J.ay))
+        if (!axis_for(shapes[j].X, few, true, &J.ax) || !axis_for(shapes[j].Y, few, false, &J.ay))
             TPT_FAIL(TPT_ERR_INVALID_DIMS, "gravity grid %ux%u exceeds the longest transform", shapes[j].X, shapes[j].Y);
         J.X = J.pitch = shapes[j].X;
         J.Y = shapes[j].Y;
