@@ -54,8 +54,9 @@ __device__ __forceinline__ const Job &stage_job(const Job *jobs, const BlockRef 
 }
 
 // ---- the three passes ------------------------------------------------------------
-// Programmatic dependent launches: the next pass's blocks are launched as this
-// one's drain, stage their job, and wait for its results.
+// In a one-grid solve they are programmatic dependent launches: the next pass's
+// blocks are launched as this one's drain, stage their job, and wait for its
+// results.
 //
 // One function per radix and step: blocks of all lengths share them.
 template <int R, bool INV> __device__ __noinline__ void row_step2(const Axis &A, uint32_t cnt) {
@@ -674,14 +675,18 @@ int FftSet::launch(cudaStream_t st, const JobIO *io) const {
         one.gy = io->gy;
         one.mass_scale_inv = io->mass_scale_inv;
     }
-    // Every pass is a programmatic dependent of the one before it, and the first
-    // pass of one grid of the work before the solve: it waits for that to
+    // Every pass of a one-grid solve is a programmatic dependent of the one
+    // before it, the first of the work before the solve: it waits for that to
     // complete, and only its launch overlaps it (a gravity tick of 153x96 cells
     // and 117,500 particles, with its other kernels dependent too, 36.2 -> 29.3
-    // us; a solve of 400x225 cells 22.6 -> 20.9). A batch's first pass
-    // is an ordinary launch: its blocks would take their places among those of
-    // the air kernels running beside it (256 grids 0.52 -> 0.57 ms).
-    auto run = [&](void (*kernel)(const Job *, const BlockRef *, const Job), const Pass &p, bool dependent) -> int {
+    // us; a solve of 400x225 cells 22.6 -> 20.9). A batch's passes are ordinary
+    // launches: blocks that wait take their places among those of the air
+    // kernels running beside them. Alone they are 1 to 6 us slower, but a step is
+    // faster, us with dependent and ordinary ones: 2 grids of 400x225 33.7 and
+    // 30.5, 16 of 64x64 23.5 and 21.8, 64 of 48x48 35.1 and 30.7, 16 of 153x96 43.5 and
+    // 37.7, 256 of 24x24 34.6 and 29.7, the mixed 256 grids 815 and 813 (64 of
+    // 100x100 94.5 and 95.6).
+    auto run = [&](void (*kernel)(const Job *, const BlockRef *, const Job), const Pass &p) -> int {
         if (p.blocks == 0) return TPT_OK;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(p.blocks);
@@ -692,16 +697,16 @@ int FftSet::launch(cudaStream_t st, const JobIO *io) const {
         at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
         at.val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = &at;
-        cfg.numAttrs = dependent ? 1 : 0;
+        cfg.numAttrs = io ? 1 : 0;
         TPT_CUDA(cudaLaunchKernelEx(&cfg, kernel, io ? (const Job *)nullptr : (const Job *)jobs,
                                     (const BlockRef *)(refs + p.first), one));
         TPT_LAUNCHED();
         return TPT_OK;
     };
-    int rc = run(k_rows_forward, rows, io != nullptr);
-    if (rc == TPT_OK) rc = run(k_columns, cols[1], true);
-    if (rc == TPT_OK) rc = run(k_columns, cols[0], true);
-    if (rc == TPT_OK) rc = run(k_rows_inverse, inv, true);
+    int rc = run(k_rows_forward, rows);
+    if (rc == TPT_OK) rc = run(k_columns, cols[1]);
+    if (rc == TPT_OK) rc = run(k_columns, cols[0]);
+    if (rc == TPT_OK) rc = run(k_rows_inverse, inv);
     return rc;
 }
 
