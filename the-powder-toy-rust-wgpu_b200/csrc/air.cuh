@@ -702,15 +702,25 @@ __device__ __forceinline__ uint32_t emap_seen(uint32_t stored, uint32_t lag) {
     return stored > lag ? stored - lag : 0u;
 }
 
-// The same for cell g of an instance, decaying its emap in place (after the
+// A cell's words of the mask rebuild. All are requested before any is used or
+// written: an ordinary load stays behind the stores before it.
+struct MaskWords {
+    uint32_t wall, emap, eair, eairh;
+    __device__ __forceinline__ MaskWords(const AirInst &I, size_t g) {
+        emap = load_after_wait(I.emap + g);
+        wall = load_after_wait(I.wall + g);
+        eair = I.eair ? load_after_wait(I.eair + g) : 0u;
+        eairh = I.eairh ? load_after_wait(I.eairh + g) : 0u;
+    }
+};
+// masks_of for cell g of an instance, decaying its emap in place (after the
 // `lag` decays it still lacks).
-__device__ __forceinline__ void masks_cell(const AirInst &I, size_t g, uint32_t &bair, uint32_t &bairh,
-                                           uint32_t lag = 0u) {
-    const uint32_t stored = I.emap[g];
-    const uint32_t raw = emap_seen(stored, lag);
+__device__ __forceinline__ void masks_cell(const AirInst &I, size_t g, const MaskWords &m, uint32_t &bair,
+                                           uint32_t &bairh, uint32_t lag = 0u) {
+    const uint32_t raw = emap_seen(m.emap, lag);
     const uint32_t next = raw != 0u ? raw - 1u : 0u;
-    if (next != stored) I.emap[g] = next;
-    masks_of(load_after_wait(I.wall + g), raw, I.eair ? load_after_wait(I.eair + g) : 0u, I.eairh ? load_after_wait(I.eairh + g) : 0u, bair, bairh);
+    if (next != m.emap) I.emap[g] = next;
+    masks_of(m.wall, raw, m.eair, m.eairh, bair, bairh);
 }
 
 }  // namespace AIR_SHAPE_NS

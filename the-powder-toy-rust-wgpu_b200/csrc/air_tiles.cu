@@ -265,7 +265,7 @@ __global__ void __launch_bounds__(NT, B_MIN_CTAS) kb_advect_heat(const AirInst *
         if (in_grid(gx, gy, I)) {
             size_t g = (size_t)gy * I.pitch + gx;
             uint32_t ba, bh;
-            masks_cell(I, g, ba, bh, emap_lag);
+            masks_cell(I, g, MaskWords(I, g), ba, bh, emap_lag);
             I.bair_out[g] = ba;
             I.bairh_out[g] = bh;
         }
