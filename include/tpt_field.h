@@ -347,10 +347,12 @@ enum {
     /* Two launches per tick over tiles (32x8, 64x8, 32x16 or 64x16 cells),
      * halos staged by TMA: pass A (pressure, velocity) writes opv/ovx/ovy,
      * pass B (smoothing, advection, vorticity, fans, heat, convection, masks)
-     * reads them. A batch of 2 million cells or more (6 million where nearly
-     * all grids are 31 or 32 cells wide) runs the same passes as strips, one
-     * per warp, of 26 to 30 columns and a number of rows that goes with the
-     * tile shape (24, 32, 16 and 40 on average), B as two launches. */
+     * reads them. A batch of 2 million cells or more (a cell without ambient
+     * heat counts a third, one of a NoUpdate instance half, and the line is 6
+     * million where nearly all grids are 31 or 32 cells wide) runs the same
+     * passes as strips, one per warp, of 26 to 30 columns, B as two launches.
+     * A strip has about as many rows as go with the tile shape (24, 32, 16 and
+     * 40), fewer where that makes less than three strips per resident warp. */
     TPT_AIR_FORM_TILES = 0,
     /* One fused launch per tick: CTAs sweep down column strips with every
      * stage pipelined over the rows (no intermediate grid in memory), plus a

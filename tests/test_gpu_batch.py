@@ -430,6 +430,25 @@ def test_which_batches_run_strips(cuda, tf, side, n, launches):
     b.close()
 
 
+@pytest.mark.parametrize("kinds,launches", [([(dict(aheat_enable=0), 24)], 2), ([(dict(aheat_enable=0), 66)], 2),
+                                            ([(dict(aheat_enable=0), 67)], 3),
+                                            ([(dict(air_mode=4), 44)], 3), ([(dict(air_mode=4), 45)], 4),
+                                            ([(dict(air_mode=4, aheat_enable=0), 44)], 2),
+                                            ([(dict(air_mode=4, aheat_enable=0), 45)], 3),
+                                            ([({}, 12), (dict(aheat_enable=0), 30)], 2),
+                                            ([({}, 12), (dict(aheat_enable=0), 31)], 3)])
+def test_cells_count_for_strips_by_what_they_do(cuda, tf, kinds, launches):
+    """Grids of 400x225: without ambient heat a cell counts a third towards
+    the 2 million from which a batch runs strips (three launches a tick, not
+    two), with NoUpdate half (and with heat too, its settle: one more)."""
+    import workloads as W
+
+    insts = [i for kw, n in kinds for i in [W.make_instance(400, 225, 3, config=W.AirConfig(newton_grav=0, **kw))] * n]
+    b = tf.Batch(insts)
+    assert b.profile_phases(2).air_launches_per_tick == launches
+    b.close()
+
+
 @pytest.mark.parametrize("form", [0, 1])
 def test_refused_tuning_leaves_the_batch_as_it_was(cuda, tf, oracle, form):
     """A tuning that is refused for its last field after an earlier one asked

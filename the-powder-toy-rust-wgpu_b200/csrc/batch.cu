@@ -96,19 +96,27 @@ constexpr uint32_t DEFAULT_TILE_X = 32, DEFAULT_TILE_Y = 8;
 // 6.0 M 515 and 532. Widths with fewer idle lanes keep the line: 30x512 2.0 M
 // 230 and 215, 60x512 214 and 195, 64x64 236 and 216, 64x512 204 and 203 (but
 // 64x2048 186 and 206), 96x512 185 and 173, 400x225 173 and 167.
+//
+// That is with ambient heat, whose pass is the tiles' dearest. Without it strips
+// win from three times the cells, and NoUpdate instances, whose tick is the heat
+// pass or the masks alone, from twice. Air alone, tiles and strips: no heat,
+// 400x225 2.1 M 123 and 142, 4.1 M 224 and 231, 5.8 M 308 and 316, 7.2 M 380 and 375;
+// sides 32 to 512 2.2 M 137 and 149, 4.0 M 243 and 245, 6.0 M 352 and 341; 512x512
+// 4.2 M 219 and 248; NoUpdate, 400x225 2.1 M 91 and 101, 3.2 M 136 and 142, 4.1 M 168
+// and 166; 64x64 2.0 M 98 and 122, 4.0 M 186 and 197; without heat 38 and 47, 77 and 74.
 constexpr size_t STRIP_MIN_CELLS = 2000000;
 static bool runs_strips(uint32_t n, const tpt_instance_desc *descs) {
-    uint64_t cells = 0, strip_rows = 0, tile_rows = 0;
+    uint64_t sixths = 0, strip_rows = 0, tile_rows = 0;  // sixths of cells, each by what it counts
     for (uint32_t i = 0; i < n; ++i) {
         const uint32_t X = descs[i].air.xcells, Y = descs[i].air.ycells;
-        cells += (uint64_t)X * Y;
+        sixths += (uint64_t)X * Y * (descs[i].air.air_mode == 4u ? 3 : descs[i].air.aheat_enable ? 6 : 2);
         for (int k = 0; k < air::STRIP_PASSES; ++k) {
             const uint32_t w = (uint32_t)air::strip_width(k);
             strip_rows += (uint64_t)((X + w - 1) / w) * Y;
             tile_rows += (uint64_t)((X + DEFAULT_TILE_X - 1) / DEFAULT_TILE_X) * Y;
         }
     }
-    return cells >= (10 * strip_rows < 18 * tile_rows ? 1 : 3) * STRIP_MIN_CELLS;
+    return sixths >= (10 * strip_rows < 18 * tile_rows ? 6 : 18) * (uint64_t)STRIP_MIN_CELLS;
 }
 
 // Splits every instance into column strips of at most lanes - 2 * SW_H
