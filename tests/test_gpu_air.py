@@ -198,3 +198,13 @@ def test_large_grid_strips(cuda, tf, oracle, X, Y, kw):
     assert X * Y >= 350000
     inst = W.make_stress_instance(X, Y, X + Y, config=W.AirConfig(**kw))
     assert_bit_exact(run_gpu(tf, cuda, inst, 2), oracle.air_steps(inst, 2), f"{X}x{Y}")
+
+
+@pytest.mark.parametrize("X,Y", [(548, 547), (548, 548), (1000, 300), (999, 300)])
+def test_grids_beside_the_strips_line(cuda, tf, oracle, X, Y):
+    """One grid on both sides of 300,000 cells, with NaN, Inf and velocities
+    past the clamp."""
+    from test_oracle_air_numpy import nonfinite_instance
+
+    inst = nonfinite_instance(X, Y, 9)
+    assert_bit_exact(run_gpu(tf, cuda, inst, 2), oracle.air_steps(inst, 2), f"{X}x{Y}", nan_equal=True)

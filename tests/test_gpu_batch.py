@@ -494,3 +494,44 @@ def test_large_batch_strips_match_oracle(cuda, tf, oracle, queue, ticks):
     cuda.cuda.synchronize()
     check_against_oracle(tf, oracle, b, insts, ticks, f"strips, {ticks} ticks")
     b.close()
+
+
+@pytest.mark.parametrize("depth,ticks", [(1, 4), (3, 5), (4, 4)])
+def test_large_batch_strips_odd_inputs(cuda, tf, oracle, depth, ticks):
+    """Strips, alone and around temporally blocked launches (whose settle of
+    the NoUpdate + heat instances is the strips'), with NaN, Inf and
+    velocities past the clamp in some instances: bit-exact."""
+    import workloads as W
+    from test_gpu_air import assert_bit_exact
+    from test_oracle_air_numpy import nonfinite_instance
+
+    insts = [nonfinite_instance(), nonfinite_instance(70, 50, 32)]
+    for i, (X, Y) in enumerate([(61, 73), (28, 49), (84, 31), (33, 97), (1100, 900), (1101, 1000)]):
+        cfg = W.AirConfig(air_mode=(4, 0, 4, 2, 0, 0)[i], aheat_enable=int(i != 2), newton_grav=0)
+        insts.append(W.make_stress_instance(X, Y, 700 + i, config=cfg))
+    b = tf.Batch(insts)
+    assert b.profile_phases(2).air_launches_per_tick == 4  # three passes and the settle
+    b.close()
+    b = tf.Batch(insts)
+    set_form(tf, b, tf.AIR_FORM_TILES, temporal_depth=depth)
+    b.step(ticks)
+    cuda.cuda.synchronize()
+    for i, inst in enumerate(insts):
+        assert_bit_exact(b.state(i), oracle.air_steps(inst, ticks), f"depth {depth} instance {i}", nan_equal=True)
+    b.close()
+
+
+def test_tiles_below_the_strips_line(cuda, tf, oracle):
+    """The largest batches that still run tiles (1.9 million cells)."""
+    import workloads as W
+
+    insts = [W.make_stress_instance(X, Y, 40 + i, config=W.AirConfig(newton_grav=0))
+             for i, (X, Y) in enumerate([(701, 733), (1023, 517), (33, 2047), (1200, 640)])]
+    b = tf.Batch(insts)
+    assert 1800000 < b.total_cells < 2000000 and b.profile_phases(2).air_launches_per_tick == 2
+    b.close()
+    b = tf.Batch(insts)
+    b.step(3)
+    cuda.cuda.synchronize()
+    check_against_oracle(tf, oracle, b, insts, 3, "tiles")
+    b.close()
