@@ -526,7 +526,8 @@ typedef struct tpt_vox_plan tpt_vox_plan;
  */
 int tpt_vox_plan_create(int form, tpt_vox_plan **out);
 int tpt_vox_plan_destroy(tpt_vox_plan *plan);
-/* The form the plan runs (TPT_VOX_CLUSTER or TPT_VOX_PER_SWEEP). */
+/* The form the plan runs (TPT_VOX_CLUSTER, TPT_VOX_PER_SWEEP or
+ * TPT_VOX_BATCHED). */
 int tpt_vox_plan_form(const tpt_vox_plan *plan);
 
 /* air_clear_kernel (air_kernel.rs:182-204): zero velocity, pressure, solid
