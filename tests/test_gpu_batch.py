@@ -416,6 +416,22 @@ def test_tuning_times_each_strip_layout_once(cuda, tf):
     b.close()
 
 
+def test_tuning_times_a_strip_layout_with_and_without_the_queue(cuda, tf):
+    """The settings of one strip layout that differ in its CTAs per SM alone
+    are not timed: 2 settings of the strips and 3 of the sweep, 2 x 20 ticks
+    each of 3 and 2 launches. (They were within the noise of each other and
+    took the places of the strided layout among the few that are timed beside
+    the gravity.)"""
+    import workloads as W
+
+    inst = W.make_instance(400, 225, 1, config=W.AirConfig(newton_grav=0))
+    b = tf.Batch([inst] * 25)
+    n0 = tf.launch_count()
+    b.tune()
+    assert 0 < tf.launch_count() - n0 <= 2 * 40 * 3 + 3 * 40 * 2
+    b.close()
+
+
 @pytest.mark.parametrize("side,n,launches", [((32, 256), 245, 2), ((31, 256), 253, 2), ((32, 256), 733, 3),
                                              ((30, 256), 261, 3), ((33, 256), 237, 3), ((64, 256), 123, 3),
                                              ((64, 256), 122, 2)])

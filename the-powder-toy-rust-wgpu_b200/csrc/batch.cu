@@ -1102,9 +1102,10 @@ int tpt_batch_tune(tpt_batch *b, tpt_stream_t stream) {
     // Phase 1: the air form and its layout, by timing 20 air ticks of each
     // candidate: the tile form at every tile shape, with static striding and
     // with the atomic work queue, at each pass's own residency (0) and at 4,
-    // 6 and 8 CTAs per SM (32x8; the larger tiles at 0 and 2); the sweep form
-    // at a few shapes (lanes per CTA x rows per strip) with as many CTAs as
-    // fit.
+    // 6 and 8 CTAs per SM (32x8; the larger tiles at 0 and 2); strips, one
+    // layout each, at their passes' own residency, which 6 and 8 CTAs are within
+    // the noise of; the sweep form at a few shapes (lanes per CTA x rows per
+    // strip) with as many CTAs as fit.
     struct Cand {
         uint32_t form, x, y, per_sm, queue;
     };
@@ -1121,8 +1122,11 @@ int tpt_batch_tune(tpt_batch *b, tpt_stream_t stream) {
             if (!seen.insert(rows).second) continue;
         }
         const bool base = sh->tx == DEFAULT_TILE_X && sh->ty == DEFAULT_TILE_Y;
+        const std::vector<uint32_t> per_sm = b->use_strips ? std::vector<uint32_t>{0u}
+                                             : base        ? std::vector<uint32_t>{0u, 4u, 6u, 8u}
+                                                           : std::vector<uint32_t>{0u, 2u};
         for (uint32_t q : {1u, 0u})
-            for (uint32_t c : base ? std::vector<uint32_t>{0u, 4u, 6u, 8u} : std::vector<uint32_t>{0u, 2u})
+            for (uint32_t c : per_sm)
                 cands.push_back({TPT_AIR_FORM_TILES, sh->tx, sh->ty, c, q});
     }
     for (auto sh : {std::make_pair(224u, 64u), std::make_pair(256u, 64u), std::make_pair(256u, 32u)})
@@ -1190,20 +1194,28 @@ int tpt_batch_tune(tpt_batch *b, tpt_stream_t stream) {
     // TUNE_TICKS ticks as a step captures it, air and gravity chains
     // together -- since the gravity
     // chain runs on the SMs the air launches leave idle, the air layout that
-    // is fastest alone need not be fastest beside it. Finalists: the air
-    // settings within 5% of the fastest air-only time (at most four), each
-    // with every gravity split (CTAs of the DFT-pair groups' branch on its
-    // own stream, as a percentage of the SMs; 0 = one stream) when the batch
-    // has both kinds of y stage.
+    // is fastest alone need not be fastest beside it. Finalists (at
+    // most four): the settings within 5% of the fastest air-only time, or of
+    // strips the two fastest layouts with and without the queue, each with
+    // every gravity split (CTAs of the DFT-pair groups' branch on its own
+    // stream, as a percentage of the SMs; 0 = one stream) when the batch has
+    // both kinds of y stage. Strips taken from the queue are 2 to 15% faster
+    // alone, but the strided ones leave SMs to the gravity at the ends of the
+    // launches: us per tick with and without the queue, air alone and the
+    // step, 3.3 M cells in 90 grids 263 and 291, 497 and 465; the 6.1 M of 128
+    // grids, late, 329 and 337, 523 and 499; but 45 grids of 400x225 274 and
+    // 314, 353 and 374.
     if (rc == TPT_OK && b->any_grav) {
         std::stable_sort(timed.begin(), timed.end(),
                          [](const std::pair<float, tpt_batch_tuning> &x, const std::pair<float, tpt_batch_tuning> &y) {
                              return x.first < y.first;
                          });
         std::vector<tpt_batch_tuning> finalists{best};
+        uint32_t strips_seen[2] = {0, 0};  // without and with the queue
         for (const auto &tt : timed) {
-            if (finalists.size() >= 4 || tt.first > 1.05f * timed.front().first) break;
-            if (memcmp(&tt.second, &best, sizeof(best)) != 0) finalists.push_back(tt.second);
+            const bool strips = b->use_strips && tt.second.air_form == TPT_AIR_FORM_TILES;
+            if (strips ? strips_seen[tt.second.work_queue]++ >= 2u : tt.first > 1.05f * timed.front().first) continue;
+            if (finalists.size() < 4 && memcmp(&tt.second, &best, sizeof(best)) != 0) finalists.push_back(tt.second);
         }
         const bool split = b->precision == TPT_PRECISION_SPLIT_BF16 && b->dft.can_split();
         const uint32_t cap = split ? b->dft.max_side_ctas() : 0u;
@@ -1212,34 +1224,42 @@ int tpt_batch_tune(tpt_batch *b, tpt_stream_t stream) {
             for (uint32_t pct : {10u, 15u, 20u, 25u, 33u, 40u, 50u}) pcts.push_back(pct);
         float step_best = 1e30f;
         tpt_batch_tuning chosen = best;
-        for (const tpt_batch_tuning &fin : finalists) {
-            for (uint32_t pct : pcts) {
-                if (rc) break;
-                tpt_batch_tuning t = fin;
-                t.grav_side_ctas =
-                    pct ? std::min<uint32_t>(cap, std::max<uint32_t>(1u, (uint32_t)b->sms * pct / 100u)) : 0u;
-                rc = tpt_batch_set_tuning(b, &t);
-                cudaGraphExec_t ex = nullptr;
-                if (rc == TPT_OK) rc = graph_for(b, TUNE_TICKS, &ex);
-                float ms = 1e30f;
-                for (int rep = 0; rep < 3 && rc == TPT_OK; ++rep) {  // warm-up, then the faster of two
-                    cudaEventRecord(e0, st);
-                    if (cudaGraphLaunch(ex, st) != cudaSuccess) {
-                        set_error("graph launch failed while tuning");
-                        rc = TPT_ERR_CUDA;
-                    }
-                    cudaEventRecord(e1, st);
-                    cudaEventSynchronize(e1);
-                    float r = 0;
-                    cudaEventElapsedTime(&r, e0, e1);
-                    if (rep > 0 && r < ms) ms = r;
+        auto time_step = [&](const tpt_batch_tuning &fin, uint32_t pct) {
+            if (rc) return;
+            tpt_batch_tuning t = fin;
+            t.grav_side_ctas = pct ? std::min<uint32_t>(cap, std::max<uint32_t>(1u, (uint32_t)b->sms * pct / 100u)) : 0u;
+            rc = tpt_batch_set_tuning(b, &t);
+            cudaGraphExec_t ex = nullptr;
+            if (rc == TPT_OK) rc = graph_for(b, TUNE_TICKS, &ex);
+            float ms = 1e30f;
+            for (int rep = 0; rep < 3 && rc == TPT_OK; ++rep) {  // warm-up, then the faster of two
+                cudaEventRecord(e0, st);
+                if (cudaGraphLaunch(ex, st) != cudaSuccess) {
+                    set_error("graph launch failed while tuning");
+                    rc = TPT_ERR_CUDA;
                 }
-                if (rc) break;
-                if (ms < step_best) {
-                    step_best = ms;
-                    chosen = t;
-                }
+                cudaEventRecord(e1, st);
+                cudaEventSynchronize(e1);
+                float r = 0;
+                cudaEventElapsedTime(&r, e0, e1);
+                if (rep > 0 && r < ms) ms = r;
             }
+            if (rc == TPT_OK && ms < step_best) {
+                step_best = ms;
+                chosen = t;
+            }
+        };
+        if (b->use_strips && split) {
+            // the layouts at one split, then the fastest one at the others: each
+            // has the same best splits (128 grids, tuning 3.0 -> 1.2 s)
+            const uint32_t first = 33u;
+            for (const tpt_batch_tuning &fin : finalists) time_step(fin, first);
+            const tpt_batch_tuning fastest = chosen;
+            for (uint32_t pct : pcts)
+                if (pct != first) time_step(fastest, pct);
+        } else {
+            for (const tpt_batch_tuning &fin : finalists)
+                for (uint32_t pct : pcts) time_step(fin, pct);
         }
         best = chosen;
     }
