@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(NT_A) k_pressure_velocity(const AirInst I) {
 }
 
 // Pass B of one tile.
-__global__ void __launch_bounds__(NT_B) k_advect_heat(const AirInst I) {
+__global__ void __launch_bounds__(NT_B, 5) k_advect_heat(const AirInst I) {
     __shared__ LayoutB1 S;
     pdl_wait();
     const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;

@@ -15,8 +15,9 @@ namespace gfft {
 
 // Threads per block, and the blocks per SM the registers are capped for (80
 // registers). What bounds the passes at this size is latency: a block's chain
-// of loads (job, grid, twiddles), barriers and instruction fetch, at 24 warps
-// per SM and 16 to 55% of the issue slots; DRAM stays below 15% of its rate.
+// of loads (job, grid, twiddles), barriers and instruction fetch, at 18 to 22
+// resident warps per SM and 41 to 46% of the issue slots; DRAM at 10 to 21% of
+// its rate (64 grids of sides 32 to 512).
 // Measured on B200, solve of 256 grids (8.1 M cells, sides 32 to 512):
 // 0.392 ms (0.988 ms with one warp per transform, padded to powers of two and
 // exchanged by lane shuffles); one 400x225 grid 20.2 us (55.3); one 1200x701
