@@ -353,3 +353,27 @@ def test_split_bf16_tiles_fill_whole_rounds(cuda, tf, oracle, X, Y, n, w, wy, to
         emax, el2 = errors(got[k], d)
         assert emax <= TOL and el2 <= TOL, (k, emax, el2)
     b.close()
+
+
+@pytest.mark.parametrize("X,Y,n,launches", [(400, 225, 12, 5), (256, 256, 8, 5), (400, 225, 64, 6), (153, 96, 16, 6)])
+def test_split_bf16_groups_beside_the_y_dft(cuda, tf, oracle, X, Y, n, launches):
+    """Beside a group that takes the y DFT another one takes the Toeplitz
+    stage (a launch more) only where that executes fewer products; the FP64
+    bars on both."""
+    import workloads as W
+
+    insts = [W.make_instance(X, Y, 70 + i % 5, mass_density=0.03) for i in range(n)]
+    insts.append(W.make_instance(54, 164, 77, mass_density=0.03))
+    b = tf.Batch(insts, precision=tf.PRECISION_SPLIT_BF16)
+    assert b.profile_phases(2).grav_launches_per_tick == launches
+    b.step(1)
+    cuda.cuda.synchronize()
+    check_clean(tf)
+    for i in (0, n):
+        got = b.state(i)
+        dx, dy = oracle.grav_solve(insts[i].xcells, insts[i].ycells, insts[i].gmask, mass_fx=insts[i].mass_fx,
+                                   dtype=np.float64)
+        for k, d in (("gx", dx), ("gy", dy)):
+            emax, el2 = errors(got[k], d)
+            assert emax <= TOL and el2 <= TOL, (i, k, emax, el2)
+    b.close()

@@ -989,6 +989,18 @@ static size_t tiles_across(size_t v, size_t t) { return (v + t - 1) / t; }
 // bytes (A's 128 rows, B's w columns), a round of tiles over the SMs lasts as
 // many of those, and its start and epilogue about 64 more.
 static size_t stage_cost(size_t tiles, uint32_t w) { return tiles_across(tiles, 148) * (128 + w); }
+// Whether the Toeplitz stage and its R^-1 execute fewer products than the y DFT
+// pair and its, at tiles of 128.
+static bool fewer_products(const ShapeGroup &s) {
+    auto padded = [](size_t v) { return (double)(tiles_across(v, MT) * MT); };
+    const size_t cols = (size_t)s.G * round_up(s.X + 1, 32);
+    const double kc = round_up(s.Y, KT), ri = 2.0 * s.X * round_up(s.X + 1, KT);
+    const double pair = padded(2 * (size_t)kc) * padded(cols) * 2 * kc + padded(s.Y) * padded(2 * cols) * 4 * kc +
+                        padded((size_t)2 * s.G * s.Y) * ri;
+    const double toe = 2.0 * (s.X + 1) * padded(2 * s.G) * round_up(s.Y, 16) * kc +
+                       2 * padded((size_t)s.G * round_up(s.Y, 8)) * ri;
+    return toe < pair;
+}
 // Tiles of R at N tiles of w complex columns, and of R^-1 at twice that in
 // real ones.
 static size_t r_tiles(const std::vector<ShapeGroup> &groups, uint32_t w) {
@@ -1085,16 +1097,26 @@ int DftSet::create(const std::vector<JobShape> &shapes) {
     I->inst_local.resize(n);
     I->hg.resize(members.size());
     // Form of a group's y stage: Toeplitz when it has at least kToeMinGroup
-    // instances and Y fits one T tile.
+    // instances and Y fits one T tile (but see below).
     auto takes_toeplitz = [&](uint32_t Y, uint32_t G) {
         return Y <= (uint32_t)T_NMAX && ymode != YMODE_DFT &&
                G >= (ymode == YMODE_TOEPLITZ ? toe_min_group : kToeMinGroup);
     };
     std::vector<ShapeGroup> counts;
+    bool dft_pair = false;  // some group's, whatever the others take
     for (const auto &mv : members) {
         const JobShape &s = shapes[mv[0]];
         counts.push_back({s.X, s.Y, (uint32_t)mv.size(), takes_toeplitz(s.Y, (uint32_t)mv.size())});
+        dft_pair = dft_pair || !counts.back().toe;
     }
+    // Beside other groups' y DFT a Toeplitz stage is a launch more, where the
+    // group could share theirs: there it has to execute fewer products. Measured
+    // on B200, us per step without and with this, of 12 grids of 400x225 and 2 or
+    // 33 others 207 and 185, 370 and 371; 8 of 400x225 and 2 165 and 141; 12 of
+    // 256x256 and 2 161 and 137; 12 of 100x100 and 90 191 and 183. (With the side
+    // branch that tuning may find they are 164 and 183, 129 and 138, 129 and 135.)
+    for (ShapeGroup &s : counts)
+        if (dft_pair && ymode == YMODE_AUTO && !fewer_products(s)) s.toe = false;
     const uint32_t width = tile_width(counts);
     const uint32_t y_width = y_tile_width(counts, width);
     // Programmatic dependent launches where a stage leaves SMs idle: one
@@ -1151,7 +1173,7 @@ int DftSet::create(const std::vector<JobShape> &shapes) {
         const double fRi = 2.0 * tiles_of(g.rowsRi, MT) * tiles_of(g.X, g.wRI) * 2 * g.kpRi * 3;
         const double fT = 2.0 * 2 * g.N1h * tiles_of(2 * g.G, MT) * g.nTy * g.kpC * 3;
         const double fRiT = 2.0 * 2 * tiles_of(g.G * g.Yp, MT) * tiles_of(g.X, g.wRI) * 2 * g.kpRi * 3;
-        g.toe = takes_toeplitz(g.Y, g.G) ? 1u : 0u;
+        g.toe = counts[gi].toe ? 1u : 0u;
         if ((rc = I->alloc(&g.aR, (size_t)2 * g.rowsR * g.kpR))) return rc;
         if ((rc = I->alloc(&H.f1, (size_t)4 * g.N1h * H.kpF1))) return rc;
         if ((rc = I->alloc(&H.g1, (size_t)4 * g.X * H.kpG1))) return rc;
