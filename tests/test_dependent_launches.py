@@ -27,3 +27,11 @@ def test_read_only_loads_are_of_constants(name):
         src = re.sub(r"//[^\n]*", "", f.read())
     used = {re.match(r"\(*([A-Za-z_]\w*(?:\.\w+)?)", a).group(1) for a in re.findall(r"__ldg\(([^;]*)", src)}
     assert used <= READ_ONLY[name], f"{name}: __ldg of {sorted(used - READ_ONLY[name])}"
+
+
+def test_the_pixel_map_is_read_after_the_wait():
+    """A canvas in NoUpdate mode without heat runs the settle pass alone, as a
+    dependent of the launch that may have written the pixel map."""
+    with open(os.path.join(CSRC, "air.cu")) as f:
+        src = re.sub(r"//[^\n]*", "", f.read())
+    assert "load_after_wait(pmap" in src and not re.search(r"__ldg\(\s*pmap", src)

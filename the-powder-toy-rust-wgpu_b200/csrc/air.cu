@@ -166,7 +166,7 @@ __global__ void k_settle(const AirInst I, const uint32_t *__restrict__ pmap, con
                 for (uint32_t dx = 0; dx < 4; ++dx) {
                     uint32_t px = cx * 4 + dx, py = cy * 4 + dy;
                     if (px >= xres || py >= yres) continue;
-                    uint32_t e = __ldg(pmap + (size_t)py * xres + px);
+                    uint32_t e = load_after_wait(pmap + (size_t)py * xres + px);
                     if (e == 0u) continue;
                     uint32_t ty = e & 0x1FFu;
                     if (ty >= nprops) continue;  // guard: no row for this id
